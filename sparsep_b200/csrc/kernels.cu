@@ -9,28 +9,46 @@ namespace sparsep {
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
+// Lets kernel k use `smem` bytes of dynamic shared memory.  The default limit
+// is 48 KB minus the kernel's static shared memory; the largest size set so
+// far is kept per device (host threads may plan concurrently, on different
+// devices).
+template <typename K>
+static cudaError_t allow_smem(K *k, std::atomic<int> (&configured)[64], size_t smem) {
+  if (smem == 0) return cudaSuccess;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::atomic<int> &c = configured[dev & 63];
+  if ((int)smem <= c.load()) return cudaSuccess;
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int cur = c.load();
+  while ((int)smem > cur && !c.compare_exchange_weak(cur, (int)smem)) {
+  }
+  return cudaSuccess;
+}
+
 template <typename T, int FMT, int RB, int CB>
 static cudaError_t launch_t(const Params<T> &P, uint32_t carry_w, int threads, size_t smem, cudaStream_t st) {
-  auto k = spmv_items<T, FMT, RB, CB>;
-  // the default dynamic limit is 48 KB minus the kernel's static shared
-  // memory; the largest size set so far is kept per device (host threads may
-  // plan concurrently, on different devices)
   static std::atomic<int> configured[64];
-  if (smem > 0) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::atomic<int> &c = configured[dev & 63];
-    if ((int)smem > c.load()) {
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      int cur = c.load();
-      while ((int)smem > cur && !c.compare_exchange_weak(cur, (int)smem)) {
-      }
-    }
-  }
-  k<<<P.nitems, threads, smem, st>>>(P, carry_w);
+  if (cudaError_t e = allow_smem(spmv_items<T, FMT, RB, CB>, configured, smem)) return e;
+  spmv_items<T, FMT, RB, CB><<<P.nitems, threads, smem, st>>>(P, carry_w);
   return cudaGetLastError();
+}
+
+// BCSR blocks: the chunk kernel where it takes the block size and type.
+template <typename T, int RB, int CB>
+static cudaError_t launch_bcsr(const Params<T> &P, int threads, size_t smem, cudaStream_t st) {
+  if constexpr (bcsr_chunk_blocks(RB, CB, sizeof(T)) == 0) {
+    return launch_t<T, SPARSEP_FMT_BCSR, RB, CB>(P, 1, threads, smem, st);
+  } else {
+    static std::atomic<int> configured[64];
+    smem = (smem + 127) / 128 * 128 + BlockStage<T, RB, CB>::SMEM;  // a tile's staged x first
+    if (cudaError_t e = allow_smem(bcsr_chunks<T, RB, CB>, configured, smem)) return e;
+    bcsr_chunks<T, RB, CB><<<P.nitems, threads, smem, st>>>(P);
+    return cudaGetLastError();
+  }
 }
 
 template <typename T>
@@ -42,9 +60,9 @@ cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int thre
     case SPARSEP_FMT_CSR: return launch_t<T, SPARSEP_FMT_CSR, 0, 0>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_COO: return launch_t<T, SPARSEP_FMT_COO, 0, 0>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_BCSR:
-      if (rb == 4 && cb == 4) return launch_t<T, SPARSEP_FMT_BCSR, 4, 4>(P, carry_w, threads, smem, st);
-      if (rb == 8 && cb == 8) return launch_t<T, SPARSEP_FMT_BCSR, 8, 8>(P, carry_w, threads, smem, st);
-      if (rb == 2 && cb == 2) return launch_t<T, SPARSEP_FMT_BCSR, 2, 2>(P, carry_w, threads, smem, st);
+      if (rb == 4 && cb == 4) return launch_bcsr<T, 4, 4>(P, threads, smem, st);
+      if (rb == 8 && cb == 8) return launch_bcsr<T, 8, 8>(P, threads, smem, st);
+      if (rb == 2 && cb == 2) return launch_bcsr<T, 2, 2>(P, threads, smem, st);
       return launch_t<T, SPARSEP_FMT_BCSR, 0, 0>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_BCOO:
       if (rb == 4 && cb == 4) return launch_t<T, SPARSEP_FMT_BCOO, 4, 4>(P, carry_w, threads, smem, st);

@@ -16,6 +16,19 @@ cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int thre
 template <typename T>
 cudaError_t launch_merge(const T *part, T *y, uint32_t nrows, uint32_t V, int sms, cudaStream_t st);
 
+// Blocks per chunk (32 KB of values) of the BCSR kernel bcsr_chunks for rb x cb
+// blocks of es-byte elements, 0 for those that spmv_items runs: other block
+// sizes, and 2x2 blocks of 8-byte types, whose 64-byte groups of lanes meet in
+// the same shared-memory banks (FP64, 1M rows, 12 blocks per block row: 73 us
+// in chunks, 62 us there).
+constexpr uint32_t bcsr_chunk_blocks(uint32_t rb, uint32_t cb, size_t es) {
+  return rb == cb && ((rb == 2 && es < 8) || rb == 4 || rb == 8)
+             ? (uint32_t)(32768 / (rb * cb * es) < 2048 ? 32768 / (rb * cb * es) : 2048)
+             : 0;
+}
+// block rows per chunk
+constexpr uint32_t BCSR_CHUNK_ROWS = 512;
+
 // Persistent TMA-pipelined CSR kernel (csr_pipe.cu) for 1D items built by the
 // automatic planner; grid = SMs x resident CTAs (capped at the item count).
 template <typename T>

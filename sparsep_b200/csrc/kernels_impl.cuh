@@ -18,8 +18,10 @@
 // (TMA) copies; their partial y goes to per-stripe slices merged on the device.
 #pragma once
 #include <cstdio>
+#include <cstring>
 
 #include "device.cuh"
+#include "kernels.hpp"
 
 namespace sparsep {
 
@@ -459,7 +461,332 @@ __device__ __forceinline__ void block_mv(const Params<T> &P, const T *__restrict
 }
 
 // ---------------------------------------------------------------------------
-// BCSR block rows, L lanes per block row
+// Dense blocks of 2x2, 4x4 and 8x8, read as the 16-byte pieces they are made
+// of: consecutive lanes take consecutive pieces, so a warp reads 512
+// contiguous bytes of block values whatever the type and the block size.  A
+// block of B bytes is spread over LPB = B / 16 lanes (one lane for blocks of
+// up to 16 bytes); a piece is RPC whole rows of the block, or a CPR-th of one.
+// ---------------------------------------------------------------------------
+template <typename T, int RB, int CB> struct Pieces {
+  static constexpr int B = RB * CB * (int)sizeof(T);
+  static constexpr int BYTES = B < 16 ? B : 16;     // of a piece
+  static constexpr int E = BYTES / (int)sizeof(T);  // elements of a piece
+  static constexpr int LPB = B / BYTES;             // lanes per block
+  static constexpr int RPC = E >= CB ? E / CB : 1;  // rows in a piece
+  static constexpr int CPR = E >= CB ? 1 : CB / E;  // pieces of a row
+  static constexpr int NX = E >= CB ? CB : E;       // x elements a piece meets
+  static constexpr int XB = NX * (int)sizeof(T);    // their bytes
+  static constexpr int W = (BYTES + 3) / 4, XW = (XB + 3) / 4;
+};
+
+// N bytes (2, 4, 8 or 16) at an address aligned to them, as 32-bit words.
+template <int N> __device__ __forceinline__ void load_words(const void *p, uint32_t *w) {
+  if constexpr (N == 16) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+  } else if constexpr (N == 8) {
+    const uint2 q = *reinterpret_cast<const uint2 *>(p);
+    w[0] = q.x, w[1] = q.y;
+  } else if constexpr (N == 4) {
+    w[0] = *reinterpret_cast<const uint32_t *>(p);
+  } else {
+    w[0] = *reinterpret_cast<const uint16_t *>(p);
+  }
+}
+
+// Element i of packed words.
+template <typename T> __device__ __forceinline__ T word_elem(const uint32_t *w, int i) {
+  if constexpr (sizeof(T) == 1) return (T)(int8_t)(w[i >> 2] >> (8 * (i & 3)));
+  else if constexpr (sizeof(T) == 2) return (T)(int16_t)(w[i >> 1] >> (16 * (i & 1)));
+  else {
+    T v;
+    if constexpr (sizeof(T) == 4) {
+      memcpy(&v, &w[i], 4);
+    } else {
+      const unsigned long long u = ((unsigned long long)w[2 * i + 1] << 32) | w[2 * i];
+      memcpy(&v, &u, 8);
+    }
+    return v;
+  }
+}
+
+// The NX elements of x that a piece of a block in block column J meets (xt: x
+// from the tile's first column), packed.  FULL: the block column lies inside
+// the matrix and x is aligned to the NX elements, so one load brings them.
+// Otherwise one by one, zeros past the last column.
+template <typename T, int RB, int CB, bool FULL>
+__device__ __forceinline__ void load_xpiece(const Params<T> &P, const Item &it, const T *__restrict__ xt, uint32_t J,
+                                            uint32_t xcol, uint32_t (&w)[Pieces<T, RB, CB>::XW]) {
+  using G = Pieces<T, RB, CB>;
+  const uint64_t c = (uint64_t)J * CB + xcol;
+  if constexpr (FULL) {
+    if (!SP_BAD(P, x_ok(P, it, it.col_off + c) && x_ok(P, it, it.col_off + c + G::NX - 1), -1011))
+      load_words<G::XB>(xt + c, w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < G::XW; ++i) w[i] = 0;
+#pragma unroll
+    for (int i = 0; i < G::NX; ++i) {
+      T v = T(0);
+      if (it.col_off + c + i < P.ncols && !SP_BAD(P, x_ok(P, it, it.col_off + c + i), -1011)) v = xt[c + i];
+      if constexpr (sizeof(T) == 8) {
+        unsigned long long u;
+        memcpy(&u, &v, 8);
+        w[2 * i] = (uint32_t)u, w[2 * i + 1] = (uint32_t)(u >> 32);
+      } else if constexpr (sizeof(T) == 4) {
+        memcpy(&w[i], &v, 4);
+      } else {
+        constexpr int PER = 4 / (int)sizeof(T), SH = 8 * (int)sizeof(T);
+        w[i / PER] |= ((uint32_t)v & ((1u << SH) - 1u)) << (SH * (i % PER));
+      }
+    }
+  }
+}
+
+// A piece times its x, added to the sums of its rows.
+template <typename T, int RB, int CB>
+__device__ __forceinline__ void piece_mv(const uint32_t (&v)[Pieces<T, RB, CB>::W],
+                                         const uint32_t (&x)[Pieces<T, RB, CB>::XW],
+                                         Acc<T> (&acc)[Pieces<T, RB, CB>::RPC]) {
+  using G = Pieces<T, RB, CB>;
+#pragma unroll
+  for (int r = 0; r < G::RPC; ++r) {
+    if constexpr (sizeof(T) == 1 && G::NX % 4 == 0) {  // four products and their sum in one instruction, exact
+#pragma unroll
+      for (int q = 0; q < G::NX / 4; ++q) acc[r] = (uint32_t)__dp4a((int)v[r * (G::NX / 4) + q], (int)x[q], (int)acc[r]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < G::NX; ++c) acc[r] += mul<T>(word_elem<T>(v, r * G::NX + c), word_elem<T>(x, c));
+    }
+  }
+}
+
+// Sums over the lanes of a group that hold other blocks (strides LPB, 2 LPB,
+// ..., L / 2), or other pieces of the same block row's row (strides below CPR).
+template <typename T, int RB, int CB, int L>
+__device__ __forceinline__ void sum_pieces(Acc<T> (&acc)[Pieces<T, RB, CB>::RPC]) {
+  using G = Pieces<T, RB, CB>;
+#pragma unroll
+  for (int w = 0; w < G::RPC; ++w) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1)
+      if (o >= G::LPB || o < G::CPR) acc[w] += __shfl_xor_sync(0xffffffffu, acc[w], o);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// BCSR in chunks: a work item is a chunk of whole block rows (at most S blocks
+// and ROWS block rows, or one longer block row).  Its values and block columns
+// come into shared memory by bulk copies; then LPB * BK lanes take a block
+// row, BK blocks at a time, and only x is read from memory by loads.
+//
+// Bound by HBM, the block values.  A lane per whole block, as every block size
+// ran before (bcsr_rows), asked for each 32-byte sector twice (lanes 64 bytes
+// apart) with 100 M instructions.  Block-banded matrices, 20 blocks per block
+// row, before -> now: FP32 4x4, 2M rows (732 MB) 191 -> 119 us, 6.1 TB/s, 94 % of
+// the measured copy rate; INT8 8x8, 2M rows (362 MB) 149 -> 62 us; INT16 4x4,
+// 1M rows 71 -> 43 us; FP64 4x4, 1M rows 229 -> 124 us.
+// What was tried on the way, FP32 4x4: the same lanes reading values straight
+// from memory 200 us (the latency of one step after another); a ring of copies
+// per warp over contiguous block rows 185 us (143 M instructions at the block
+// rows' ends); persistent CTAs with two chunks in flight 176 us and with x
+// gathered a chunk ahead 160 us (24 warps per SM cannot hide the x loads).
+// Chunks of 24 / 28 / 40 KB: 133 / 125 / 127 us against 119 us for 32 KB, five
+// CTAs per SM; 46 instead of 40 registers (four CTAs) 126 us.
+// ---------------------------------------------------------------------------
+template <typename T, int RB, int CB> struct BlockStage {
+  using G = Pieces<T, RB, CB>;
+  static constexpr int S = (int)bcsr_chunk_blocks(RB, CB, sizeof(T)), ROWS = (int)BCSR_CHUNK_ROWS;
+  // 4-block (16-byte) alignment at both ends of the copies
+  static constexpr int COL = (S + 8) * G::B, PTR = COL + (S + 8) * 4;
+  static constexpr int SMEM = (PTR + (ROWS + 1) * 4 + 127) / 128 * 128;
+};
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ void expect_bytes(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// Bounded wait of every thread of the CTA for a barrier phase; false (for all)
+// when it ran out: the error word is set, and the copies get one more bounded
+// wait.
+__device__ __forceinline__ bool cta_wait(uint64_t *bar, uint32_t parity, int *err) {
+  auto spin = [&]() {
+    uint32_t done = 0;
+    for (uint32_t i = 0; i < (1u << 22) && !done; ++i)
+      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                   : "=r"(done)
+                   : "r"(smem_u32(bar)), "r"(parity)
+                   : "memory");
+    return done != 0;
+  };
+  if (!__syncthreads_or(!spin())) return true;
+  if (threadIdx.x == 0 && err) atomicExch(err, SPARSEP_ETIMEDOUT);
+  spin();
+  return false;
+}
+
+// The chunk's block rows [it.a0, it.a1): starts in srp (as in browptr), blocks
+// staged from sval / scol on.
+template <typename T, int RB, int CB, int BK, bool FULL>
+__device__ __forceinline__ void bcsr_rows_staged(const Params<T> &P, const Item &it, const T *__restrict__ xt,
+                                                 const uint32_t *srp, const unsigned char *sval,
+                                                 const uint32_t *scol) {
+  using G = Pieces<T, RB, CB>;
+  using A = Acc<T>;
+  constexpr int L = G::LPB * BK, GN = 32 / L;  // lanes per block row, block rows per warp
+  T *out = out_base(P, it);
+  const uint32_t k = (uint32_t)(it.a1 - it.a0), b0 = srp[0];
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane / L, gl = lane % L, q = gl % G::LPB, bi = gl / G::LPB;
+  const uint32_t xcol = (uint32_t)(q % G::CPR) * G::NX;
+  sval += q * G::BYTES;
+  for (uint32_t base = warp * GN; base < k; base += nw * GN) {
+    const uint32_t i = base + g;
+    A acc[G::RPC];
+#pragma unroll
+    for (int w = 0; w < G::RPC; ++w) acc[w] = A(0);
+    if (i < k) {
+      const uint32_t e = srp[i + 1] - b0;
+      uint32_t b = srp[i] - b0 + bi;
+      // two blocks a step: their x on the way together
+      for (; b + BK < e; b += 2 * BK) {
+        uint32_t v[2][G::W], x[2][G::XW];
+        const uint32_t J0 = scol[b], J1 = scol[b + BK];
+        load_xpiece<T, RB, CB, FULL>(P, it, xt, J0, xcol, x[0]);
+        load_xpiece<T, RB, CB, FULL>(P, it, xt, J1, xcol, x[1]);
+        load_words<G::BYTES>(sval + b * G::B, v[0]);
+        load_words<G::BYTES>(sval + (b + BK) * G::B, v[1]);
+        piece_mv<T, RB, CB>(v[0], x[0], acc);
+        piece_mv<T, RB, CB>(v[1], x[1], acc);
+      }
+      if (b < e) {
+        uint32_t v[G::W], x[G::XW];
+        load_xpiece<T, RB, CB, FULL>(P, it, xt, scol[b], xcol, x);
+        load_words<G::BYTES>(sval + b * G::B, v);
+        piece_mv<T, RB, CB>(v, x, acc);
+      }
+    }
+    __syncwarp();
+    sum_pieces<T, RB, CB, L>(acc);
+    if (i < k && bi == 0 && q % G::CPR == 0) {
+      const uint64_t row = (uint64_t)it.row_off + (it.a0 + i) * RB + (q / G::CPR) * G::RPC;
+#pragma unroll
+      for (int w = 0; w < G::RPC; ++w)
+        if (row + w < it.row_end) put<T>(P, out, row + w, acc[w]);
+    }
+  }
+}
+
+// A block row of more blocks than a chunk holds: the CTA's warps share its
+// blocks and read them straight from memory; warp sums added in warp order.
+template <typename T, int RB, int CB, bool FULL>
+__device__ void bcsr_long_row(const Params<T> &P, const Item &it, const T *__restrict__ xt, Acc<T> *red) {
+  using G = Pieces<T, RB, CB>;
+  using A = Acc<T>;
+  constexpr int STEP = 32 / G::LPB;
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = lane % G::LPB, bi = lane / G::LPB;
+  const uint32_t xcol = (uint32_t)(q % G::CPR) * G::NX;
+  A acc[G::RPC];
+#pragma unroll
+  for (int w = 0; w < G::RPC; ++w) acc[w] = A(0);
+#pragma unroll 2
+  for (uint64_t b = it.n0 + warp * STEP + bi; b < it.n1; b += nw * STEP) {
+    uint32_t v[G::W], x[G::XW];
+    load_words<G::BYTES>(reinterpret_cast<const char *>(P.bval) + b * G::B + q * G::BYTES, v);
+    load_xpiece<T, RB, CB, FULL>(P, it, xt, P.bcolind[b], xcol, x);
+    piece_mv<T, RB, CB>(v, x, acc);
+  }
+  __syncwarp();
+  sum_pieces<T, RB, CB, 32>(acc);
+#pragma unroll
+  for (int w = 0; w < G::RPC; ++w)
+    if (bi == 0 && q % G::CPR == 0) red[warp * RB + (q / G::CPR) * G::RPC + w] = acc[w];
+  __syncthreads();
+  const uint64_t row = (uint64_t)it.row_off + it.a0 * RB + threadIdx.x;
+  if (threadIdx.x < RB && row < it.row_end) {
+    A t = A(0);
+    for (int w = 0; w < nw; ++w) t += red[w * RB + threadIdx.x];
+    put<T>(P, out_base(P, it), row, t);
+  }
+}
+
+template <typename T, int RB, int CB>
+__global__ void __launch_bounds__(512, 3) bcsr_chunks(Params<T> P) {
+  using G = Pieces<T, RB, CB>;
+  using St = BlockStage<T, RB, CB>;
+  constexpr int M = 32 / G::LPB;  // most blocks a warp holds
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  __shared__ uint64_t bar, xbar;
+  unsigned char *sm = dyn_smem + (P.smem_bytes + 127) / 128 * 128;  // behind a tile's staged x
+  uint32_t *srp = reinterpret_cast<uint32_t *>(sm + St::PTR);
+  const Item it = P.items[blockIdx.x];
+  const uint64_t A0 = it.n0 & ~3ull, A1 = (it.n1 + 3) & ~3ull;  // the arrays are padded past their end
+  const bool longer = it.n1 - it.n0 > (uint64_t)St::S, stage = it.n0 < it.n1 && !longer;
+  if (SP_BAD(P, A1 <= P.n_idx && A1 * (RB * CB) <= P.n_val, -1013)) return;
+  if (SP_BAD(P, it.ptr_base + it.a1 < P.n_rowptr && it.a1 - it.a0 <= St::ROWS, -1012)) return;
+  mbar_init(&bar);
+  if (threadIdx.x == 0 && stage) {
+    const uint32_t n = (uint32_t)(A1 - A0);
+    expect_bytes(&bar, n * (uint32_t)(G::B + 4));
+    bulk_load(sm + St::COL, P.bcolind + A0, n * 4, &bar);
+    bulk_load(sm, reinterpret_cast<const char *>(P.bval) + A0 * G::B, n * G::B, &bar);
+  }
+  for (uint32_t i = threadIdx.x; i <= (uint32_t)(it.a1 - it.a0); i += blockDim.x)
+    srp[i] = __ldcs(P.rowptr + it.ptr_base + it.a0 + i);
+  const T *xb = P.x;
+  if (it.xw > 0) {
+    uint32_t phase = 0;
+    mbar_init(&xbar);
+    xb = stage_x<T>(P.x, it.xlo, it.xw, dyn_smem, &xbar, phase, P.err, P.smem_bytes,
+                    reinterpret_cast<uintptr_t>(P.x + P.n_xalloc), P.fault_wait);
+  }
+  const T *xt = xb + it.col_off;
+  // x is read piece by piece where it is aligned to them and every block
+  // column of the chunk lies inside the matrix
+  bool whole = (reinterpret_cast<uintptr_t>(xt) & (G::XB - 1)) == 0;
+  const uint32_t jfull = it.col_off < P.ncols ? (P.ncols - it.col_off) / CB : 0;
+  const bool ragged = it.col_off + (uint64_t)jfull * CB < P.ncols;
+  if (longer) {
+    Acc<T> *red = reinterpret_cast<Acc<T> *>(sm);
+    if (whole && !ragged) bcsr_long_row<T, RB, CB, true>(P, it, xt, red);
+    else bcsr_long_row<T, RB, CB, false>(P, it, xt, red);
+    return;
+  }
+  if (stage) {
+    if (!cta_wait(&bar, 0, P.err)) return;
+  } else {
+    __syncthreads();
+  }
+  const uint32_t lead = (uint32_t)(it.n0 - A0);
+  const unsigned char *sval = sm + lead * G::B;
+  const uint32_t *scol = reinterpret_cast<const uint32_t *>(sm + St::COL) + lead;
+  if (whole && ragged) {
+    bool in = true;
+    for (uint32_t b = threadIdx.x; b < it.n1 - it.n0; b += blockDim.x) in &= scol[b] < jfull;
+    whole = !__syncthreads_or(!in);
+  }
+  auto go = [&](auto n) {
+    constexpr int BK = decltype(n)::value;
+    if (whole) bcsr_rows_staged<T, RB, CB, BK, true>(P, it, xt, srp, sval, scol);
+    else bcsr_rows_staged<T, RB, CB, BK, false>(P, it, xt, srp, sval, scol);
+  };
+  const int bk = it.lanes < M ? it.lanes : M;
+  if constexpr (M >= 8) if (bk >= 8) go(std::integral_constant<int, 8>());
+  if constexpr (M >= 4) if (bk == 4) go(std::integral_constant<int, 4>());
+  if constexpr (M >= 2) if (bk == 2) go(std::integral_constant<int, 2>());
+  if (bk == 1) go(std::integral_constant<int, 1>());
+}
+
+// ---------------------------------------------------------------------------
+// BCSR block rows of the other block sizes, L lanes per block row
 // ---------------------------------------------------------------------------
 template <typename T, int RB, int CB, int L>
 __device__ void bcsr_rows(const Params<T> &P, const Item &it, const T *__restrict__ xb) {

@@ -6,7 +6,8 @@
 // (support/partition.h) and scatters the pieces with dpu_push_xfer
 // (spmv/1D/CSR-row/host/app.c:221-252).  Here the same partitions become CTA
 // work items over one device copy of the matrix; nr_parts > 0 reproduces the
-// reference split exactly (one part = one CTA, one tasklet = one warp) and
+// reference split exactly (one part = one CTA, one tasklet = one warp; a BCSR
+// part of 2x2, 4x4 or 8x8 blocks is cut further into chunks of one CTA each) and
 // nr_parts = 0 lets the planner size items for the GPU.
 #include <algorithm>
 #include <climits>
@@ -175,6 +176,9 @@ static constexpr uint64_t AUTO_ITEM_ELEMS = 4096;
 static constexpr uint64_t AUTO_ITEM_ENTRIES = 8192;  // stored block entries per item
 static constexpr size_t STAGE_AUTO_MAX = 96 * 1024;
 static constexpr size_t STAGE_MAX = 200 * 1024;
+// The BCSR chunk kernel holds a chunk (up to 43 KB) beside a staged x, and x is
+// staged for it only where that is asked for: its x comes in vector loads.
+static constexpr size_t STAGE_MAX_BCSR = 176 * 1024;
 
 struct Opts {
   sparsep_opts o;
@@ -511,9 +515,10 @@ static int begin_plan(sparsep_plan **out, int dtype, int format, int scheme, con
 
 static int stage_width(const sparsep_plan *p, const sparsep_opts &o, uint32_t w) {
   size_t bytes = (size_t)w * p->esize + 32;
+  const bool chunks = p->format == SPARSEP_FMT_BCSR && bcsr_chunk_blocks(p->rb, p->cb, p->esize);
   if (o.stage_x == 0 || w == 0) return 0;
-  if (o.stage_x > 0) return bytes <= STAGE_MAX ? (int)w : 0;
-  return bytes <= STAGE_AUTO_MAX ? (int)w : 0;
+  if (o.stage_x > 0) return bytes <= (chunks ? STAGE_MAX_BCSR : STAGE_MAX) ? (int)w : 0;
+  return !chunks && bytes <= STAGE_AUTO_MAX ? (int)w : 0;
 }
 
 static uint64_t compulsory_csr(uint64_t nnz, uint64_t nrows, uint64_t ncols, size_t s) {
@@ -1309,7 +1314,26 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
   p->cb = cb;
   std::vector<Item> items;
   const bool faithful = oo.nr_parts > 0;
-  const uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb));
+  uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb)), nparts = 0;
+  const uint64_t S = bcsr_chunk_blocks(rb, cb, sizeof(T));
+  // Blocks of a block row that a chunk's lanes take at a time: about an eighth
+  // of them, so that a warp works on several block rows at once and its last
+  // step is nearly full.
+  auto chunk_lanes = [](uint64_t m) -> uint32_t {
+    uint32_t l = 1;
+    while (l < 8 && l * 2 <= (m + 4) / 8) l *= 2;
+    return l;
+  };
+  uint64_t rcap = UINT64_MAX;
+  if (S) {
+    per = std::min<uint64_t>(S, std::max<uint64_t>(32, nblocks / (4 * (uint64_t)p->sms)));
+    // whole passes of the CTA's warps over the chunk's block rows
+    const uint64_t m = std::max<uint64_t>(1, nblocks * rb / (std::max<uint64_t>(1, nrows) * V));
+    const uint64_t lpb = std::max<uint64_t>(1, (uint64_t)rb * cb * sizeof(T) / 16);
+    const uint64_t lanes = std::min<uint64_t>(32, lpb * (oo.lanes ? (uint64_t)oo.lanes : chunk_lanes(m)));
+    const uint64_t pass = 32 / lanes * (oo.nr_workers > 0 ? oo.nr_workers : 8);
+    rcap = std::min<uint64_t>(BCSR_CHUNK_ROWS, per / m >= pass ? per / m / pass * pass : UINT64_MAX);
+  }
   for (size_t i = 0; i < tiles.size(); ++i) {
     Tile t = tiles[i];
     t.xw = stage_width(p, oo, t.xw);
@@ -1322,25 +1346,30 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
         Item it = make_item(t, ITEM_ROWS);
         it.a0 = x0;
         it.a1 = x1;
+        it.n0 = t.nnz_base + bp[x0];
+        it.n1 = t.nnz_base + bp[x1];
         uint64_t m = ((uint64_t)bp[x1] - bp[x0] + (x1 - x0) - 1) / (x1 - x0);
-        it.lanes = oo.lanes ? (uint16_t)oo.lanes : (uint16_t)pow2ceil((m + 1) / 2);
+        it.lanes = oo.lanes ? (uint16_t)oo.lanes : (uint16_t)(S ? chunk_lanes(m) : pow2ceil((m + 1) / 2));
         items.push_back(it);
       };
-      if (faithful) {
-        emit(a, b);
-        continue;
-      }
-      uint64_t s0 = a, acc = 0;
-      for (uint64_t r = a; r < b; ++r) {
-        uint64_t n = (uint64_t)bp[r + 1] - bp[r];
-        if (r > s0 && acc + n > per) {
-          emit(s0, r);
-          s0 = r;
-          acc = 0;
+      // block rows [x0, x1) in items of at most cap blocks and rcap block rows
+      auto cut = [&](uint64_t x0, uint64_t x1, uint64_t cap, uint64_t rcap) {
+        uint64_t s0 = x0, acc = 0;
+        for (uint64_t r = x0; r < x1; ++r) {
+          uint64_t n = (uint64_t)bp[r + 1] - bp[r];
+          if (r > s0 && (acc + n > cap || r - s0 >= rcap)) {
+            emit(s0, r);
+            s0 = r;
+            acc = 0;
+          }
+          acc += n;
         }
-        acc += n;
-      }
-      emit(s0, b);
+        emit(s0, x1);
+      };
+      if (a < b) ++nparts;
+      if (faithful && !S) emit(a, b);
+      else if (faithful) cut(a, b, S, rcap);  // a part's chunks run on several CTAs
+      else cut(a, b, per, rcap);
     }
   }
   set_out_mode(p, oo, V, false, 1);
@@ -1354,6 +1383,7 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
   p->info.compulsory_bytes = nblocks * (4 + (uint64_t)rb * cb * sizeof(T)) + (nbr + 1) * 4 +
                              (uint64_t)ncols * sizeof(T) + (uint64_t)nrows * sizeof(T);
   if ((st = finish_plan(p, items, o2))) return st;
+  if (faithful) p->info.items = nparts;
   p->t[0] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   *out = guard.release();
   return SPARSEP_OK;

@@ -137,6 +137,8 @@ struct Item {
   uint32_t xlo, xw;     // stage x[xlo, xlo+xw) in shared memory when xw > 0
   uint32_t slot;        // partial-y slice (2D lock-free)
   uint16_t kind, lanes;
+  // ITEM_ELEMS: the rows that the item shares with its neighbours (RowGroup):
+  // its first row {cslot, first, nchunk}, its last {chunk, crow, n1}
   uint32_t crow;        // ITEM_LONG: output row
   uint32_t chunk;       // ITEM_LONG: chunk index within the row (0 owns the row)
   uint32_t worker_bal;  // ITEM_ROWS: sparsep_balance across warps
@@ -174,7 +176,7 @@ template <typename T> struct Params {
   unsigned long long *carry_val;
   unsigned long long *carry_idx;  // output index or ~0ull
   unsigned int *done;             // completion counter, reset by the last CTA
-  unsigned int *row_cnt;          // per long row arrival counters (pipelined CSR)
+  unsigned int *row_cnt;          // arrival counters: per long CSR row, per row shared by COO / BCOO items
   unsigned int *band_cnt;         // when set: items finished per row band of y (one counter per band)
   int *err;                       // device error word (bounded waits, checked builds)
   // array extents, used by the bounds-checked build (-DSPARSEP_CHECK)

@@ -51,6 +51,22 @@ static cudaError_t launch_bcsr(const Params<T> &P, int threads, size_t smem, cud
   }
 }
 
+template <typename T, int RB, int CB>
+static cudaError_t launch_bcoo(const Params<T> &P, int threads, size_t smem, cudaStream_t st) {
+  static std::atomic<int> configured[64];
+  smem = (smem + 127) / 128 * 128 + BcooStage<T, RB, CB>::SMEM;
+  if (cudaError_t e = allow_smem(bcoo_chunks<T, RB, CB>, configured, smem)) return e;
+  bcoo_chunks<T, RB, CB><<<P.nitems, threads, smem, st>>>(P);
+  return cudaGetLastError();
+}
+template <typename T, bool ATOMIC>
+static cudaError_t launch_coo(const Params<T> &P, int threads, size_t smem, cudaStream_t st) {
+  static std::atomic<int> configured[64];
+  if (cudaError_t e = allow_smem(coo_items<T, ATOMIC>, configured, smem)) return e;
+  coo_items<T, ATOMIC><<<P.nitems, threads, smem, st>>>(P);
+  return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int threads, size_t smem,
                          cudaStream_t st) {
@@ -58,16 +74,18 @@ cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int thre
   const uint32_t rb = P.rb, cb = P.cb;
   switch (fmt) {
     case SPARSEP_FMT_CSR: return launch_t<T, SPARSEP_FMT_CSR, 0, 0>(P, carry_w, threads, smem, st);
-    case SPARSEP_FMT_COO: return launch_t<T, SPARSEP_FMT_COO, 0, 0>(P, carry_w, threads, smem, st);
+    case SPARSEP_FMT_COO:
+      return P.out_mode == OUT_ATOMIC ? launch_coo<T, true>(P, threads, smem, st)
+                                      : launch_coo<T, false>(P, threads, smem, st);
     case SPARSEP_FMT_BCSR:
       if (rb == 4 && cb == 4) return launch_bcsr<T, 4, 4>(P, threads, smem, st);
       if (rb == 8 && cb == 8) return launch_bcsr<T, 8, 8>(P, threads, smem, st);
       if (rb == 2 && cb == 2) return launch_bcsr<T, 2, 2>(P, threads, smem, st);
       return launch_t<T, SPARSEP_FMT_BCSR, 0, 0>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_BCOO:
-      if (rb == 4 && cb == 4) return launch_t<T, SPARSEP_FMT_BCOO, 4, 4>(P, carry_w, threads, smem, st);
-      if (rb == 8 && cb == 8) return launch_t<T, SPARSEP_FMT_BCOO, 8, 8>(P, carry_w, threads, smem, st);
-      if (rb == 2 && cb == 2) return launch_t<T, SPARSEP_FMT_BCOO, 2, 2>(P, carry_w, threads, smem, st);
+      if (rb == 4 && cb == 4) return launch_bcoo<T, 4, 4>(P, threads, smem, st);
+      if (rb == 8 && cb == 8) return launch_bcoo<T, 8, 8>(P, threads, smem, st);
+      if (rb == 2 && cb == 2) return launch_bcoo<T, 2, 2>(P, threads, smem, st);
       return launch_t<T, SPARSEP_FMT_BCOO, 0, 0>(P, carry_w, threads, smem, st);
   }
   return cudaErrorInvalidValue;

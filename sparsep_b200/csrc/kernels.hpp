@@ -29,6 +29,20 @@ constexpr uint32_t bcsr_chunk_blocks(uint32_t rb, uint32_t cb, size_t es) {
 // block rows per chunk
 constexpr uint32_t BCSR_CHUNK_ROWS = 512;
 
+// Nonzeros per automatic COO item: 4096, fewer where that leaves less than six
+// items per SM (1.5 M nonzeros, FP32: 20 us in 366 items, 16.5 us in 733; 16.7 M:
+// 94 us in items of 2048, 91 us of 4096).
+constexpr uint32_t coo_item_elems(uint64_t nnz) {
+  return nnz >= 4096 * 888ull ? 4096 : nnz <= 512 * 888ull ? 512 : (uint32_t)((nnz / 888 + 3) & ~3ull);
+}
+// Blocks per BCOO chunk (bcoo_chunks, 32 KB of values at most), 0 for the block
+// sizes that spmv_items runs.
+constexpr uint32_t bcoo_chunk_blocks(uint32_t rb, uint32_t cb, size_t es) {
+  return rb == cb && (rb == 2 || rb == 4 || rb == 8)
+             ? (uint32_t)(32768 / (rb * cb * es) < 1024 ? 32768 / (rb * cb * es) : 1024)
+             : 0;
+}
+
 // Persistent TMA-pipelined CSR kernel (csr_pipe.cu) for 1D items built by the
 // automatic planner; grid = SMs x resident CTAs (capped at the item count).
 template <typename T>

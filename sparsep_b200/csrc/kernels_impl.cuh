@@ -26,7 +26,6 @@
 namespace sparsep {
 
 constexpr unsigned long long NO_CARRY = ~0ull;
-constexpr int COO_K = 4;  // elements per thread per chunk
 
 // ---------------------------------------------------------------------------
 // output helpers
@@ -125,6 +124,113 @@ __device__ void csr_rows(const Params<T> &P, const Item &it, const T *__restrict
     we = wb + q + (warp < (int)rem ? 1 : 0);
   }
   for (uint64_t base = wb; base < we; base += G) do_row(base + g, base + g < we);
+}
+
+// ---------------------------------------------------------------------------
+// Sums of the rows in a warp's stream of products (CSR rows, COO nonzeros), in
+// windows of 32 lanes x K consecutive products.  A lane writes the rows that
+// begin and end with it, a segmented scan over the lanes gives the others; a
+// window inside one row only adds to the lanes' sums.  The part of the warp's
+// first row and of its last one are left to the caller, since other warps may
+// have parts of them too.
+// ---------------------------------------------------------------------------
+template <typename A> __device__ __forceinline__ A warp_sum(A v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <typename A> struct RowStream {
+  A acc = A(0), osum = A(0);  // the open row's sum: a part per lane (windows inside the row) and the rest
+  uint32_t open;              // the open row
+  bool heads = false;         // a row began inside the stream: the first row's sum is in *first
+  bool pend = false;          // acc holds something
+};
+
+// One window: products v, bit j of `hb` set where a row begins with the lane's
+// product j, the row in rk[j].  put(row, sum) writes a row; *first takes the sum
+// of the stream's first row once it has ended.
+template <int K, typename A, typename Put>
+__device__ __forceinline__ void row_window(RowStream<A> &S, const A (&v)[K], uint32_t hb, const uint32_t (&rk)[K],
+                                           A *first, Put put) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool h0 = hb & 1u, brk = hb > 1u;
+  const uint32_t mh = __ballot_sync(FULL, h0), mb = __ballot_sync(FULL, brk), m = mh | mb;
+  A run = v[0];
+  if (m == 0) {  // the window lies inside the open row
+#pragma unroll
+    for (int j = 1; j < K; ++j) run += v[j];
+    S.acc += run;
+    S.pend = true;
+    return;
+  }
+  // the lane's products: its first row's part, rows of its own, its last row's part
+  A hd = A(0);
+  uint32_t row = rk[0];
+  bool one = true;  // still in the first row
+#pragma unroll
+  for (int j = 1; j < K; ++j) {
+    const bool h = (hb >> j) & 1u;
+    if (h && !one) put(row, run);
+    hd = h && one ? run : hd;
+    one = one && !h;
+    run = h ? v[j] : run + v[j];
+    row = h ? rk[j] : row;
+  }
+  // the row that a lane goes on with is the last that began before it
+  const uint32_t upto = FULL >> (31 - lane), below = m & (upto >> 1);
+  const uint32_t from = __shfl_sync(FULL, row, below ? 31 - __clz(below) : 0);
+  const uint32_t in = below ? from : S.open;
+  const uint32_t row0 = h0 ? rk[0] : in;  // the lane's first row
+  if (!h0 && !brk) row = in;              // and its last one
+  // sums over the lanes since the last row began
+  const int s = m & upto ? 31 - __clz(m & upto) : 0;
+  A sc = run;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const A o = __shfl_up_sync(FULL, sc, d);
+    if (lane - d >= s) sc += o;
+  }
+  const A up = __shfl_up_sync(FULL, sc, 1);
+  if (lane > 0 && !h0) hd += up;  // the first row's part with what lanes before have of it
+  // The open row ends before lane 0's products (c < 0), or in lane c: in its first
+  // row (brk) or with its last.
+  if (S.pend) S.osum += warp_sum<A>(S.acc);
+  const int cb = mb ? __ffs(mb) - 1 : 32, ch = mh ? __ffs(mh) - 2 : 32, c = cb < ch ? cb : ch;
+  const bool ends = lane < 31 && ((mh >> (lane + 1)) & 1u);  // the lane's last row ends with it
+  if (S.heads) {
+    const A add = lane == c ? S.osum : A(0);
+    if (c < 0 && lane == 0) put(S.open, S.osum);
+    if (brk) put(row0, hd + add);
+    if (ends) put(row, brk ? sc : sc + add);
+  } else {
+    const bool mine = lane == c;
+    if (mine || (c < 0 && lane == 0)) *first = S.osum + (c < 0 ? A(0) : brk ? hd : sc);
+    if (brk && !mine) put(row0, hd);
+    if (ends && (brk || !mine)) put(row, sc);
+  }
+  S.heads = true;
+  S.pend = false;
+  S.acc = A(0);
+  S.osum = __shfl_sync(FULL, sc, 31);
+  S.open = __shfl_sync(FULL, row, 31);
+}
+
+// What a CTA's warps leave of their streams: warp w's first row k0 with its
+// part, and where a row began inside (heads) its last row k1 with its part.
+template <typename A> struct StreamEnds {
+  A first[16], last[16];
+  uint32_t k0[16], k1[16], heads[16];
+};
+template <typename A> __device__ __forceinline__ void leave_ends(StreamEnds<A> &E, int w, RowStream<A> &S) {
+  const A rest = S.osum + (S.pend ? warp_sum<A>(S.acc) : A(0));
+  if ((threadIdx.x & 31) == 0) {
+    if (S.heads) E.last[w] = rest;
+    else E.first[w] = rest;
+    E.k1[w] = S.open;
+    E.heads[w] = S.heads;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -331,10 +437,6 @@ __device__ void csr_long(const Params<T> &P, const Item &it, const T *__restrict
   }
 }
 
-// ---------------------------------------------------------------------------
-// Units of the element-wise paths: COO elements (W = 1) and BCOO blocks
-// (W = rb).  A unit has a key (output row / block row) and W products.
-// ---------------------------------------------------------------------------
 // the reference's AoS nonzero for element type T
 template <typename T> struct ElemOf;
 template <> struct ElemOf<int8_t> { using type = sparsep_elem_i8; };
@@ -343,61 +445,6 @@ template <> struct ElemOf<int32_t> { using type = sparsep_elem_i32; };
 template <> struct ElemOf<int64_t> { using type = sparsep_elem_i64; };
 template <> struct ElemOf<float> { using type = sparsep_elem_f32; };
 template <> struct ElemOf<double> { using type = sparsep_elem_f64; };
-
-template <typename T, int W>
-struct Unit {
-  long long key;
-  Acc<T> v[W];
-};
-
-// Load the 4 COO elements of aligned group g (reference elem_t layout:
-// {u32 rowind, u32 colind, val_dt val}, 12 bytes for types up to 4 bytes and
-// 16 bytes for 8-byte types).
-template <typename T>
-__device__ __forceinline__ void load_coo4(const Params<T> &P, const Item &it, const T *__restrict__ xb,
-                                          uint64_t g, Unit<T, 1> (&u)[4], uint64_t lo, uint64_t hi) {
-  if (4 * g + 3 >= P.n_elems) {
-    // last group of an array without padding: load only the elements that exist
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t e = 4 * g + k;
-      u[k].key = LLONG_MAX;
-      u[k].v[0] = Acc<T>(0);
-      if (e < P.n_elems && e >= lo && e < hi) {
-        const auto *el = reinterpret_cast<const typename ElemOf<T>::type *>(P.elems) + e;
-        u[k].key = (long long)it.row_off + el->rowind;
-        u[k].v[0] = mul<T>(el->val, xload(xb, (uint64_t)it.col_off + el->colind, it.xw > 0));
-      }
-    }
-    return;
-  }
-  if constexpr (sizeof(T) <= 4) {
-    const char *base = reinterpret_cast<const char *>(P.elems) + g * 48;
-    uint4 w0 = ld_stream4(base), w1 = ld_stream4(base + 16), w2 = ld_stream4(base + 32);
-    uint32_t w[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      uint64_t e = 4 * g + k;
-      bool ok = e >= lo && e < hi && !SP_BAD(P, !(e >= lo && e < hi) || x_ok(P, it, (uint64_t)it.col_off + w[3 * k + 1]), -1009);
-      T val;
-      if constexpr (sizeof(T) == 1) val = (T)(int8_t)(w[3 * k + 2] & 0xFF);
-      else if constexpr (sizeof(T) == 2) val = (T)(int16_t)(w[3 * k + 2] & 0xFFFF);
-      else val = __builtin_bit_cast(T, w[3 * k + 2]);
-      u[k].key = ok ? (long long)it.row_off + w[3 * k] : LLONG_MAX;
-      u[k].v[0] = ok ? mul<T>(val, xload(xb, (uint64_t)it.col_off + w[3 * k + 1], it.xw > 0)) : Acc<T>(0);
-    }
-  } else {
-    const char *base = reinterpret_cast<const char *>(P.elems) + g * 64;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      uint4 w = ld_stream4(base + 16 * k);
-      uint64_t e = 4 * g + k;
-      bool ok = e >= lo && e < hi && !SP_BAD(P, !(e >= lo && e < hi) || x_ok(P, it, (uint64_t)it.col_off + w.y), -1009);
-      T val = __builtin_bit_cast(T, ((unsigned long long)w.w << 32) | w.z);
-      u[k].key = ok ? (long long)it.row_off + w.x : LLONG_MAX;
-      u[k].v[0] = ok ? mul<T>(val, xload(xb, (uint64_t)it.col_off + w.y, it.xw > 0)) : Acc<T>(0);
-    }
-  }
-}
 
 // Row-vector of CB elements of a dense block row, at an address aligned to CB*sizeof(T).
 template <typename T, int CB>
@@ -613,36 +660,38 @@ __device__ __forceinline__ void expect_bytes(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
-// Bounded wait of every thread of the CTA for a barrier phase; false (for all)
-// when it ran out: the error word is set, and the copies get one more bounded
-// wait.
+// Bounded wait of the CTA for a barrier phase; false (for all) when it ran out:
+// the error word is set, and the copies get one more bounded wait.  The first
+// warp polls, suspended up to ~20 us per try, and the others wait for it at the
+// CTA's barrier, out of the way of the other CTAs (COO FP32, 1M-row power-law
+// matrix: 122 us with every warp polling, 116 us).
 __device__ __forceinline__ bool cta_wait(uint64_t *bar, uint32_t parity, int *err) {
-  auto spin = [&]() {
+  auto poll = [&]() {
     uint32_t done = 0;
-    for (uint32_t i = 0; i < (1u << 22) && !done; ++i)
-      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+    for (uint32_t i = 0; i < (1u << 18) && !done; ++i)
+      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
                    : "=r"(done)
-                   : "r"(smem_u32(bar)), "r"(parity)
+                   : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
                    : "memory");
     return done != 0;
   };
-  if (!__syncthreads_or(!spin())) return true;
+  if (!__syncthreads_or(threadIdx.x < 32 && !poll())) return true;
   if (threadIdx.x == 0 && err) atomicExch(err, SPARSEP_ETIMEDOUT);
-  spin();
+  if (threadIdx.x < 32) poll();
   return false;
 }
 
-// The chunk's block rows [it.a0, it.a1): starts in srp (as in browptr), blocks
-// staged from sval / scol on.
-template <typename T, int RB, int CB, int BK, bool FULL>
-__device__ __forceinline__ void bcsr_rows_staged(const Params<T> &P, const Item &it, const T *__restrict__ xt,
-                                                 const uint32_t *srp, const unsigned char *sval,
-                                                 const uint32_t *scol) {
+// k block rows whose blocks are staged from sval on, block columns from scol on
+// (CS apart), block row i at [srp[i], srp[i + 1]) - srp[0].  put_row(i, r, sum)
+// takes row r of block row i from the lane that holds its sum.
+template <typename T, int RB, int CB, int BK, bool FULL, int CS, typename Put>
+__device__ __forceinline__ void block_rows_staged(const Params<T> &P, const Item &it, const T *__restrict__ xt,
+                                                  uint32_t k, const uint32_t *srp, const unsigned char *sval,
+                                                  const uint32_t *scol, Put put_row) {
   using G = Pieces<T, RB, CB>;
   using A = Acc<T>;
   constexpr int L = G::LPB * BK, GN = 32 / L;  // lanes per block row, block rows per warp
-  T *out = out_base(P, it);
-  const uint32_t k = (uint32_t)(it.a1 - it.a0), b0 = srp[0];
+  const uint32_t b0 = srp[0];
   const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / L, gl = lane % L, q = gl % G::LPB, bi = gl / G::LPB;
   const uint32_t xcol = (uint32_t)(q % G::CPR) * G::NX;
@@ -658,7 +707,7 @@ __device__ __forceinline__ void bcsr_rows_staged(const Params<T> &P, const Item 
       // two blocks a step: their x on the way together
       for (; b + BK < e; b += 2 * BK) {
         uint32_t v[2][G::W], x[2][G::XW];
-        const uint32_t J0 = scol[b], J1 = scol[b + BK];
+        const uint32_t J0 = scol[b * CS], J1 = scol[(b + BK) * CS];
         load_xpiece<T, RB, CB, FULL>(P, it, xt, J0, xcol, x[0]);
         load_xpiece<T, RB, CB, FULL>(P, it, xt, J1, xcol, x[1]);
         load_words<G::BYTES>(sval + b * G::B, v[0]);
@@ -668,7 +717,7 @@ __device__ __forceinline__ void bcsr_rows_staged(const Params<T> &P, const Item 
       }
       if (b < e) {
         uint32_t v[G::W], x[G::XW];
-        load_xpiece<T, RB, CB, FULL>(P, it, xt, scol[b], xcol, x);
+        load_xpiece<T, RB, CB, FULL>(P, it, xt, scol[b * CS], xcol, x);
         load_words<G::BYTES>(sval + b * G::B, v);
         piece_mv<T, RB, CB>(v, x, acc);
       }
@@ -676,17 +725,47 @@ __device__ __forceinline__ void bcsr_rows_staged(const Params<T> &P, const Item 
     __syncwarp();
     sum_pieces<T, RB, CB, L>(acc);
     if (i < k && bi == 0 && q % G::CPR == 0) {
-      const uint64_t row = (uint64_t)it.row_off + (it.a0 + i) * RB + (q / G::CPR) * G::RPC;
 #pragma unroll
-      for (int w = 0; w < G::RPC; ++w)
-        if (row + w < it.row_end) put<T>(P, out, row + w, acc[w]);
+      for (int w = 0; w < G::RPC; ++w) put_row(i, (q / G::CPR) * G::RPC + w, acc[w]);
     }
   }
 }
 
+// The same for the item's number of blocks at a time, as far as a warp holds them.
+template <typename T, int RB, int CB, int CS, typename Put>
+__device__ __forceinline__ void block_rows_any(const Params<T> &P, const Item &it, const T *__restrict__ xt,
+                                               uint32_t k, const uint32_t *srp, const unsigned char *sval,
+                                               const uint32_t *scol, uint32_t lanes, bool whole, Put put_row) {
+  constexpr uint32_t M = 32 / Pieces<T, RB, CB>::LPB;
+  auto go = [&](auto n) {
+    constexpr int BK = decltype(n)::value;
+    if (whole) block_rows_staged<T, RB, CB, BK, true, CS>(P, it, xt, k, srp, sval, scol, put_row);
+    else block_rows_staged<T, RB, CB, BK, false, CS>(P, it, xt, k, srp, sval, scol, put_row);
+  };
+  const uint32_t bk = lanes < M ? lanes : M;
+  if constexpr (M >= 8) if (bk >= 8) go(std::integral_constant<int, 8>());
+  if constexpr (M >= 4) if (bk == 4) go(std::integral_constant<int, 4>());
+  if constexpr (M >= 2) if (bk == 2) go(std::integral_constant<int, 2>());
+  if (bk == 1) go(std::integral_constant<int, 1>());
+}
+
+// Whether x can be read piece by piece: it is aligned to the pieces and the
+// chunk's n block columns (CS apart) lie inside the matrix.  A barrier where the
+// tile's last block column is ragged.
+template <typename T, int RB, int CB, int CS>
+__device__ __forceinline__ bool x_whole(const Params<T> &P, const Item &it, const T *xt, const uint32_t *scol,
+                                        uint32_t n) {
+  if (reinterpret_cast<uintptr_t>(xt) & (Pieces<T, RB, CB>::XB - 1)) return false;
+  const uint32_t jfull = it.col_off < P.ncols ? (P.ncols - it.col_off) / CB : 0;
+  if (it.col_off + (uint64_t)jfull * CB >= P.ncols) return true;
+  bool in = true;
+  for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) in &= scol[b * CS] < jfull;
+  return !__syncthreads_or(!in);
+}
+
 // A block row of more blocks than a chunk holds: the CTA's warps share its
 // blocks and read them straight from memory; warp sums added in warp order.
-template <typename T, int RB, int CB, bool FULL>
+template <typename T, int RB, int CB>
 __device__ void bcsr_long_row(const Params<T> &P, const Item &it, const T *__restrict__ xt, Acc<T> *red) {
   using G = Pieces<T, RB, CB>;
   using A = Acc<T>;
@@ -701,7 +780,7 @@ __device__ void bcsr_long_row(const Params<T> &P, const Item &it, const T *__res
   for (uint64_t b = it.n0 + warp * STEP + bi; b < it.n1; b += nw * STEP) {
     uint32_t v[G::W], x[G::XW];
     load_words<G::BYTES>(reinterpret_cast<const char *>(P.bval) + b * G::B + q * G::BYTES, v);
-    load_xpiece<T, RB, CB, FULL>(P, it, xt, P.bcolind[b], xcol, x);
+    load_xpiece<T, RB, CB, false>(P, it, xt, P.bcolind[b], xcol, x);
     piece_mv<T, RB, CB>(v, x, acc);
   }
   __syncwarp();
@@ -722,7 +801,6 @@ template <typename T, int RB, int CB>
 __global__ void __launch_bounds__(512, 3) bcsr_chunks(Params<T> P) {
   using G = Pieces<T, RB, CB>;
   using St = BlockStage<T, RB, CB>;
-  constexpr int M = 32 / G::LPB;  // most blocks a warp holds
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   __shared__ uint64_t bar, xbar;
   unsigned char *sm = dyn_smem + (P.smem_bytes + 127) / 128 * 128;  // behind a tile's staged x
@@ -749,15 +827,9 @@ __global__ void __launch_bounds__(512, 3) bcsr_chunks(Params<T> P) {
                     reinterpret_cast<uintptr_t>(P.x + P.n_xalloc), P.fault_wait);
   }
   const T *xt = xb + it.col_off;
-  // x is read piece by piece where it is aligned to them and every block
-  // column of the chunk lies inside the matrix
-  bool whole = (reinterpret_cast<uintptr_t>(xt) & (G::XB - 1)) == 0;
-  const uint32_t jfull = it.col_off < P.ncols ? (P.ncols - it.col_off) / CB : 0;
-  const bool ragged = it.col_off + (uint64_t)jfull * CB < P.ncols;
+  T *out = out_base(P, it);
   if (longer) {
-    Acc<T> *red = reinterpret_cast<Acc<T> *>(sm);
-    if (whole && !ragged) bcsr_long_row<T, RB, CB, true>(P, it, xt, red);
-    else bcsr_long_row<T, RB, CB, false>(P, it, xt, red);
+    bcsr_long_row<T, RB, CB>(P, it, xt, reinterpret_cast<Acc<T> *>(sm));
     return;
   }
   if (stage) {
@@ -766,23 +838,13 @@ __global__ void __launch_bounds__(512, 3) bcsr_chunks(Params<T> P) {
     __syncthreads();
   }
   const uint32_t lead = (uint32_t)(it.n0 - A0);
-  const unsigned char *sval = sm + lead * G::B;
   const uint32_t *scol = reinterpret_cast<const uint32_t *>(sm + St::COL) + lead;
-  if (whole && ragged) {
-    bool in = true;
-    for (uint32_t b = threadIdx.x; b < it.n1 - it.n0; b += blockDim.x) in &= scol[b] < jfull;
-    whole = !__syncthreads_or(!in);
-  }
-  auto go = [&](auto n) {
-    constexpr int BK = decltype(n)::value;
-    if (whole) bcsr_rows_staged<T, RB, CB, BK, true>(P, it, xt, srp, sval, scol);
-    else bcsr_rows_staged<T, RB, CB, BK, false>(P, it, xt, srp, sval, scol);
-  };
-  const int bk = it.lanes < M ? it.lanes : M;
-  if constexpr (M >= 8) if (bk >= 8) go(std::integral_constant<int, 8>());
-  if constexpr (M >= 4) if (bk == 4) go(std::integral_constant<int, 4>());
-  if constexpr (M >= 2) if (bk == 2) go(std::integral_constant<int, 2>());
-  if (bk == 1) go(std::integral_constant<int, 1>());
+  const bool whole = x_whole<T, RB, CB, 1>(P, it, xt, scol, (uint32_t)(it.n1 - it.n0));
+  block_rows_any<T, RB, CB, 1>(P, it, xt, (uint32_t)(it.a1 - it.a0), srp, sm + lead * G::B, scol, it.lanes, whole,
+                               [&](uint32_t i, uint32_t r, Acc<T> sum) {
+                                 const uint64_t row = (uint64_t)it.row_off + (it.a0 + i) * RB + r;
+                                 if (row < it.row_end) put<T>(P, out, row, sum);
+                               });
 }
 
 // ---------------------------------------------------------------------------
@@ -831,37 +893,435 @@ __device__ void bcsr_rows(const Params<T> &P, const Item &it, const T *__restric
 }
 
 // ---------------------------------------------------------------------------
-// Element-wise lock-free path (COO W=1, BCOO W=rb): block segmented scan.
-// Keys are output rows (COO) or output block rows (BCOO, row = key*rb + r).
-// The item writes every row in [own0, own1): sums of complete row runs, zeros
-// for rows without units; a run reaching own1 is a carry for the fix-up.
+// Rows shared by several element items.  A COO item is a range of nonzeros (a
+// BCOO item of blocks), so its first and its last row may go on in its
+// neighbours.  The planner numbers those rows: each has a counter and knows
+// its items [f, f + n), consecutive ones.  Every item of the row leaves its part
+// in its slots (2 item: as the row's last item, 2 item + 1: as an earlier one)
+// and counts itself; the last to arrive adds the parts in item order, the row's
+// last item's part last, writes the row and clears the counter.  Every item
+// arrives, also after a failed wait (with zeros), so the counters are zero
+// between launches.
 // ---------------------------------------------------------------------------
-// Output row of key k, lane r: COO keys are output rows; BCOO keys are
-// tile-local block rows (row = row_off + k*rb + r).
+struct RowGroup {
+  uint32_t cnt, f, n;  // counter, first item, items (0: the row is the item's own)
+};
+__device__ __forceinline__ RowGroup first_row_group(const Item &it) { return {it.cslot, it.first, it.nchunk}; }
+__device__ __forceinline__ RowGroup last_row_group(const Item &it) { return {it.chunk, it.crow, (uint32_t)it.n1}; }
+
+// An item's part of a shared row (of the W rows of a shared block row): lane r < W
+// of the warp holds row r, which belongs at out[row0 + r].
+template <typename T> struct SharedPart {
+  RowGroup g{0, 0, 0};  // n = 0: none
+  uint64_t row0 = 0;
+  Acc<T> part = Acc<T>(0);
+};
+
+// One warp leaves the parts of the item's first and last row, counts the item
+// in for both at once, and adds up the rows that are complete by that.  Rows from
+// `row_end` on are dropped.
 template <typename T, int W>
-__device__ __forceinline__ uint64_t key_row(const Item &it, long long k, uint32_t r, uint32_t rb) {
-  if constexpr (W == 1) return (uint64_t)k;
-  else return (uint64_t)it.row_off + (uint64_t)k * rb + r;
+__device__ void arrive(const Params<T> &P, T *out, uint32_t item, uint64_t row_end, const SharedPart<T> &first,
+                       const SharedPart<T> &last) {
+  using A = Acc<T>;
+  const uint32_t lane = threadIdx.x & 31;
+  auto slot = [](const RowGroup &g, uint32_t i) {
+    return (uint64_t)(2 * (uint64_t)i + (i == g.f + g.n - 1 ? 0 : 1)) * W;
+  };
+  if (SP_BAD(P, (2 * (uint64_t)item + 2) * W <= P.n_carry, -1018)) return;
+  if (lane < W) {
+    if (first.g.n) P.carry_val[slot(first.g, item) + lane] = acc_bits(first.part);
+    if (last.g.n) P.carry_val[slot(last.g, item) + lane] = acc_bits(last.part);
+  }
+  __threadfence();  // the parts are visible before the arrival
+  __syncwarp();
+  unsigned int prev = 0;
+  if (lane == 0 && first.g.n) prev = atomicAdd(P.row_cnt + first.g.cnt, 1u);
+  if (lane == 1 && last.g.n) prev = atomicAdd(P.row_cnt + last.g.cnt, 1u);
+  for (int which = 0; which < 2; ++which) {
+    const SharedPart<T> &s = which ? last : first;
+    if (s.g.n == 0 || __shfl_sync(0xffffffffu, prev, which) != s.g.n - 1) continue;
+    __threadfence();
+    const RowGroup g = s.g;
+    A sum = A(0);
+    if constexpr (W == 1) {  // 32 parts per round trip, added one after the other
+      for (uint32_t c0 = 0; c0 + 1 < g.n; c0 += 32) {
+        const uint32_t c = c0 + lane;
+        const A v = c + 1 < g.n ? bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + c))) : A(0);
+        for (uint32_t j = 0; j < 32 && c0 + j + 1 < g.n; ++j) {
+          const A t = __shfl_sync(0xffffffffu, v, j);
+          sum = c0 + j ? sum + t : t;
+        }
+      }
+    } else if (lane < W) {
+#pragma unroll 4
+      for (uint32_t c = 0; c + 1 < g.n; ++c) {
+        const A t = bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + c) + lane));
+        sum = c ? sum + t : t;
+      }
+    }
+    if (lane < W) {
+      sum = bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + g.n - 1) + lane)) + sum;
+      if (s.row0 + lane < row_end && !SP_BAD(P, s.row0 + lane < P.nrows, -1015))
+        out[s.row0 + lane] = from_acc<T>(sum);
+    }
+    if (lane == 0) P.row_cnt[g.cnt] = 0;  // ready for the next launch
+  }
 }
 
-template <typename T, int W>
-__device__ __forceinline__ void zero_rows(const Params<T> &P, const Item &it, T *out, long long k0, long long k1,
-                                          uint32_t rb) {
+// ---------------------------------------------------------------------------
+// COO nonzeros (AoS, sorted by row) as a stream of products: each warp takes an
+// even share of the item's nonzeros, K consecutive ones per lane and window
+// (128-bit loads, the next window's under way); a row begins where the row index
+// changes.  One barrier, then warp 0 joins the rows cut by the warps' boundaries.
+//
+// Bound by the gathers of x, each a line that L1 has to hold while it is under
+// way: 16.7 M of them at random columns take 67 us by themselves, and what the
+// kernel takes of L1 as shared memory it loses in gathers in flight.  FP32 on the
+// 1M-row power-law matrix (210 MB): block-wide segmented scans, 4 nonzeros per
+// thread, and a last CTA that added all carries 172 us; this 90 us.  The same
+// stream over chunks brought into shared memory by bulk copies 116 us, with
+// windows dealt out through 1.5 KB of it per warp 112 us, 8 warps per CTA 100 us,
+// x a window ahead (64 registers) 107 us.  FP64 203 -> 102 us; equal tiles 16 x 16
+// of the 524,309-row matrix 116 -> 94 us.
+//
+// GROUPS: the planner numbered the rows that items share; otherwise the item's
+// first row goes to y as far as the item has it, and a last row that goes on in
+// the next item to the item's carry slot (carry_fixup adds the carries).
+// ---------------------------------------------------------------------------
+template <typename T, bool GROUPS, bool ATOMIC>
+__device__ __forceinline__ void coo_stream(const Params<T> &P, const Item &it, const T *__restrict__ xb,
+                                           uint32_t item_id) {
+  using A = Acc<T>;
+  constexpr int EB = (int)sizeof(typename ElemOf<T>::type);
+  constexpr int K = sizeof(T) <= 4 ? 4 : 2;  // elements per lane, in whole 16-byte units
+  constexpr int W = K * EB / 4;
+  constexpr uint32_t FULL = 0xffffffffu, WIN = 32 * K;
+  __shared__ StreamEnds<A> ends;
+  T *out = out_base(P, it);
+  const bool staged = it.xw > 0;
+  const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t row_end = it.row_end, row_off = it.row_off;
+  auto write = [&](uint32_t row, A sum) {
+    if (row >= row_end || SP_BAD(P, row < P.nrows, -1015)) return;
+    if constexpr (ATOMIC) atomic_add_out<T>(out + row, sum);
+    else out[row] = from_acc<T>(sum);
+  };
+  // rows r0 + from, r0 + from + step, ... below r1, which have no nonzeros
+  auto zeros = [&](uint32_t r0, uint32_t r1, uint32_t from, uint32_t step) {
+    if (r1 > row_end) r1 = row_end;
+    for (uint64_t r = (uint64_t)r0 + from; r < r1; r += step) write((uint32_t)r, A(0));
+  };
+  if (it.a0 >= it.a1) {  // a tile without nonzeros
+    if (!ATOMIC) zeros(it.own0, it.own1, threadIdx.x, blockDim.x);
+    if (!GROUPS && !ATOMIC && threadIdx.x == 0) P.carry_idx[item_id] = NO_CARRY;
+    return;
+  }
+  // Positions count from the multiple of 4 elements at or before the item's: the
+  // item's are [lead, tn), what lies around them in whole windows counts as
+  // zeros of the rows beside.
+  const uint64_t e0 = it.a0 & ~3ull;
+  const uint64_t lead = it.a0 - e0, tn = it.a1 - e0;
+  const uint64_t per = (tn + nw * WIN - 1) / (nw * WIN) * WIN;
+  const uint64_t begin = warp * per < tn ? warp * per : tn, end = begin + per < tn ? begin + per : tn;
+  const char *el = static_cast<const char *>(P.elems) + e0 * EB;
+  const T *xt = xb + it.col_off;
+  if (begin < end && !SP_BAD(P, it.a1 <= P.n_elems, -1009)) {
+    auto key_at = [&](uint64_t i) { return *reinterpret_cast<const uint32_t *>(el + i * EB); };
+    uint32_t w[W];
+    auto fetch = [&](uint64_t b) {
+      const uint64_t i = b + lane * K;
+      if (i >= tn) return;
+      if (e0 + i + K <= P.n_elems) {
+#pragma unroll
+        for (int q = 0; q < W / 4; ++q) {
+          const uint4 v = ld_stream4(el + i * EB + 16 * q);
+          w[4 * q] = v.x, w[4 * q + 1] = v.y, w[4 * q + 2] = v.z, w[4 * q + 3] = v.w;
+        }
+      } else {  // the last elements of an array without padding
+#pragma unroll
+        for (int q = 0; q < W; ++q)
+          if (i + q * 4 / EB < tn) w[q] = *reinterpret_cast<const uint32_t *>(el + i * EB + 4 * q);
+      }
+    };
+    RowStream<A> S;
+    S.open = key_at(begin > lead ? begin : lead) + row_off;
+    if (lane == 0) ends.k0[warp] = S.open;
+    uint32_t last = S.open;  // the row of the nonzero before the window
+    fetch(begin);
+    for (uint64_t b = begin; b < end; b += WIN) {
+      uint32_t k[K];
+      A v[K];
+      {
+        T x[K], vx[K];
+        const bool edge = b < lead || b + WIN > tn;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          const uint64_t i = b + lane * K + j;
+          bool in = !edge || (i >= lead && i < tn);
+          k[j] = in ? w[j * EB / 4] + row_off : FULL;
+          const uint32_t col = w[j * EB / 4 + 1];
+          vx[j] = in ? word_elem<T>(w + j * EB / 4 + 2, 0) : T(0);
+          if (SP_BAD(P, !in || x_ok(P, it, (uint64_t)it.col_off + col), -1009)) in = false;
+          x[j] = in ? xload(xt, col, staged) : T(0);
+        }
+        if (b + WIN < end) fetch(b + WIN);
+#pragma unroll
+        for (int j = 0; j < K; ++j) v[j] = mul<T>(vx[j], x[j]);
+      }
+      if (b < lead || b + WIN > tn) {
+        const uint32_t tail = key_at(tn - 1) + row_off;
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+          if (k[j] == FULL) k[j] = b + lane * K + j < lead ? last : tail;
+      }
+      uint32_t prev = __shfl_up_sync(FULL, k[K - 1], 1);
+      if (lane == 0) prev = last;
+      uint32_t hb = k[0] != prev ? 1u : 0u, gap = k[0] - prev;
+#pragma unroll
+      for (int j = 1; j < K; ++j) {
+        const uint32_t d = k[j] - k[j - 1];
+        hb |= (d ? 1u : 0u) << j;
+        gap = d > gap ? d : gap;
+      }
+      if constexpr (!ATOMIC) {
+        if (__any_sync(FULL, gap > 1)) {  // rows without nonzeros in between
+          zeros(prev, k[0], 1, 1);
+#pragma unroll
+          for (int j = 1; j < K; ++j) zeros(k[j - 1], k[j], 1, 1);
+        }
+      }
+      last = __shfl_sync(FULL, k[K - 1], 31);
+      row_window<K, A>(S, v, hb, k, &ends.first[warp], write);
+    }
+    leave_ends<A>(ends, warp, S);
+  }
+  __syncthreads();
+  if (warp != 0 || SP_BAD(P, it.a1 <= P.n_elems, -1009)) return;
+  // rows cut by the warps' boundaries, in order (the whole warp follows, lane 0 writes)
+  SharedPart<T> first_part, last_part;
+  if constexpr (GROUPS) {
+    first_part.g = first_row_group(it);
+    last_part.g = last_row_group(it);
+  }
+  uint32_t cur = ends.k0[0];
+  A sum = ends.first[0];
+  bool first = true;  // `cur` is the item's first row
+  auto close = [&]() {
+    if (first && first_part.g.n) {
+      first_part.row0 = cur;
+      first_part.part = sum;
+    } else if (lane == 0) {
+      write(cur, sum);
+    }
+    first = false;
+  };
+  if (!ATOMIC) zeros(it.own0, cur, lane, 32);
+  for (int w = 0; w < nw && w * per < tn; ++w) {
+    if (w) {
+      if (ends.k0[w] == cur) {
+        sum += ends.first[w];
+      } else {
+        close();
+        if (!ATOMIC) zeros(cur, ends.k0[w], lane + 1, 32);
+        cur = ends.k0[w];
+        sum = ends.first[w];
+      }
+    }
+    if (ends.heads[w]) {
+      close();
+      cur = ends.k1[w];
+      sum = ends.last[w];
+    }
+  }
+  if constexpr (GROUPS) {
+    if (last_part.g.n) {  // goes on in the next item
+      if (first) first_part.g.n = 0;  // and came from the one before
+      last_part.row0 = cur;
+      last_part.part = sum;
+    } else {
+      close();
+      if (!ATOMIC) zeros(cur, it.own1, lane + 1, 32);
+    }
+    if (first_part.g.n + last_part.g.n) arrive<T, 1>(P, out, item_id, row_end, first_part, last_part);
+  } else if (ATOMIC || cur < it.own1) {
+    if (lane == 0) {
+      write(cur, sum);
+      if (!ATOMIC) P.carry_idx[item_id] = NO_CARRY;
+    }
+    if (!ATOMIC) zeros(cur, it.own1, lane + 1, 32);
+  } else if (lane == 0) {
+    P.carry_idx[item_id] = cur < row_end ? out_index(P, it, cur) : NO_CARRY;
+    P.carry_val[item_id] = acc_bits(sum);
+  }
+}
+
+template <typename T, bool ATOMIC> __global__ void __launch_bounds__(512) coo_items(Params<T> P) {
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  __shared__ uint64_t xbar;
+  const Item it = P.items[blockIdx.x];
+  const T *xb = P.x;
+  if (it.xw > 0 && it.a0 < it.a1) {
+    uint32_t phase = 0;
+    mbar_init(&xbar);
+    xb = stage_x<T>(P.x, it.xlo, it.xw, dyn_smem, &xbar, phase, P.err, P.smem_bytes,
+                    reinterpret_cast<uintptr_t>(P.x + P.n_xalloc), P.fault_wait);
+  }
+  coo_stream<T, !ATOMIC, ATOMIC>(P, it, xb, blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// BCOO in chunks of up to S blocks (sorted by block row), 2x2, 4x4 and 8x8:
+// values and block indices come into shared memory by bulk copies, the block
+// rows' starts are found there (a ballot per 32 blocks and a scan of the
+// ballots), and then the block rows are summed as BCSR's are.  INT16 4x4, 1M rows,
+// 20 blocks per block row (204 MB): a block per thread and block-wide scans of
+// 4-wide sums 291 us, this 76 us.
+// ---------------------------------------------------------------------------
+template <typename T, int RB, int CB> struct BcooStage {
+  using G = Pieces<T, RB, CB>;
+  static constexpr int S = (int)bcoo_chunk_blocks(RB, CB, sizeof(T));
+  static constexpr int IND = (S + 8) * G::B, RUN = IND + (S + 8) * (int)sizeof(sparsep_bind);
+  static constexpr int SMEM = (RUN + (S + 1) * 4 + 127) / 128 * 128;
+  static_assert(S <= 1024, "a warp scans the chunk's ballots");
+};
+
+template <typename T, int RB, int CB>
+__global__ void __launch_bounds__(512, 3) bcoo_chunks(Params<T> P) {
+  using A = Acc<T>;
+  using G = Pieces<T, RB, CB>;
+  using St = BcooStage<T, RB, CB>;
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  __shared__ uint64_t bar, xbar;
+  __shared__ uint32_t ballots[St::S / 32 + 1];
+  __shared__ A s_first[RB], s_last[RB];
+  unsigned char *sm = dyn_smem + (P.smem_bytes + 127) / 128 * 128;  // behind a tile's staged x
+  const Item it = P.items[blockIdx.x];
+  T *out = out_base(P, it);
+  const bool atomic = P.out_mode == OUT_ATOMIC;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t n = (uint32_t)(it.a1 - it.a0);
+  const uint64_t A0 = it.a0 & ~3ull, A1 = (it.a1 + 3) & ~3ull;  // the arrays are padded past their end
+  const RowGroup ga = first_row_group(it), gb = last_row_group(it);
+  auto row_of = [&](uint64_t key) { return (uint64_t)it.row_off + key * RB; };
+  auto zero_rows = [&](uint64_t r0, uint64_t r1) {  // by the whole CTA
+    if (!atomic)
+      for (uint64_t r = r0 + threadIdx.x; r < r1 && r < it.row_end; r += blockDim.x) put<T>(P, out, r, A(0));
+  };
+  if (n == 0) {
+    zero_rows(row_of(it.own0), row_of(it.own1));
+    return;
+  }
+  bool good = !SP_BAD(P, A1 <= P.n_elems && A1 * (RB * CB) <= P.n_val && n <= St::S, -1014);
+  mbar_init(&bar);
+  if (threadIdx.x == 0 && good) {
+    const uint32_t m = (uint32_t)(A1 - A0);
+    expect_bytes(&bar, m * (uint32_t)(G::B + sizeof(sparsep_bind)));
+    bulk_load(sm + St::IND, P.bind + A0, m * (uint32_t)sizeof(sparsep_bind), &bar);
+    bulk_load(sm, reinterpret_cast<const char *>(P.bval) + A0 * G::B, m * G::B, &bar);
+  }
+  const T *xb = P.x;
+  if (it.xw > 0) {
+    uint32_t phase = 0;
+    mbar_init(&xbar);
+    xb = stage_x<T>(P.x, it.xlo, it.xw, dyn_smem, &xbar, phase, P.err, P.smem_bytes,
+                    reinterpret_cast<uintptr_t>(P.x + P.n_xalloc), P.fault_wait);
+  }
+  if (good) good = cta_wait(&bar, 0, P.err);
+  // parts of the first and last block row that other items share (one and the
+  // same block row counts as the last)
+  SharedPart<T> first_part{ga, 0, A(0)}, last_part{gb, 0, A(0)};
+  if (gb.n && ga.cnt == gb.cnt) first_part.g.n = 0;
+  if (!good) {  // give the item up, but arrive
+    first_part.row0 = row_of(it.own0);
+    last_part.row0 = row_of(it.own1);
+    if (warp == 0 && ga.n + gb.n) arrive<T, RB>(P, out, blockIdx.x, it.row_end, first_part, last_part);
+    return;
+  }
+  const uint32_t lead = (uint32_t)(it.a0 - A0);
+  const sparsep_bind *ind = reinterpret_cast<const sparsep_bind *>(sm + St::IND) + lead;
+  uint32_t *run = reinterpret_cast<uint32_t *>(sm + St::RUN);
+  // block rows' first blocks, in order
+  const uint32_t words = (n + 31) / 32;
+  for (uint32_t b = threadIdx.x; b < words * 32; b += blockDim.x) {
+    const uint32_t m = __ballot_sync(0xffffffffu, b < n && (b == 0 || ind[b].rowind != ind[b - 1].rowind));
+    if (lane == 0) ballots[b / 32] = m;
+  }
+  __syncthreads();
+  const uint32_t mine = lane < words ? ballots[lane] : 0u;
+  uint32_t before = __popc(mine);  // inclusive, then exclusive
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, before, d);
+    if (lane >= d) before += o;
+  }
+  const uint32_t k = __shfl_sync(0xffffffffu, before, 31);  // block rows
+  before -= __popc(mine);
+  for (uint32_t b = threadIdx.x; b < words * 32; b += blockDim.x) {
+    const uint32_t m = __shfl_sync(0xffffffffu, mine, b / 32);
+    const uint32_t at = __shfl_sync(0xffffffffu, before, b / 32);
+    if ((m >> lane) & 1u) run[at + __popc(m & ((1u << lane) - 1u))] = b;
+  }
+  if (threadIdx.x == 0) run[k] = n;
+  __syncthreads();
+  // rows of no block: before the first, between two, after the last block row
+  if (!atomic) {
+    zero_rows(row_of(it.own0), row_of(ind[0].rowind));
+    for (uint32_t i = threadIdx.x + 1; i < k; i += blockDim.x)
+      for (uint64_t r = row_of((uint64_t)ind[run[i] - 1].rowind + 1); r < row_of(ind[run[i]].rowind) && r < it.row_end; ++r)
+        put<T>(P, out, r, A(0));
+    if (!gb.n) zero_rows(row_of((uint64_t)ind[n - 1].rowind + 1), row_of(it.own1));
+  }
+  const T *xt = xb + it.col_off;
+  const uint32_t *scol = &ind[0].colind;
+  const bool whole = x_whole<T, RB, CB, 2>(P, it, xt, scol, n);
+  block_rows_any<T, RB, CB, 2>(P, it, xt, k, run, sm + lead * G::B, scol, it.lanes, whole,
+                               [&](uint32_t i, uint32_t r, A sum) {
+                                 if (i + 1 == k && gb.n) {
+                                   s_last[r] = sum;
+                                 } else if (i == 0 && ga.n) {
+                                   s_first[r] = sum;
+                                 } else {
+                                   const uint64_t row = row_of(ind[run[i]].rowind) + r;
+                                   if (row < it.row_end) put<T>(P, out, row, sum);
+                                 }
+                               });
+  if (!ga.n && !gb.n) return;
+  __syncthreads();
+  if (warp != 0) return;
+  first_part.row0 = row_of(ind[0].rowind);
+  last_part.row0 = row_of(ind[n - 1].rowind);
+  if (lane < RB) first_part.part = s_first[lane], last_part.part = s_last[lane];
+  arrive<T, RB>(P, out, blockIdx.x, it.row_end, first_part, last_part);
+}
+
+// ---------------------------------------------------------------------------
+// BCOO blocks of the other sizes (rb <= BCOO_W): block segmented scan, a block
+// per thread.  Keys are tile-local block rows (row = row_off + key * rb + r).
+// The item writes every row of block rows [own0, own1): sums of complete runs,
+// zeros for block rows without blocks; a run reaching own1 is a carry for the
+// fix-up.
+// ---------------------------------------------------------------------------
+constexpr int BCOO_W = 16;
+
+template <typename T>
+__device__ __forceinline__ void zero_block_rows(const Params<T> &P, const Item &it, T *out, long long k0,
+                                                long long k1) {
   // keys strictly inside (k0, k1)
   for (long long k = k0 + 1; k < k1; ++k)
-    for (uint32_t r = 0; r < (W == 1 ? 1u : rb); ++r) {
-      const uint64_t row = key_row<T, W>(it, k, r, rb);
+    for (uint32_t r = 0; r < P.rb; ++r) {
+      const uint64_t row = (uint64_t)it.row_off + (uint64_t)k * P.rb + r;
       if (row < it.row_end && !SP_BAD(P, row < P.nrows, -1015)) out[row] = T(0);
     }
 }
 
-template <typename T, int W>
+template <typename T>
 __device__ __forceinline__ void write_run(const Params<T> &P, const Item &it, T *out, long long key,
-                                          const Acc<T> (&v)[W], uint32_t rb, bool atomic) {
+                                          const Acc<T> (&v)[BCOO_W], bool atomic) {
 #pragma unroll
-  for (int r = 0; r < W; ++r) {
-    if (r >= (int)rb) break;
-    const uint64_t row = key_row<T, W>(it, key, r, rb);
+  for (int r = 0; r < BCOO_W; ++r) {
+    if (r >= (int)P.rb) break;
+    const uint64_t row = (uint64_t)it.row_off + (uint64_t)key * P.rb + r;
     if (row >= it.row_end) continue;
     if (SP_BAD(P, row < P.nrows, -1015)) continue;
     if (atomic) atomic_add_out<T>(out + row, v[r]);
@@ -869,138 +1329,71 @@ __device__ __forceinline__ void write_run(const Params<T> &P, const Item &it, T 
   }
 }
 
-// Units per thread per chunk: COO 4 elements, BCOO 1 block.
-template <typename T, int W, int RB, int CB>
-__device__ __forceinline__ void load_units(const Params<T> &P, const Item &it, const T *__restrict__ xb,
-                                           uint64_t t0, Unit<T, W> (&u)[W == 1 ? COO_K : 1], uint64_t lo,
-                                           uint64_t hi) {
-  if constexpr (W == 1) {
-    load_coo4<T>(P, it, xb, t0, u, lo, hi);
-  } else {
-    const uint64_t b = t0;
-    const bool ok = b >= lo && b < hi;
-#pragma unroll
-    for (int r = 0; r < W; ++r) u[0].v[r] = Acc<T>(0);
-    u[0].key = LLONG_MAX;
-    if (ok && !SP_BAD(P, b < P.n_elems, -1014)) {
-      const sparsep_bind bi = P.bind[b];
-      u[0].key = (long long)bi.rowind;
-      block_mv<T, RB, CB>(P, xb, b, bi.colind, it.col_off, u[0].v, it);
-    }
-  }
-}
-
-template <typename T, int W, int RB, int CB>
-__device__ void elems_lf(const Params<T> &P, const Item &it, const T *__restrict__ xb, uint32_t item_id,
-                         uint32_t cw) {
-  // cw = carry slots per item (1 for COO, rb for BCOO), the scratch stride
+template <typename T>
+__device__ void bcoo_lf(const Params<T> &P, const Item &it, const T *__restrict__ xb, uint32_t item_id, uint32_t cw) {
+  // cw = carry slots per item (rb), the scratch stride
   using A = Acc<T>;
+  constexpr int W = BCOO_W;
   using KVT = KV<A, W>;
-  constexpr int K = (W == 1) ? COO_K : 1;
   __shared__ KVT scan_smem[32];
   __shared__ KVT tail_smem;
-  __shared__ long long heads_smem[512];
+  __shared__ long long keys_smem[512];
   T *out = out_base(P, it);
-  const uint32_t rb = W == 1 ? 1u : (RB > 0 ? RB : P.rb);
   const uint64_t lo = it.a0, hi = it.a1;
   const bool atomic = P.out_mode == OUT_ATOMIC;
 
   if (SP_BAD(P, (uint64_t)(item_id + 1) * cw <= P.n_carry || atomic, -1018)) return;
   if (lo >= hi) {  // empty: only zero the owned rows
-    if (!atomic && threadIdx.x == 0) zero_rows<T, W>(P, it, out, (long long)it.own0 - 1, it.own1, rb);
+    if (!atomic && threadIdx.x == 0) zero_block_rows<T>(P, it, out, (long long)it.own0 - 1, it.own1);
     if (!atomic && threadIdx.x < cw) P.carry_idx[(uint64_t)item_id * cw + threadIdx.x] = NO_CARRY;
     return;
   }
-  // thread groups: COO aligned 4-element groups, BCOO single blocks
-  const uint64_t g_first = (W == 1) ? lo / 4 : lo;
-  const uint64_t g_last = (W == 1) ? (hi + 3) / 4 : hi;  // exclusive
   KVT carry;
   carry.k = (long long)it.own0 - 1;
 #pragma unroll
   for (int i = 0; i < W; ++i) carry.v[i] = A(0);
 
-  for (uint64_t cg = g_first; cg < g_last; cg += blockDim.x) {
+  for (uint64_t cg = lo; cg < hi; cg += blockDim.x) {
     const uint64_t g = cg + threadIdx.x;
-    Unit<T, W> u[K];
-    if (g < g_last) {
-      load_units<T, W, RB, CB>(P, it, xb, g, u, lo, hi);
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        u[k].key = LLONG_MAX;
-#pragma unroll
-        for (int i = 0; i < W; ++i) u[k].v[i] = A(0);
-      }
-    }
-    // thread-local runs
-    long long head = LLONG_MAX, tail = LLONG_MAX;
-    A head_acc[W], run[W];
-#pragma unroll
-    for (int i = 0; i < W; ++i) head_acc[i] = run[i] = A(0);
-    bool first = true, any = false;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (u[k].key == LLONG_MAX) continue;
-      if (!any) {
-        head = tail = u[k].key;
-        any = true;
-      } else if (u[k].key != tail) {
-        if (first) {
-#pragma unroll
-          for (int i = 0; i < W; ++i) head_acc[i] = run[i];
-          first = false;
-        } else {
-          write_run<T, W>(P, it, out, tail, run, rb, atomic);
-        }
-        if (!atomic) zero_rows<T, W>(P, it, out, tail, u[k].key, rb);
-        tail = u[k].key;
-#pragma unroll
-        for (int i = 0; i < W; ++i) run[i] = A(0);
-      }
-#pragma unroll
-      for (int i = 0; i < W; ++i) run[i] += u[k].v[i];
-    }
     KVT mine;
-    mine.k = tail;
+    mine.k = LLONG_MAX;
 #pragma unroll
-    for (int i = 0; i < W; ++i) mine.v[i] = run[i];
-    heads_smem[threadIdx.x] = any ? head : LLONG_MAX;  // read after the scan's barriers
+    for (int i = 0; i < W; ++i) mine.v[i] = A(0);
+    if (g < hi && !SP_BAD(P, g < P.n_elems, -1014)) {
+      const sparsep_bind bi = P.bind[g];
+      mine.k = (long long)bi.rowind;
+      block_mv<T, 0, 0>(P, xb, g, bi.colind, it.col_off, mine.v, it);
+    }
+    const bool any = mine.k != LLONG_MAX;
+    keys_smem[threadIdx.x] = mine.k;  // read after the scan's barriers
     KVT ex, in;
     block_seg_scan<A, W>(mine, carry, ex, in, scan_smem);
-    const uint64_t last_g = (g_last < cg + blockDim.x ? g_last : cg + blockDim.x) - 1;
-    // a tail run is complete when the next thread starts another key; the
-    // chunk's last thread hands its tail on instead
-    if (any && g != last_g && heads_smem[threadIdx.x + 1] != tail) write_run<T, W>(P, it, out, tail, in.v, rb, atomic);
+    const uint64_t last_g = (hi < cg + blockDim.x ? hi : cg + blockDim.x) - 1;
+    // a run is complete when the next thread starts another key; the chunk's
+    // last thread hands its run on instead
+    if (any && g != last_g && keys_smem[threadIdx.x + 1] != mine.k) write_run<T>(P, it, out, mine.k, in.v, atomic);
     // likewise the run handed over by the previous chunk
-    if (threadIdx.x == 0 && carry.k >= (long long)it.own0 && head != carry.k)
-      write_run<T, W>(P, it, out, carry.k, carry.v, rb, atomic);
-    if (any) {
-      if (!atomic) zero_rows<T, W>(P, it, out, ex.k, head, rb);
-      if (head != tail) {
-        A h[W];
-#pragma unroll
-        for (int i = 0; i < W; ++i) h[i] = head_acc[i] + (ex.k == head ? ex.v[i] : A(0));
-        write_run<T, W>(P, it, out, head, h, rb, atomic);
-      }
-    }
-    // the chunk's last thread with units hands its tail to the next chunk
+    if (threadIdx.x == 0 && carry.k >= (long long)it.own0 && mine.k != carry.k)
+      write_run<T>(P, it, out, carry.k, carry.v, atomic);
+    if (any && !atomic) zero_block_rows<T>(P, it, out, ex.k, mine.k);
+    // the chunk's last thread with a block hands its run to the next chunk
     if (g == last_g) tail_smem = in;
     __syncthreads();
     carry = tail_smem;
     __syncthreads();
   }
-  // final tail of the item
+  // final run of the item
   if (threadIdx.x == 0) {
     if (atomic) {
-      write_run<T, W>(P, it, out, carry.k, carry.v, rb, true);
+      write_run<T>(P, it, out, carry.k, carry.v, true);
     } else if (carry.k < (long long)it.own1) {
-      write_run<T, W>(P, it, out, carry.k, carry.v, rb, false);
-      zero_rows<T, W>(P, it, out, carry.k, it.own1, rb);
+      write_run<T>(P, it, out, carry.k, carry.v, false);
+      zero_block_rows<T>(P, it, out, carry.k, it.own1);
       for (uint32_t i = 0; i < cw; ++i) P.carry_idx[(uint64_t)item_id * cw + i] = NO_CARRY;
     } else {
       for (uint32_t i = 0; i < cw && i < (uint32_t)W; ++i) {
-        const uint64_t row = key_row<T, W>(it, carry.k, i, rb);
-        const bool ok = i < rb && row < it.row_end;
+        const uint64_t row = (uint64_t)it.row_off + (uint64_t)carry.k * P.rb + i;
+        const bool ok = i < P.rb && row < it.row_end;
         P.carry_idx[(uint64_t)item_id * cw + i] = ok ? out_index(P, it, row) : NO_CARRY;
         P.carry_val[(uint64_t)item_id * cw + i] = acc_bits(carry.v[i]);
       }
@@ -1015,17 +1408,29 @@ __device__ void elems_lf(const Params<T> &P, const Item &it, const T *__restrict
 template <typename T>
 __device__ void carry_fixup(const Params<T> &P, uint32_t nslots, uint32_t W) {
   using A = Acc<T>;
-  for (uint32_t s = threadIdx.x; s < nslots; s += blockDim.x) {
-    const unsigned long long idx = __ldcg(P.carry_idx + s);
-    if (idx == NO_CARRY) continue;
-    if (SP_BAD(P, idx < (uint64_t)P.nslots * P.nrows, -1016)) continue;
-    if (s >= W && __ldcg(P.carry_idx + s - W) == idx) continue;  // not the first of its run
-    A sum = bits_acc<A>(__ldcg(P.carry_val + s));
-    for (uint32_t t = s + W; t < nslots && __ldcg(P.carry_idx + t) == idx; t += W)
-      sum += bits_acc<A>(__ldcg(P.carry_val + t));
-    T *p = (P.out_mode == OUT_PARTIAL ? P.part : P.y) + idx;
-    T cur = __ldcg(p);
-    *p = from_acc<T>(to_acc<T>(cur) + sum);
+  constexpr int U = 4;  // slots a thread reads in one round trip
+  for (uint32_t s0 = threadIdx.x; s0 < nslots; s0 += U * blockDim.x) {
+    unsigned long long idx[U], prev[U], val[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t s = s0 + u * blockDim.x;
+      const bool in = s < nslots;
+      idx[u] = in ? __ldcg(P.carry_idx + s) : NO_CARRY;
+      prev[u] = in && s >= W ? __ldcg(P.carry_idx + s - W) : NO_CARRY;
+      val[u] = in ? __ldcg(P.carry_val + s) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t s = s0 + u * blockDim.x;
+      if (idx[u] == NO_CARRY || prev[u] == idx[u]) continue;  // none, or not the first of its run
+      if (SP_BAD(P, idx[u] < (uint64_t)P.nslots * P.nrows, -1016)) continue;
+      A sum = bits_acc<A>(val[u]);
+      for (uint32_t t = s + W; t < nslots && __ldcg(P.carry_idx + t) == idx[u]; t += W)
+        sum += bits_acc<A>(__ldcg(P.carry_val + t));
+      T *p = (P.out_mode == OUT_PARTIAL ? P.part : P.y) + idx[u];
+      T cur = __ldcg(p);
+      *p = from_acc<T>(to_acc<T>(cur) + sum);
+    }
   }
 }
 
@@ -1061,8 +1466,6 @@ __global__ void __launch_bounds__(512) spmv_items(Params<T> P, uint32_t carry_w)
         default: csr_rows<T, 32>(P, it, xb); break;
       }
     }
-  } else if constexpr (FMT == SPARSEP_FMT_COO) {
-    elems_lf<T, 1, 0, 0>(P, it, xb, item_id, carry_w);
   } else if constexpr (FMT == SPARSEP_FMT_BCSR) {
     switch (it.lanes) {
       case 1: bcsr_rows<T, RB, CB, 1>(P, it, xb); break;
@@ -1073,7 +1476,7 @@ __global__ void __launch_bounds__(512) spmv_items(Params<T> P, uint32_t carry_w)
       default: bcsr_rows<T, RB, CB, 32>(P, it, xb); break;
     }
   } else {
-    elems_lf<T, (RB > 0 ? RB : 16), RB, CB>(P, it, xb, item_id, carry_w);
+    bcoo_lf<T>(P, it, xb, item_id, carry_w);
   }
 
   // lock-free carries: the last CTA to finish adds them (threadfence reduction)

@@ -13,7 +13,7 @@
 // The scratch is a file-scope __device__ array of MAX_ITEMS carry slots
 // (16 bytes each, about 1 MB); every GPU that loads the library holds it until
 // the process exits.  Calls share it, so calls that overlap on the GPU race.
-// Each call derives its work items from blockIdx (4096 nonzeros each), so no
+// Each call derives its work items from blockIdx (coo_item_elems each), so no
 // plan or item table is needed either.
 #include <cstring>
 #include <mutex>
@@ -25,20 +25,21 @@
 namespace sparsep {
 namespace noalloc {
 
-constexpr uint32_t ELEMS_PER_ITEM = 4096;
 constexpr uint32_t MAX_ITEMS = 1u << 16;  // nonzeros <= 2^28 (one carry slot per item)
 
 // [0, MAX_ITEMS): carry values, [MAX_ITEMS, 2*MAX_ITEMS): carry targets,
 // [2*MAX_ITEMS]: completion counter
 static __device__ __align__(256) unsigned long long g_scratch[2 * MAX_ITEMS + 2];
 
-__global__ void __launch_bounds__(256) coo_f32(Params<float> P, uint64_t nnz) {
+constexpr int THREADS = 128;  // as the plans' default
+
+__global__ void __launch_bounds__(THREADS) coo_f32(Params<float> P, uint64_t nnz, uint32_t item) {
   __shared__ uint32_t is_last;
   const uint32_t k = blockIdx.x;
   const auto *el = reinterpret_cast<const sparsep_elem_f32 *>(P.elems);
   Item it;
-  it.a0 = (uint64_t)k * ELEMS_PER_ITEM;
-  it.a1 = it.a0 + ELEMS_PER_ITEM < nnz ? it.a0 + ELEMS_PER_ITEM : nnz;
+  it.a0 = (uint64_t)k * item;
+  it.a1 = it.a0 + item < nnz ? it.a0 + item : nnz;
   it.ptr_base = it.nnz_base = 0;
   it.row_off = it.col_off = 0;
   // item k owns the rows from its first nonzero's row to the next item's first
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(256) coo_f32(Params<float> P, uint64_t nnz) {
   it.kind = ITEM_ELEMS;
   it.lanes = 0;
   it.row_end = P.nrows;
-  elems_lf<float, 1, 0, 0>(P, it, P.x, k, 1);
+  coo_stream<float, false, false>(P, it, P.x, k);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -107,7 +108,8 @@ extern "C" int sparsep_spmv_cooe_f32_noalloc(const sparsep_elem_f32 *d_elems, ui
                                              uint32_t ncols, const float *d_x, float *d_y, void *stream) {
   if (!d_x || !d_y || (nnz && !d_elems)) return SPARSEP_EINVAL;
   if ((reinterpret_cast<uintptr_t>(d_elems) & 15) != 0) return SPARSEP_EINVAL;  // 16-byte vector loads
-  const uint64_t nitems = ((uint64_t)nnz + noalloc::ELEMS_PER_ITEM - 1) / noalloc::ELEMS_PER_ITEM;
+  const uint32_t item = coo_item_elems(nnz);
+  const uint64_t nitems = ((uint64_t)nnz + item - 1) / item;
   if (nitems > noalloc::MAX_ITEMS) return SPARSEP_ERANGE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int dev = 0;
@@ -153,6 +155,6 @@ extern "C" int sparsep_spmv_cooe_f32_noalloc(const sparsep_elem_f32 *d_elems, ui
   P.n_xalloc = ncols;
   P.n_carry = nitems;
   P.nslots = 1;
-  noalloc::coo_f32<<<(unsigned)nitems, 256, 0, st>>>(P, nnz);
+  noalloc::coo_f32<<<(unsigned)nitems, noalloc::THREADS, 0, st>>>(P, nnz, item);
   return noalloc_status(cudaGetLastError());
 }

@@ -68,7 +68,9 @@ struct sparsep_plan {
   unsigned int *band_cnt = nullptr;       // device counters: items finished, over all host calls
   uint32_t band_calls = 0;                // host calls whose kernel was launched (mod 2^32)
   cudaStream_t copy_stream = nullptr;
-  unsigned int *row_cnt = nullptr;  // long-row arrival counters (pipelined CSR)
+  unsigned int *row_cnt = nullptr;  // arrival counters: long CSR rows, rows shared by COO / BCOO items
+  uint32_t ngroups = 0;             // rows shared by COO / BCOO items
+  bool by_groups = false;           // COO / BCOO items join shared rows by those, not by a carry fix-up
   uint64_t n_rowptr = 0, n_idx = 0, n_val = 0, n_elems = 0;  // allocated extents
   bool stage = false;
   bool pipe = false;  // 1D CSR auto items run on the pipelined persistent kernel
@@ -172,13 +174,13 @@ static uint32_t pow2ceil(uint64_t v) {
 static constexpr uint64_t AUTO_ITEM_NNZ = 4080;
 static constexpr uint64_t AUTO_ITEM_ROWS = 1024;
 static constexpr uint64_t AUTO_LONG_CHUNK = 4096;
-static constexpr uint64_t AUTO_ITEM_ELEMS = 4096;
 static constexpr uint64_t AUTO_ITEM_ENTRIES = 8192;  // stored block entries per item
 static constexpr size_t STAGE_AUTO_MAX = 96 * 1024;
 static constexpr size_t STAGE_MAX = 200 * 1024;
-// The BCSR chunk kernel holds a chunk (up to 43 KB) beside a staged x, and x is
-// staged for it only where that is asked for: its x comes in vector loads.
-static constexpr size_t STAGE_MAX_BCSR = 176 * 1024;
+// The chunk kernels (BCSR and BCOO of the common block sizes) hold a chunk (up to
+// 46 KB) beside a staged x, which they stage only where that is asked for: it
+// comes in vector loads.
+static constexpr size_t STAGE_MAX_CHUNKS = 176 * 1024;
 
 struct Opts {
   sparsep_opts o;
@@ -300,13 +302,16 @@ static void number_long_rows(std::vector<Item> &items) {
 // from its first unit's key to the next item's first key.
 template <typename KeyFn>
 static void elem_tile_items(std::vector<Item> &items, const Tile &t, uint64_t e0, uint64_t e1, uint32_t k_lo,
-                            uint32_t k_hi, const std::vector<uint64_t> &cuts_in, KeyFn key) {
-  std::vector<uint64_t> cuts = cuts_in;  // boundaries inside (e0, e1), sorted
-  std::vector<uint64_t> b;
+                            uint32_t k_hi, const std::vector<uint64_t> &cuts_in, uint64_t cap, const KeyFn &key) {
+  std::vector<uint64_t> b;  // boundaries: the cuts inside (e0, e1), and every cap units in between
   b.push_back(e0);
-  for (uint64_t c : cuts)
-    if (c > e0 && c < e1) b.push_back(c);
-  b.push_back(e1);
+  auto upto = [&](uint64_t c) {
+    while (cap && c - b.back() > cap) b.push_back(b.back() + cap);
+    b.push_back(c);
+  };
+  for (uint64_t c : cuts_in)
+    if (c > b.back() && c < e1) upto(c);
+  upto(e1);
   for (size_t i = 0; i + 1 < b.size(); ++i) {
     Item it = make_item(t, ITEM_ELEMS);
     it.a0 = b[i];
@@ -316,6 +321,54 @@ static void elem_tile_items(std::vector<Item> &items, const Tile &t, uint64_t e0
     if (it.own1 < it.own0) it.own1 = it.own0;
     items.push_back(it);
   }
+}
+
+// Numbers the rows (keys) that consecutive items of one tile share, from group
+// `ngroups` on: items [first, items.size()) are the tile's (RowGroup in
+// kernels_impl.cuh).
+template <typename KeyFn>
+static void group_shared_rows(std::vector<Item> &items, size_t first, uint32_t &ngroups, const KeyFn &key) {
+  const size_t n = items.size();
+  auto shared = [&](size_t i) {  // item i's last row goes on in item i + 1
+    return i + 1 < n && items[i].a0 < items[i].a1 && items[i + 1].a0 < items[i + 1].a1 &&
+           key(items[i].a1 - 1) == key(items[i + 1].a0);
+  };
+  for (size_t i = first; i + 1 < n;) {
+    if (!shared(i)) {
+      ++i;
+      continue;
+    }
+    size_t l = i + 1;  // the row's last item
+    while (key(items[l].a0) == key(items[l].a1 - 1) && shared(l)) ++l;
+    const uint32_t g = ngroups++, f = (uint32_t)i, cnt = (uint32_t)(l - i + 1);
+    for (size_t k = i; k < l; ++k) {  // goes on in the next item
+      items[k].chunk = g;
+      items[k].crow = f;
+      items[k].n1 = cnt;
+    }
+    for (size_t k = i + 1; k <= l; ++k) {  // came from the one before
+      items[k].cslot = g;
+      items[k].first = f;
+      items[k].nchunk = cnt;
+    }
+    i = l;
+  }
+}
+
+// Blocks of a block row that a chunk's lanes take at a time, for block rows of m
+// blocks: about an eighth of them, so that a warp works on several block rows at
+// once and its last step is nearly full.
+static uint32_t chunk_lanes(uint64_t m) {
+  uint32_t l = 1;
+  while (l < 8 && l * 2 <= (m + 4) / 8) l *= 2;
+  return l;
+}
+
+// Blocks per BCOO item: a chunk, less where that leaves SMs idle.
+static uint64_t bcoo_item_blocks(uint32_t rb, uint32_t cb, size_t es, uint64_t nblocks) {
+  const uint64_t S = bcoo_chunk_blocks(rb, cb, es);
+  if (!S) return std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb));
+  return std::min<uint64_t>(S, std::max<uint64_t>(32, (nblocks / 592 + 3) & ~3ull));
 }
 
 static std::vector<uint64_t> even_cuts(uint64_t e0, uint64_t e1, uint64_t per) {
@@ -411,12 +464,15 @@ static int finish_plan(sparsep_plan *p, std::vector<Item> &items, const sparsep_
     p->info.scratch_bytes += b;
   }
   if (p->carry_w) {
-    size_t n = (size_t)p->nitems * p->carry_w + 1;
+    size_t n = (size_t)p->nitems * p->carry_w * (p->by_groups ? 2 : 1) + 1;
     st = dalloc(p, n * 8, (void **)&p->carry_val);
-    if (!st) st = dalloc(p, n * 8, (void **)&p->carry_idx);
-    if (!st) st = dalloc(p, 16, (void **)&p->done);
+    p->info.scratch_bytes += n * 8;
+    if (!st && !p->by_groups) {
+      st = dalloc(p, n * 8, (void **)&p->carry_idx);
+      if (!st) st = dalloc(p, 16, (void **)&p->done);
+      p->info.scratch_bytes += n * 8 + 16;
+    }
     if (st) return st;
-    p->info.scratch_bytes += n * 16 + 16;
   }
   st = dalloc(p, 16, (void **)&p->err);
   if (st) return st;
@@ -426,7 +482,7 @@ static int finish_plan(sparsep_plan *p, std::vector<Item> &items, const sparsep_
     if (st) return st;
     CK(cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking));
   }
-  uint32_t nlong = 0;
+  uint32_t nlong = p->ngroups;
   for (const Item &it : items) nlong += it.kind == ITEM_LONG && it.chunk == 0;
   if (nlong) {
     st = dalloc(p, (size_t)nlong * 4, (void **)&p->row_cnt);
@@ -442,7 +498,10 @@ static int finish_plan(sparsep_plan *p, std::vector<Item> &items, const sparsep_
     }
   }
   p->smem = smem;
-  int workers = o.nr_workers > 0 ? o.nr_workers : 8;
+  // 4 warps per CTA, for more CTAs on an SM out of step with each other, where an
+  // item is small and brings no x of its own
+  const bool small = p->format == SPARSEP_FMT_COO && !p->stage && p->nnz <= 4096ull * p->nitems;
+  int workers = o.nr_workers > 0 ? o.nr_workers : small ? 4 : 8;
   p->threads = 32 * workers;
   for (auto &e : p->ev) CK(cudaEventCreate(&e));
   p->info.dtype = p->dtype;
@@ -515,10 +574,14 @@ static int begin_plan(sparsep_plan **out, int dtype, int format, int scheme, con
 
 static int stage_width(const sparsep_plan *p, const sparsep_opts &o, uint32_t w) {
   size_t bytes = (size_t)w * p->esize + 32;
-  const bool chunks = p->format == SPARSEP_FMT_BCSR && bcsr_chunk_blocks(p->rb, p->cb, p->esize);
+  size_t most = STAGE_MAX, most_auto = STAGE_AUTO_MAX;
+  if ((p->format == SPARSEP_FMT_BCSR && bcsr_chunk_blocks(p->rb, p->cb, p->esize)) ||
+             (p->format == SPARSEP_FMT_BCOO && bcoo_chunk_blocks(p->rb, p->cb, p->esize))) {
+    most = STAGE_MAX_CHUNKS;
+    most_auto = 0;
+  }
   if (o.stage_x == 0 || w == 0) return 0;
-  if (o.stage_x > 0) return bytes <= (chunks ? STAGE_MAX_BCSR : STAGE_MAX) ? (int)w : 0;
-  return !chunks && bytes <= STAGE_AUTO_MAX ? (int)w : 0;
+  return bytes <= (o.stage_x > 0 ? most : most_auto) ? (int)w : 0;
 }
 
 static uint64_t compulsory_csr(uint64_t nnz, uint64_t nrows, uint64_t ncols, size_t s) {
@@ -1050,7 +1113,7 @@ struct ElemTile {
 template <typename T>
 static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint64_t nnz, uint64_t nunits,
                       uint32_t V, const void *elems, size_t elem_size, const std::vector<ElemTile> &tiles,
-                      std::function<uint32_t(uint64_t)> key, uint64_t per_item, const sparsep_opts *o,
+                      const std::function<uint32_t(uint64_t)> &key, uint64_t per_item, const sparsep_opts *o,
                       sparsep_plan **out, const typename Types<T>::bcoo *B = nullptr, uint32_t rb = 1,
                       uint32_t cb = 1) {
   sparsep_plan *p = nullptr;
@@ -1066,15 +1129,27 @@ static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint6
   p->cb = cb;
   std::vector<Item> items;
   const bool faithful = oo.nr_parts > 0;
+  // COO, and BCOO in chunks of at most `cap` blocks: shared rows are numbered;
+  // the general BCOO kernel leaves carries
+  const uint64_t cap = fmt == SPARSEP_FMT_COO ? 0 : bcoo_chunk_blocks(rb, cb, sizeof(T));
+  p->by_groups = fmt == SPARSEP_FMT_COO || cap != 0;
+  uint64_t nparts = 0;
+  set_out_mode(p, oo, V, true, fmt == SPARSEP_FMT_BCOO ? rb : 1);
   for (const ElemTile &et : tiles) {
     Tile t = et.t;
     t.xw = stage_width(p, oo, t.xw);
     std::vector<uint64_t> cuts = et.cuts;
     if (!faithful) cuts = even_cuts(et.e0, et.e1, per_item);
-    elem_tile_items(items, t, et.e0, et.e1, et.k_lo, et.k_hi, cuts, key);
+    for (uint64_t c : cuts) nparts += c > et.e0 && c < et.e1;
+    ++nparts;
+    const size_t first = items.size();
+    elem_tile_items(items, t, et.e0, et.e1, et.k_lo, et.k_hi, cuts, cap, key);
+    if (p->by_groups && p->out_mode != OUT_ATOMIC) group_shared_rows(items, first, p->ngroups, key);
   }
-  const uint32_t W = fmt == SPARSEP_FMT_BCOO ? rb : 1;
-  set_out_mode(p, oo, V, true, W);
+  if (cap) {
+    const uint32_t m = (uint32_t)std::min<uint64_t>(nunits * rb / (std::max<uint64_t>(1, nrows) * V), UINT32_MAX);
+    for (Item &it : items) it.lanes = (uint16_t)(oo.lanes ? (uint32_t)oo.lanes : chunk_lanes(m));
+  }
   if (fmt == SPARSEP_FMT_COO) {
     if ((st = upload(p, elems, nunits, elem_size, 8, &p->elems))) return st;
     p->n_elems = nunits + 8;
@@ -1089,6 +1164,7 @@ static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint6
                                (uint64_t)nrows * sizeof(T);
   }
   if ((st = finish_plan(p, items, oo))) return st;
+  if (faithful) p->info.items = nparts;
   p->t[0] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   *out = guard.release();
   return SPARSEP_OK;
@@ -1152,7 +1228,7 @@ static int plan_cooe(const typename Types<T>::cooe *A, const sparsep_opts *o, sp
   }
   std::vector<ElemTile> tiles{et};
   return plan_elems<T>(SPARSEP_FMT_COO, SPARSEP_1D, A->nrows, A->ncols, A->nnz, A->nnz, 1, A->nnzs, sizeof(E), tiles,
-                       [el](uint64_t u) { return el[u].rowind; }, AUTO_ITEM_ELEMS, o, out);
+                       [el](uint64_t u) { return el[u].rowind; }, coo_item_elems(A->nnz), o, out);
 }
 
 // SoA COO (the CSR-family reader's output, in file order): sorted into the
@@ -1223,7 +1299,7 @@ static int plan_dcoo(const typename Types<T>::dcoo *A, const sparsep_opts *o, sp
     for (uint64_t n = et.e0; n < et.e1; ++n) roff[n] = et.t.row_off;
   auto key = [el, r = std::move(roff)](uint64_t u) { return el[u].rowind + r[u]; };
   return plan_elems<T>(SPARSEP_FMT_COO, SPARSEP_2D_EQUAL, A->nrows, A->ncols, A->nnz, A->nnz, V, A->nnzs, sizeof(E),
-                       tiles, key, AUTO_ITEM_ELEMS, &oo, out);
+                       tiles, key, coo_item_elems(A->nnz), &oo, out);
 }
 
 template <typename T, typename S>
@@ -1266,7 +1342,7 @@ static int plan_stripes_coo(int scheme, const S *A, const uint32_t *widths, cons
   if (o2.nr_parts == 0) {
     // GPU sizing, but never coarser than the reference's H parts per stripe
     for (auto &et : tiles) {
-      auto extra = even_cuts(et.e0, et.e1, AUTO_ITEM_ELEMS);
+      auto extra = even_cuts(et.e0, et.e1, coo_item_elems(A->nnz));
       et.cuts.insert(et.cuts.end(), extra.begin(), extra.end());
       std::sort(et.cuts.begin(), et.cuts.end());
       et.cuts.erase(std::unique(et.cuts.begin(), et.cuts.end()), et.cuts.end());
@@ -1274,7 +1350,7 @@ static int plan_stripes_coo(int scheme, const S *A, const uint32_t *widths, cons
     o2.nr_parts = 1;  // cuts are final
   }
   return plan_elems<T>(SPARSEP_FMT_COO, scheme, A->nrows, A->ncols, A->nnz, A->nnz, V, A->nnzs, sizeof(E), tiles,
-                       [el](uint64_t u) { return el[u].rowind; }, AUTO_ITEM_ELEMS, &o2, out);
+                       [el](uint64_t u) { return el[u].rowind; }, coo_item_elems(A->nnz), &o2, out);
 }
 
 template <typename T>
@@ -1316,14 +1392,6 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
   const bool faithful = oo.nr_parts > 0;
   uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb)), nparts = 0;
   const uint64_t S = bcsr_chunk_blocks(rb, cb, sizeof(T));
-  // Blocks of a block row that a chunk's lanes take at a time: about an eighth
-  // of them, so that a warp works on several block rows at once and its last
-  // step is nearly full.
-  auto chunk_lanes = [](uint64_t m) -> uint32_t {
-    uint32_t l = 1;
-    while (l < 8 && l * 2 <= (m + 4) / 8) l *= 2;
-    return l;
-  };
   uint64_t rcap = UINT64_MAX;
   if (S) {
     per = std::min<uint64_t>(S, std::max<uint64_t>(32, nblocks / (4 * (uint64_t)p->sms)));
@@ -1553,7 +1621,7 @@ static int plan_bcoo(const typename Types<T>::bcoo *A, const sparsep_opts *o, sp
                                  ob.part_balance == SPARSEP_BAL_NNZ_ELEM ? wp : std::vector<uint64_t>{});
   }
   const uint32_t rb = (uint32_t)A->row_block_size, cb = (uint32_t)A->col_block_size;
-  uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb));
+  uint64_t per = bcoo_item_blocks(rb, cb, sizeof(T), A->num_blocks);
   return plan_elems<T>(SPARSEP_FMT_BCOO, SPARSEP_1D, A->nrows, A->ncols, A->nnz, A->num_blocks, 1, nullptr, 0, {et},
                        [bi](uint64_t u) { return bi[u].rowind; }, per, &oo, out, A, rb, cb);
 }
@@ -1599,7 +1667,7 @@ static int plan_tiles_bcoo(int scheme, const S *A, uint32_t ntiles, const uint32
   B.bind = A->bind;
   B.bval = A->bval;
   sparsep_opts o2 = oo;
-  uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb));
+  uint64_t per = bcoo_item_blocks(rb, cb, sizeof(T), A->nblocks);
   if (o2.nr_parts == 0) {
     for (auto &et : tiles) {
       auto extra = even_cuts(et.e0, et.e1, per);
@@ -1696,8 +1764,9 @@ static int run_t(sparsep_plan *p, const void *d_x, void *d_y, cudaStream_t s, un
   P.part = static_cast<T *>(p->part);
   P.out_mode = p->out_mode;
   P.carry_val = p->carry_w ? p->carry_val : nullptr;
-  // CSR long rows complete through per-row counters; the carry list and the
-  // last-CTA fix-up serve the element-wise (COO / BCOO) formats
+  // CSR long rows and the rows shared by COO / BCOO chunks complete through
+  // per-row counters; the carry list and the last-CTA fix-up serve the BCOO
+  // block sizes without chunks
   P.carry_idx = (p->carry_w && p->format != SPARSEP_FMT_CSR) ? p->carry_idx : nullptr;
   P.done = p->done;
   P.row_cnt = p->row_cnt;
@@ -1709,7 +1778,7 @@ static int run_t(sparsep_plan *p, const void *d_x, void *d_y, cudaStream_t s, un
   P.n_elems = p->n_elems;
   P.n_x = p->ncols;
   P.n_xalloc = x == p->xpad ? (uint64_t)p->ncols + 64 : p->ncols;  // staging reads into the slack
-  P.n_carry = p->carry_w ? (uint64_t)p->nitems * p->carry_w + 1 : 0;
+  P.n_carry = p->carry_w ? (uint64_t)p->nitems * p->carry_w * (p->by_groups ? 2 : 1) + 1 : 0;
   P.nslots = p->out_mode == OUT_PARTIAL ? p->V : 1;
   P.smem_bytes = (uint32_t)p->smem;
   P.fault_wait = wait_fault();

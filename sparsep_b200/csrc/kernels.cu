@@ -29,11 +29,11 @@ static cudaError_t allow_smem(K *k, std::atomic<int> (&configured)[64], size_t s
   return cudaSuccess;
 }
 
-template <typename T, int FMT, int RB, int CB>
+template <typename T, int FMT, int RB, int CB, int CAP = 0>
 static cudaError_t launch_t(const Params<T> &P, uint32_t carry_w, int threads, size_t smem, cudaStream_t st) {
   static std::atomic<int> configured[64];
-  if (cudaError_t e = allow_smem(spmv_items<T, FMT, RB, CB>, configured, smem)) return e;
-  spmv_items<T, FMT, RB, CB><<<P.nitems, threads, smem, st>>>(P, carry_w);
+  if (cudaError_t e = allow_smem(spmv_items<T, FMT, RB, CB, CAP>, configured, smem)) return e;
+  spmv_items<T, FMT, RB, CB, CAP><<<P.nitems, threads, smem, st>>>(P, carry_w);
   return cudaGetLastError();
 }
 
@@ -68,12 +68,14 @@ static cudaError_t launch_coo(const Params<T> &P, int threads, size_t smem, cuda
 }
 
 template <typename T>
-cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int threads, size_t smem,
+cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int threads, size_t smem, bool slim,
                          cudaStream_t st) {
   if (P.nitems == 0) return cudaSuccess;
   const uint32_t rb = P.rb, cb = P.cb;
   switch (fmt) {
-    case SPARSEP_FMT_CSR: return launch_t<T, SPARSEP_FMT_CSR, 0, 0>(P, carry_w, threads, smem, st);
+    case SPARSEP_FMT_CSR:
+      return slim ? launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), true)>(P, carry_w, threads, smem, st)
+                  : launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), false)>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_COO:
       return P.out_mode == OUT_ATOMIC ? launch_coo<T, true>(P, threads, smem, st)
                                       : launch_coo<T, false>(P, threads, smem, st);
@@ -106,7 +108,7 @@ cudaError_t launch_merge(const T *part, T *y, uint32_t nrows, uint32_t V, int sm
 #ifndef SPARSEP_KT
 #define SPARSEP_KT float
 #endif
-template cudaError_t launch_items<SPARSEP_KT>(const Params<SPARSEP_KT> &, int, uint32_t, int, size_t, cudaStream_t);
+template cudaError_t launch_items<SPARSEP_KT>(const Params<SPARSEP_KT> &, int, uint32_t, int, size_t, bool, cudaStream_t);
 template cudaError_t launch_merge<SPARSEP_KT>(const SPARSEP_KT *, SPARSEP_KT *, uint32_t, uint32_t, int, cudaStream_t);
 
 }  // namespace sparsep

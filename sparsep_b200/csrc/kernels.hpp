@@ -7,9 +7,10 @@
 namespace sparsep {
 
 // Launch the work-item kernel for format `fmt` (sparsep_format) with one CTA
-// per item.  carry_w = carry slots per item (1 for CSR/COO, rb for BCOO).
+// per item.  carry_w = carry slots per item (1 for CSR/COO, rb for BCOO); slim:
+// CSR items of at most csr_chunk_nnz(.., true) nonzeros.
 template <typename T>
-cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int threads, size_t smem,
+cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int threads, size_t smem, bool slim,
                          cudaStream_t st);
 
 // y[r] = sum over the V partial slices of row r, in slice order.
@@ -28,6 +29,16 @@ constexpr uint32_t bcsr_chunk_blocks(uint32_t rb, uint32_t cb, size_t es) {
 }
 // block rows per chunk
 constexpr uint32_t BCSR_CHUNK_ROWS = 512;
+
+// Nonzeros whose products the CSR row kernel holds in shared memory at a time (and
+// a quarter as many rows): 8 KB of them in the slim form, 16 KB in the wide one.
+// A gather of x holds a line of L1 while it is under way, and shared memory is
+// taken from L1: with 32 KB of FP64 products per CTA the gathers stood in line
+// (1M-row power-law matrix, FP64 188 us; 16 KB 107 us; 8 KB and 4 warps per CTA 93
+// us; FP32 with 16 KB 87 us, 8 KB and 4 warps 83.5 us).  Automatic items are slim;
+// parts and tiles, whose items are the caller's, keep the wide form (2048 parts of
+// the FP32 matrix: 8192 nonzeros each).
+constexpr int csr_chunk_nnz(size_t es, bool slim) { return (slim ? 8192 : 16384) / (es == 8 ? 8 : 4); }
 
 // Nonzeros per automatic COO item: 4096, fewer where that leaves less than six
 // items per SM (1.5 M nonzeros, FP32: 20 us in 366 items, 16.5 us in 733; 16.7 M:

@@ -235,28 +235,15 @@ template <typename A> __device__ __forceinline__ void leave_ends(StreamEnds<A> &
 
 // ---------------------------------------------------------------------------
 // CSR rows, staged ("stream") form used when lanes = auto.  A chunk of up to
-// CSR_RCAP rows / CSR_CAP nonzeros is moved in three coalesced sweeps: its
-// rowptr slice into shared memory, then every nonzero (128-bit loads of colind
+// CSR_CAP nonzeros and a quarter as many rows is moved in three coalesced sweeps:
+// its rowptr slice into shared memory, then every nonzero (128-bit loads of colind
 // and values) times its gathered x into a shared product array; rows are then
 // summed from shared memory (a thread per short row, a warp per long row) and
 // written with consecutive threads on consecutive rows.  A row longer than the
 // chunk capacity is reduced by the whole CTA straight from global memory.
+// Bound by the gathers (see csr_chunk_nnz for what CSR_CAP costs them).
 // ---------------------------------------------------------------------------
-// x gathers each thread keeps in flight in the chunk's product pass: 4 x this.
-// On the 1M-row Zipf FP32 matrix: 1 (40 registers, 6 CTAs/SM) 93.2 us; 2 (62
-// registers, 4 CTAs/SM) 99.4 us -- occupancy buys more than depth here.
-#ifndef SPARSEP_CSR_GATHER
-#define SPARSEP_CSR_GATHER 1
-#endif
-#ifndef SPARSEP_CSR_CAP
-#define SPARSEP_CSR_CAP 4096
-#endif
-#ifndef SPARSEP_CSR_SHORT
-#define SPARSEP_CSR_SHORT 48
-#endif
-constexpr int CSR_CAP = SPARSEP_CSR_CAP;      // nonzeros per chunk
-constexpr int CSR_RCAP = 1024;                // rows per chunk
-constexpr int CSR_SHORT = SPARSEP_CSR_SHORT;  // rows up to this length are summed by one thread
+constexpr int CSR_SHORT = 48;  // rows up to this length are summed by one thread
 
 // sum of a[s, e) x over the whole CTA (thread 0 gets the total)
 template <typename T>
@@ -286,12 +273,13 @@ __device__ Acc<T> cta_range_sum(const Params<T> &P, const Item &it, const T *__r
   return tot;
 }
 
-template <typename T>
+template <typename T, int CSR_CAP>
 __device__ void csr_stream(const Params<T> &P, const Item &it, const T *__restrict__ xb) {
   using A = Acc<T>;
+  constexpr int CSR_RCAP = CSR_CAP / 4;  // rows per chunk
   __shared__ A prods[CSR_CAP];
   __shared__ uint32_t srp[CSR_RCAP + 1];
-  __shared__ uint32_t longs[CSR_RCAP];
+  __shared__ uint16_t longs[CSR_RCAP];
   __shared__ uint32_t nlong;
   __shared__ A red[32];
   T *out = out_base(P, it);
@@ -324,44 +312,25 @@ __device__ void csr_stream(const Params<T> &P, const Item &it, const T *__restri
       continue;
     }
     const uint64_t s0 = (uint64_t)base + it.nnz_base, e0 = (uint64_t)srp[k] + it.nnz_base;
-    // R groups of 4 nonzeros per thread per pass: their index and value loads,
-    // then all 4R x gathers in flight at once, then the products
-    constexpr int R = SPARSEP_CSR_GATHER;
-    for (uint64_t g0 = (s0 >> 2) + threadIdx.x; 4 * g0 < e0; g0 += (uint64_t)R * blockDim.x) {
-      uint32_t cc[R][4];
-      Vec4<T> v4[R];
-      bool live[R];
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const uint64_t j = 4 * (g0 + (uint64_t)i * blockDim.x);
-        live[i] = j < e0 && !SP_BAD(P, j + 3 < P.n_idx && j + 3 < P.n_val, -1002);
-        if (live[i]) {
-          const uint4 c4 = ld_stream4(P.colind + j);
-          v4[i] = ld_vals4<T>(P.val + j);
-          cc[i][0] = c4.x, cc[i][1] = c4.y, cc[i][2] = c4.z, cc[i][3] = c4.w;
-        }
-      }
-      T xv[R][4];
+    // per thread and pass 4 nonzeros: their index and value loads, then all x
+    // gathers in flight at once, then the products
+    for (uint64_t j = (s0 & ~3ull) + 4 * threadIdx.x; j < e0; j += 4 * blockDim.x) {
+      if (SP_BAD(P, j + 3 < P.n_idx && j + 3 < P.n_val, -1002)) break;
+      const uint4 c4 = ld_stream4(P.colind + j);
+      const Vec4<T> v4 = ld_vals4<T>(P.val + j);
+      const uint32_t cc[4] = {c4.x, c4.y, c4.z, c4.w};
+      T xv[4];
       uint32_t bad = 0;
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint64_t j = 4 * (g0 + (uint64_t)i * blockDim.x) + q;
-          if (live[i] && j >= s0 && j < e0) {
-            const uint64_t col = (uint64_t)it.col_off + cc[i][q];
-            if (SP_BAD(P, x_ok(P, it, col), -1003)) bad |= 1u << (4 * i + q);
-            else xv[i][q] = xload(xb, col, staged);
-          }
+      for (int q = 0; q < 4; ++q)
+        if (j + q >= s0 && j + q < e0) {
+          const uint64_t col = (uint64_t)it.col_off + cc[q];
+          if (SP_BAD(P, x_ok(P, it, col), -1003)) bad |= 1u << q;
+          else xv[q] = xload(xb, col, staged);
         }
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint64_t j = 4 * (g0 + (uint64_t)i * blockDim.x) + q;
-          if (live[i] && j >= s0 && j < e0)
-            prods[j - s0] = (bad >> (4 * i + q)) & 1u ? A(0) : mul<T>(v4[i].v[q], xv[i][q]);
-        }
+      for (int q = 0; q < 4; ++q)
+        if (j + q >= s0 && j + q < e0) prods[j + q - s0] = (bad >> q) & 1u ? A(0) : mul<T>(v4.v[q], xv[q]);
     }
     __syncthreads();
     // short rows: one thread each; long rows are queued for the warps
@@ -372,7 +341,7 @@ __device__ void csr_stream(const Params<T> &P, const Item &it, const T *__restri
         for (uint32_t q = a; q < b; ++q) acc += prods[q];
         put<T>(P, out, it.row_off + r + i, acc);
       } else {
-        longs[atomicAdd(&nlong, 1u)] = i;
+        longs[atomicAdd(&nlong, 1u)] = (uint16_t)i;
       }
     }
     __syncthreads();
@@ -1437,7 +1406,7 @@ __device__ void carry_fixup(const Params<T> &P, uint32_t nslots, uint32_t W) {
 // ---------------------------------------------------------------------------
 // The item kernel
 // ---------------------------------------------------------------------------
-template <typename T, int FMT, int RB, int CB>
+template <typename T, int FMT, int RB, int CB, int CAP>
 __global__ void __launch_bounds__(512) spmv_items(Params<T> P, uint32_t carry_w) {
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   __shared__ uint64_t mbar;
@@ -1457,7 +1426,7 @@ __global__ void __launch_bounds__(512) spmv_items(Params<T> P, uint32_t carry_w)
       csr_long<T>(P, it, xb, item_id);
     } else {
       switch (it.lanes) {
-        case 0: csr_stream<T>(P, it, xb); break;
+        case 0: csr_stream<T, CAP>(P, it, xb); break;
         case 1: csr_rows<T, 1>(P, it, xb); break;
         case 2: csr_rows<T, 2>(P, it, xb); break;
         case 4: csr_rows<T, 4>(P, it, xb); break;

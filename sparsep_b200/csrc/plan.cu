@@ -74,6 +74,7 @@ struct sparsep_plan {
   uint64_t n_rowptr = 0, n_idx = 0, n_val = 0, n_elems = 0;  // allocated extents
   bool stage = false;
   bool pipe = false;  // 1D CSR auto items run on the pipelined persistent kernel
+  bool slim = false;  // CSR items of the row kernel's slim form
   int pipe_grid = 0;
   uint32_t max_item_nnz = 0;
   cudaStream_t stream = nullptr;
@@ -229,12 +230,13 @@ static Item make_item(const Tile &t, uint16_t kind) {
 // item; otherwise split by nnz, with rows longer than AUTO_ITEM_NNZ chunked
 // into LONG items when allow_long.
 static void csr_tile_items(std::vector<Item> &items, const Tile &t, const uint32_t *rp, uint64_t r0, uint64_t r1,
-                           const sparsep_opts &o, bool faithful, bool allow_long) {
-  // item size: <= AUTO_ITEM_NNZ nonzeros, or the option's target rounded to a
-  // stage size (2048 or 4096) less the 16 slots of copy alignment
-  const uint64_t ITEM_NNZ = (o.item_nnz > 0 && o.item_nnz <= 2048) ? 2032 : AUTO_ITEM_NNZ;
-  const uint64_t ROWS_CAP = ITEM_NNZ <= 2032 ? 512 : AUTO_ITEM_ROWS;
-  const uint64_t LONG_CHUNK = ITEM_NNZ <= 2032 ? 2048 : AUTO_LONG_CHUNK;
+                           const sparsep_opts &o, bool faithful, bool allow_long, uint64_t slim = 0,
+                           uint64_t slim_rows = 0) {
+  // item size: the slim form's, or <= AUTO_ITEM_NNZ nonzeros, or the option's
+  // target rounded to a stage size (2048 or 4096) less the 16 slots of copy alignment
+  const uint64_t ITEM_NNZ = slim ? slim : (o.item_nnz > 0 && o.item_nnz <= 2048) ? 2032 : AUTO_ITEM_NNZ;
+  const uint64_t ROWS_CAP = slim ? slim_rows : ITEM_NNZ <= 2032 ? 512 : AUTO_ITEM_ROWS;
+  const uint64_t LONG_CHUNK = slim || ITEM_NNZ <= 2032 ? 2048 : AUTO_LONG_CHUNK;
   auto emit = [&](uint64_t a, uint64_t b) {
     if (a >= b) return;
     Item it = make_item(t, ITEM_ROWS);
@@ -362,6 +364,13 @@ static uint32_t chunk_lanes(uint64_t m) {
   uint32_t l = 1;
   while (l < 8 && l * 2 <= (m + 4) / 8) l *= 2;
   return l;
+}
+
+// Nonzeros per automatic CSR item: what the slim form holds at a time, less (down
+// to two per thread) where that leaves SMs idle: 4096 rows of 8 nonzeros run as
+// 128 items instead of 16.
+static uint64_t csr_item_nnz(size_t es, uint64_t nnz, int sms) {
+  return std::min<uint64_t>(csr_chunk_nnz(es, true), std::max<uint64_t>(256, (nnz / (4 * (uint64_t)sms) + 3) & ~3ull));
 }
 
 // Blocks per BCOO item: a chunk, less where that leaves SMs idle.
@@ -500,7 +509,7 @@ static int finish_plan(sparsep_plan *p, std::vector<Item> &items, const sparsep_
   p->smem = smem;
   // 4 warps per CTA, for more CTAs on an SM out of step with each other, where an
   // item is small and brings no x of its own
-  const bool small = p->format == SPARSEP_FMT_COO && !p->stage && p->nnz <= 4096ull * p->nitems;
+  const bool small = p->slim || (p->format == SPARSEP_FMT_COO && !p->stage && p->nnz <= 4096ull * p->nitems);
   int workers = o.nr_workers > 0 ? o.nr_workers : small ? 4 : 8;
   p->threads = 32 * workers;
   for (auto &e : p->ev) CK(cudaEventCreate(&e));
@@ -951,7 +960,10 @@ static int plan_csr(const typename Types<T>::csr *A, const sparsep_opts *o, spar
         return SPARSEP_OK;
       }
     }
-    csr_tile_items(items, t, A->rowptr, 0, A->nrows, oo, false, true);
+    // the slim form of the row kernel for automatic items
+    p->slim = oo.lanes == 0 && oo.pipeline != 1 && oo.item_nnz <= 0;
+    csr_tile_items(items, t, A->rowptr, 0, A->nrows, oo, false, true, p->slim ? csr_item_nnz(sizeof(T), A->nnz, p->sms) : 0,
+                   csr_chunk_nnz(sizeof(T), true) / 4);
     number_long_rows(items);
     for (auto &it : items) has_long |= it.kind == ITEM_LONG;
   }
@@ -1814,7 +1826,7 @@ static int run_t(sparsep_plan *p, const void *d_x, void *d_y, cudaStream_t s, un
     return SPARSEP_OK;
   }
   if (p->pipe) CK(launch_csr_pipe<T>(P, p->sms, s, &p->pipe_grid, p->max_item_nnz));
-  else CK(launch_items<T>(P, p->format, p->carry_w, p->threads, p->smem, s));
+  else CK(launch_items<T>(P, p->format, p->carry_w, p->threads, p->smem, p->slim, s));
   if (p->out_mode == OUT_PARTIAL) {
     CK(cudaEventRecord(p->ev[2], s));
     CK(launch_merge<T>(static_cast<const T *>(p->part), static_cast<T *>(d_y), p->nrows, p->V, p->sms, s));

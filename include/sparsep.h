@@ -587,7 +587,7 @@ int sparsep_batch_item_kinds(const sparsep_batch *b, uint64_t *window_items, uin
 /* d_rows / d_cols / d_vals: nnz device entries in any order; d_rowptr:
  * nrows + 1, d_colind / d_vals_out: nnz.  Rows ascending, input order kept
  * inside a row (stable).  EINVAL if a row index is >= nrows.  Allocates its
- * own scratch (16 bytes per nonzero); synchronises the stream. */
+ * own scratch (20 to 36 bytes per nonzero); synchronises the stream. */
 #define SPARSEP_DECLARE_C2C(T, S)                                                                               \
   int sparsep_coo2csr_device_##S(const uint32_t *d_rows, const uint32_t *d_cols, const T *d_vals, uint32_t nnz, \
                                  uint32_t nrows, uint32_t *d_rowptr, uint32_t *d_colind, T *d_vals_out,         \
@@ -617,9 +617,8 @@ SPARSEP_DECLARE_PLAN_DEVICE(double, f64)
 /* spmv/1D/BCSR-nnz/support/matrix.h:202-485, csr2bcsr + sortBCSRMatrix +   */
 /* countNNZperBlockBCSRMatrix)                                              */
 /* ------------------------------------------------------------------------ */
-/* Two steps.  sparsep_bcsr_layout_device sorts the nonzeros of a device CSR
- * (rowptr nrows + 1, colind nnz) into rb x cb blocks and returns the block
- * count; EINVAL for a malformed rowptr or a column >= ncols.  The fill then
+/* Two steps.  sparsep_bcsr_layout_device finds the rb x cb blocks of a device
+ * CSR (rowptr nrows + 1, colind nnz) and returns the block count; EINVAL for a malformed rowptr or a column >= ncols.  The fill then
  * writes caller-allocated device arrays: browptr[ceil(nrows/rb) + 1],
  * bcolind[nblocks], bval[nblocks * rb * cb] (row-major blocks, blocks of a
  * block row by ascending block column, a later duplicate entry overwrites an

@@ -3,10 +3,11 @@
 // spmv/1D/CSR-row/support/matrix.h:113-152) produces: rows in order, and
 // inside a row the input order kept (a stable sort by row).
 //
-// Stable LSD radix sort (radix.cuh) of (row, input index) pairs, 4 bits per
-// pass, only as many passes as the row count needs (20 bits -> 5 passes for
-// 1M rows).  Then rowptr[r] = first sorted position with row >= r (a binary search per
-// row), and columns / values are gathered through the sorted input indices.
+// Stable LSD radix sort (radix.cuh) of (row, column, value) records, only as many
+// passes as the row count needs (20 bits -> 3 passes for 1M rows); the last pass
+// writes the columns and values where they belong, so nothing is gathered
+// afterwards.  Then rowptr[r] = first sorted position with row >= r (a binary
+// search per row).
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -33,21 +34,16 @@ __global__ void rowptr_kernel(const uint32_t *__restrict__ key, uint32_t n, uint
   rowptr[r] = lo;
 }
 
-template <int ES>
-__global__ void gather(const uint32_t *__restrict__ idx, uint32_t n, const uint32_t *__restrict__ cols,
-                       const unsigned char *__restrict__ vals, uint32_t *__restrict__ cols_out,
-                       unsigned char *__restrict__ vals_out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t s = idx[i];
-    cols_out[i] = cols[s];
-    for (int b = 0; b < ES; ++b) vals_out[(size_t)i * ES + b] = vals[(size_t)s * ES + b];
-  }
-}
-
 }  // namespace c2c
 }  // namespace sparsep
 
 using namespace sparsep::c2c;
+
+template <size_t N> struct UintOf;
+template <> struct UintOf<1> { using type = uint8_t; };
+template <> struct UintOf<2> { using type = uint16_t; };
+template <> struct UintOf<4> { using type = uint32_t; };
+template <> struct UintOf<8> { using type = unsigned long long; };
 
 static int c2c_err(cudaError_t e) {
   if (e == cudaSuccess) return SPARSEP_OK;
@@ -57,51 +53,56 @@ static int c2c_err(cudaError_t e) {
   return e == cudaErrorMemoryAllocation ? SPARSEP_ENOMEM : SPARSEP_EIO;
 }
 
-// Device COO (rows, cols, vals of es bytes each) -> device CSR.
-static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const void *vals, size_t es, uint32_t nnz,
-                          uint32_t nrows, uint32_t *rowptr, uint32_t *colind, void *vals_out, cudaStream_t s) {
+// Device COO (rows, cols, vals) -> device CSR, V an unsigned type of the values' size.
+template <typename V>
+static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *vals, uint32_t nnz, uint32_t nrows,
+                          uint32_t *rowptr, uint32_t *colind, V *vals_out, cudaStream_t s) {
+  using namespace sparsep::radix;
   if (!rowptr || nrows == 0xFFFFFFFFu || (nnz && (!rows || !cols || !vals || !colind || !vals_out)))
     return SPARSEP_EINVAL;
   int bits = 0;
   while (bits < 32 && (nrows - 1) >> bits) ++bits;  // bits of the largest row index
   if (nrows <= 1) bits = 0;
-  uint32_t *buf = nullptr;
-  int *bad = nullptr;
-  const size_t words = 2 * (size_t)nnz + sparsep::radix::radix_scratch_words(nnz);
-  int st = c2c_err(sparsep::dev_malloc((void **)&buf, words * 4));
-  if (!st) st = c2c_err(sparsep::dev_malloc((void **)&bad, sizeof(int)));
-  if (st) {
-    sparsep::dev_free(buf);
-    sparsep::dev_free(bad);
-    return st;
-  }
-  const uint32_t *key = nullptr, *idx = nullptr;
-  int h_bad = 0;
-  st = c2c_err(cudaMemsetAsync(bad, 0, sizeof(int), s));
-  if (!st)
-    st = c2c_err(sparsep::radix::radix_sort<uint32_t>(rows, nnz, bits, buf, buf + nnz, buf + 2 * (size_t)nnz, &key,
-                                                        &idx, s, bad, nrows));
-  if (!st) st = c2c_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
-  if (!st) st = c2c_err(cudaStreamSynchronize(s));
-  if (!st && h_bad) st = SPARSEP_EINVAL;  // a row index >= nrows
-  if (!st) {
-    rowptr_kernel<<<(nrows + 1 + 255) / 256, 256, 0, s>>>(nnz ? key : nullptr, nnz, nrows, rowptr);
-    if (nnz) {
-      const unsigned grid = (unsigned)std::min<uint32_t>(4096, (nnz + 255) / 256);
-      const auto *v = static_cast<const unsigned char *>(vals);
-      auto *vo = static_cast<unsigned char *>(vals_out);
-      switch (es) {
-        case 1: gather<1><<<grid, 256, 0, s>>>(idx, nnz, cols, v, colind, vo); break;
-        case 2: gather<2><<<grid, 256, 0, s>>>(idx, nnz, cols, v, colind, vo); break;
-        case 4: gather<4><<<grid, 256, 0, s>>>(idx, nnz, cols, v, colind, vo); break;
-        default: gather<8><<<grid, 256, 0, s>>>(idx, nnz, cols, v, colind, vo); break;
+  const int np = passes(bits);
+  // records of the passes before the last (two sets at most), the last pass's
+  // keys in a set that is free by then, the digit counts, a flag
+  const size_t n = nnz, sets = np > 2 ? 2 : 1, vb = ((n * sizeof(V)) + 15) & ~(size_t)15;
+  const size_t kb = ((n * 4) + 15) & ~(size_t)15, set = 2 * kb + vb;
+  unsigned char *buf = nullptr;
+  int st = c2c_err(sparsep::ws_malloc((void **)&buf, sets * set + kb + count_words(nnz) * 4 + 64, s));
+  if (st) return st;
+  auto key_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set); };
+  auto col_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set + kb); };
+  auto val_of = [&](size_t q) { return reinterpret_cast<V *>(buf + q * set + 2 * kb); };
+  uint32_t *last_key = reinterpret_cast<uint32_t *>(buf + sets * set);
+  uint32_t *counts = reinterpret_cast<uint32_t *>(buf + sets * set + kb);
+  int *bad = reinterpret_cast<int *>(counts + count_words(nnz));
+  const uint32_t *key = rows, *col = cols;
+  const V *val = vals;
+  if (nnz) {
+    int h_bad = 0;
+    st = c2c_err(cudaMemsetAsync(bad, 0, sizeof(int), s));
+    for (int p = 0, shift = 0; !st && p < np; shift += pass_bits(bits, p, np), ++p) {
+      const int b = pass_bits(bits, p, np);
+      const bool last = p + 1 == np;
+      uint32_t *ko = last ? last_key : key_of(p % 2), *co = last ? colind : col_of(p % 2);
+      V *vo = last ? vals_out : val_of(p % 2);
+      st = c2c_err(count_pass<uint32_t>(key, nnz, shift, b, counts, s, p ? nullptr : bad, nrows));
+      if (!st && p == 0) {  // nothing of the outputs is written for a row index >= nrows
+        st = c2c_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+        if (!st) st = c2c_err(cudaStreamSynchronize(s));
+        if (!st && h_bad) st = SPARSEP_EINVAL;
       }
+      if (!st) st = c2c_err(scatter_pass<uint32_t, V>(key, col, val, nnz, shift, b, counts, ko, co, vo, s));
+      key = ko, col = co, val = vo;
     }
-    st = c2c_err(cudaGetLastError());
-    if (!st) st = c2c_err(cudaStreamSynchronize(s));
   }
-  sparsep::dev_free(buf);
-  sparsep::dev_free(bad);
+  if (!st) {
+    rowptr_kernel<<<(nrows + 1 + 255) / 256, 256, 0, s>>>(key, nnz, nrows, rowptr);
+    st = c2c_err(cudaGetLastError());
+  }
+  sparsep::ws_free(buf, s);
+  if (!st) st = c2c_err(cudaStreamSynchronize(s));
   return st;
 }
 
@@ -109,8 +110,9 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const void
   int sparsep_coo2csr_device_##S(const uint32_t *d_rows, const uint32_t *d_cols, const T *d_vals, uint32_t nnz, \
                                  uint32_t nrows, uint32_t *d_rowptr, uint32_t *d_colind, T *d_vals_out,         \
                                  void *stream) {                                                                \
-    return coo2csr_device(d_rows, d_cols, d_vals, sizeof(T), nnz, nrows, d_rowptr, d_colind, d_vals_out,       \
-                          static_cast<cudaStream_t>(stream));                                                   \
+    using V = UintOf<sizeof(T)>::type;                                                                          \
+    return coo2csr_device<V>(d_rows, d_cols, reinterpret_cast<const V *>(d_vals), nnz, nrows, d_rowptr,         \
+                             d_colind, reinterpret_cast<V *>(d_vals_out), static_cast<cudaStream_t>(stream));   \
   }
 
 extern "C" {

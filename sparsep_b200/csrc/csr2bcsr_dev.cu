@@ -6,17 +6,28 @@
 // duplicate entry of a position overwrites an earlier one, and
 // nnz_per_block[b] = the block's entries != 0.
 //
+// A block row's nonzeros are consecutive in the CSR, so nothing is sorted
+// globally: a warp takes a block row and finds its block columns with a hash table
+// in shared memory.
 // layout (type-independent, sparsep_bcsr_layout_device):
+//   count  per block row, its distinct block columns; rowptr and columns checked
+//   scan   of the counts -> browptr
+// fill (per element type, sparsep_csr2bcsr_device_<t>):
+//   the block columns again, ranked; the blocks put together in shared memory
+//   where they fit (else in place), 32 nonzeros at a time in input order, so that
+//   a later duplicate of a position overwrites an earlier one; the nonzero values
+//   of each block counted.
+// Matrices with a block row of more than LIM_LARGE nonzeros go through a sort of
+// all nonzeros by (block row, block column) instead (radix.cuh):
 //   keys   per nonzero k: its row r (binary search in rowptr) and the key
-//          (r / rb) << jbits | colind[k] / cb; rowptr and columns checked
-//   sort   stable radix sort of the keys (radix.cuh) carrying k, so that the
-//          entries of one block stay in input order
+//          (r / rb) << jbits | colind[k] / cb
+//   sort   stable, carrying k, so that the entries of one block stay in input order
 //   heads  a block starts where the sorted key changes: exclusive scan of the
 //          head flags -> block start positions and block keys
-// fill (per element type, sparsep_csr2bcsr_device_<t>):
-//   browptr  lower bound of each block row among the block keys
-//   blocks   one thread per block: zero it, write its entries in input order,
-//            count the nonzero values; bcolind from the key
+//   fill   browptr by lower bound among the block keys, one thread per block
+// FP32, 10.5 M nonzeros in 1 M blocks of 4x4 (COO -> CSR -> BCSR as one ingest): 8.1
+// ms with the sort for every matrix and scratch from cudaMalloc, of which 1.9 ms in
+// kernels.
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -38,6 +49,217 @@ __global__ void check_rowptr(const uint32_t *__restrict__ rowptr, uint32_t nrows
   if (blockIdx.x == 0 && threadIdx.x == 0 && (rowptr[0] != 0 || rowptr[nrows] != nnz)) atomicExch(bad, 1);
 }
 
+// ---------------------------------------------------------------------------
+// A block row per warp
+// ---------------------------------------------------------------------------
+constexpr int LIM_SMALL = 256, LIM_LARGE = 2048;  // nonzeros of a block row
+constexpr uint32_t EMPTY = 0xFFFFFFFFu;           // no block column: columns are below 2^32 - 1
+template <int LIM> struct Table {
+  static constexpr int SLOTS = 2 * LIM;
+  static constexpr int WARPS = LIM == LIM_SMALL ? 4 : 1;  // block rows per CTA
+  static constexpr int BLOCKS = LIM == LIM_SMALL ? 2048 : 8192;  // bytes for a block row's blocks
+};
+
+struct BlockRow {
+  uint32_t r0, k0, k1;  // first row, nonzeros [k0, k1)
+};
+// Block row I of a CSR whose rowptr may be malformed (checked elsewhere): ranges
+// stay inside the arrays.
+__device__ __forceinline__ BlockRow block_row(const uint32_t *__restrict__ rowptr, uint32_t nrows, uint32_t nnz,
+                                              uint32_t rb, uint32_t I) {
+  const uint64_t r0 = (uint64_t)I * rb, r1 = r0 + rb < nrows ? r0 + rb : nrows;
+  BlockRow b;
+  b.r0 = (uint32_t)r0;
+  b.k0 = rowptr[r0] < nnz ? rowptr[r0] : nnz;
+  b.k1 = rowptr[r1] < nnz ? rowptr[r1] : nnz;
+  if (b.k1 < b.k0) b.k1 = b.k0;
+  return b;
+}
+__device__ __forceinline__ uint32_t block_col(uint32_t c, uint32_t cb, int cshift) {
+  return cshift >= 0 ? c >> cshift : c / cb;
+}
+// Slots used of a table for m nonzeros (a power of two, at least 2 m), as a shift
+// of the 32-bit hash.
+__device__ __forceinline__ int table_shift(uint32_t m) { return m <= 16 ? 27 : __clz(2 * m - 1); }
+__device__ __forceinline__ uint32_t hash(uint32_t J, int shift) { return (J * 0x9E3779B1u) >> shift; }
+// The slot of J; *fresh: it was not there before.
+__device__ __forceinline__ uint32_t insert(uint32_t *t, uint32_t J, int shift, bool *fresh) {
+  const uint32_t mask = (1u << (32 - shift)) - 1u;
+  for (uint32_t s = hash(J, shift);; s = (s + 1) & mask) {  // at least half of the slots stay empty
+    const uint32_t old = atomicCAS(t + s, EMPTY, J);
+    if (old == EMPTY || old == J) {
+      *fresh = old == EMPTY;
+      return s;
+    }
+  }
+}
+__device__ __forceinline__ uint32_t find(const uint32_t *t, uint32_t J, int shift) {  // J is in the table
+  const uint32_t mask = (1u << (32 - shift)) - 1u;
+  uint32_t s = hash(J, shift);
+  for (uint32_t i = 0; i < mask && t[s] != J; ++i) s = (s + 1) & mask;
+  return s;
+}
+// Calls f(I) with the whole warp for the block rows I of (lo, LIM] nonzeros: a warp
+// per block row for the many short ones, 32 looked over at a time for the few long ones.
+template <int LIM, typename F>
+__device__ __forceinline__ void each_block_row(const uint32_t *__restrict__ rowptr, uint32_t nrows, uint32_t nnz,
+                                               uint32_t rb, uint32_t nbr, uint32_t lo, F f) {
+  constexpr uint32_t W = Table<LIM>::WARPS;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr (LIM == LIM_SMALL) {
+    for (uint64_t I = (uint64_t)blockIdx.x * W + warp; I < nbr; I += (uint64_t)gridDim.x * W) f((uint32_t)I);
+  } else {
+    for (uint64_t I0 = ((uint64_t)blockIdx.x * W + warp) * 32; I0 < nbr; I0 += (uint64_t)gridDim.x * W * 32) {
+      uint32_t m = 0;
+      if (I0 + lane < nbr) {
+        const BlockRow b = block_row(rowptr, nrows, nnz, rb, (uint32_t)(I0 + lane));
+        m = b.k1 - b.k0;
+      }
+      for (uint32_t some = __ballot_sync(0xffffffffu, m > lo && m <= LIM); some; some &= some - 1)
+        f((uint32_t)I0 + __ffs(some) - 1);
+    }
+  }
+}
+
+// cnt[I] = blocks of block row I, for block rows of (lo, LIM] nonzeros (and the
+// empty ones); flag[0]: a bad column, flag[1]: a longer block row.
+template <int LIM>
+__global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
+    count_blocks(const uint32_t *__restrict__ rowptr, uint32_t nrows, const uint32_t *__restrict__ colind, uint32_t nnz,
+                 uint32_t ncols, uint32_t rb, uint32_t cb, int cshift, uint32_t nbr, uint32_t lo,
+                 uint32_t *__restrict__ cnt, int *__restrict__ flag) {
+  using Tb = Table<LIM>;
+  __shared__ uint32_t table[Tb::WARPS][Tb::SLOTS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  each_block_row<LIM>(rowptr, nrows, nnz, rb, nbr, lo, [&](uint32_t I) {
+    const BlockRow br = block_row(rowptr, nrows, nnz, rb, I);
+    const uint32_t m = br.k1 - br.k0;
+    if (m > LIM_LARGE && lane == 0) flag[1] = 1;
+    if (m == 0 && lane == 0) cnt[I] = 0;
+    if (m <= lo || m > LIM) return;
+    const int shift = table_shift(m);
+    uint32_t *t = table[warp];
+    for (uint32_t i = lane; i < 1u << (32 - shift); i += 32) t[i] = EMPTY;
+    __syncwarp();
+    uint32_t mine = 0;
+    for (uint32_t k = br.k0 + lane; k < br.k1; k += 32) {
+      uint32_t c = colind[k];
+      if (c >= ncols) {
+        flag[0] = 1;
+        c = 0;
+      }
+      bool fresh;
+      insert(t, block_col(c, cb, cshift), shift, &fresh);
+      mine += fresh;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) cnt[I] = mine;
+    __syncwarp();
+  });
+}
+
+template <typename T, int LIM>
+__global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
+    fill_rows(const uint32_t *__restrict__ rowptr, uint32_t nrows, const uint32_t *__restrict__ colind, uint32_t nnz,
+              uint32_t ncols, const T *__restrict__ values, uint32_t rb, uint32_t cb, int cshift, uint32_t nbr,
+              uint32_t lo, const uint32_t *__restrict__ browptr, uint32_t *__restrict__ bcolind, T *__restrict__ bval,
+              uint32_t *__restrict__ nnz_per_block) {
+  using Tb = Table<LIM>;
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ uint32_t table[Tb::WARPS][Tb::SLOTS];
+  __shared__ uint16_t rank_of[Tb::WARPS][Tb::SLOTS];
+  __shared__ uint32_t list[Tb::WARPS][LIM];
+  __shared__ uint32_t count[Tb::WARPS];
+  __shared__ __align__(16) unsigned char blocks[Tb::WARPS][Tb::BLOCKS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t *t = table[warp], *l = list[warp];
+  uint16_t *rk = rank_of[warp];
+  const uint64_t bs = (uint64_t)rb * cb;
+  each_block_row<LIM>(rowptr, nrows, nnz, rb, nbr, lo, [&](uint32_t I) {
+    const BlockRow br = block_row(rowptr, nrows, nnz, rb, I);
+    const uint32_t m = br.k1 - br.k0;
+    if (m <= lo || m > LIM) return;
+    const int shift = table_shift(m);
+    for (uint32_t i = lane; i < 1u << (32 - shift); i += 32) t[i] = EMPTY;
+    if (lane == 0) count[warp] = 0;
+    __syncwarp();
+    for (uint32_t k = br.k0 + lane; k < br.k1; k += 32) {
+      const uint32_t c = colind[k], J = block_col(c < ncols ? c : 0, cb, cshift);
+      bool fresh;
+      insert(t, J, shift, &fresh);
+      if (fresh) l[atomicAdd(&count[warp], 1u)] = J;
+    }
+    __syncwarp();
+    const uint32_t b0 = browptr[I], room = browptr[I + 1] - b0;
+    const uint32_t D = count[warp] < room ? count[warp] : room;  // equal, while colind is as it was counted
+    for (uint32_t d = lane; d < D; d += 32) {
+      const uint32_t J = l[d];
+      uint32_t r = 0;
+      for (uint32_t e = 0; e < D; ++e) r += l[e] < J;
+      rk[find(t, J, shift)] = (uint16_t)r;
+      if (r < room) bcolind[b0 + r] = J;
+    }
+    __syncwarp();
+    // the blocks: in shared memory where they fit, else where they belong
+    T *gout = bval + b0 * bs;
+    const uint64_t ne = D * bs;
+    const bool in_smem = ne * sizeof(T) <= (uint64_t)Tb::BLOCKS;
+    T *blk = in_smem ? reinterpret_cast<T *>(blocks[warp]) : gout;
+    for (uint64_t e = lane; e < ne; e += 32) blk[e] = T(0);
+    // ends of the block row's rows, one per lane
+    const uint32_t rend = lane < rb && br.r0 + lane + 1 <= nrows ? rowptr[br.r0 + lane + 1] : 0xFFFFFFFFu;
+    __syncwarp();
+    for (uint32_t k = br.k0; k < br.k1; k += 32) {  // input order: a later duplicate wins
+      const bool in = k + lane < br.k1;
+      uint32_t rl = 0;  // row in the block: the block row's rows that end at or before this nonzero
+      if (rb <= 32) {
+        for (uint32_t q = 0; q + 1 < rb; ++q) rl += __shfl_sync(FULL, rend, q) <= k + lane;
+      } else if (in) {
+        uint32_t a = 0, b = rb - 1;
+        while (a < b) {
+          const uint32_t mid = (a + b) >> 1;
+          const uint64_t r = (uint64_t)br.r0 + mid + 1;
+          if (r <= nrows && rowptr[r] <= k + lane) a = mid + 1; else b = mid;
+        }
+        rl = a;
+      }
+      uint64_t pos = ~(uint64_t)lane;  // its own, for lanes without a nonzero
+      T v = T(0);
+      if (in) {
+        uint32_t c = colind[k + lane];
+        if (c >= ncols) c = 0;
+        const uint32_t J = block_col(c, cb, cshift);
+        pos = rk[find(t, J, shift)] * bs + (uint64_t)rl * cb + (c - J * cb);
+        v = values[k + lane];
+      }
+      const unsigned same = __match_any_sync(FULL, (unsigned long long)pos);
+      if (in && pos < ne && lane == 31 - __clz(same)) blk[pos] = v;
+      __syncwarp();
+    }
+    for (uint32_t d = lane; d < D; d += 32) {
+      uint32_t nz = 0;
+      for (uint32_t q = 0, e = d % (uint32_t)bs; q < bs; ++q) {  // lanes start apart: other banks
+        nz += blk[d * bs + e] != T(0);
+        e = e + 1 == bs ? 0 : e + 1;
+      }
+      nnz_per_block[b0 + d] = nz;
+    }
+    if (in_smem) {
+      const uint64_t bytes = ne * sizeof(T);
+      if (((reinterpret_cast<uintptr_t>(gout) | bytes) & 15) == 0) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(blk);
+        for (uint64_t e = lane; e < bytes / 16; e += 32) reinterpret_cast<uint4 *>(gout)[e] = src[e];
+      } else {
+        for (uint64_t e = lane; e < ne; e += 32) gout[e] = blk[e];
+      }
+    }
+    __syncwarp();
+  });
+}
+
+// ---------------------------------------------------------------------------
+// All nonzeros sorted by block
+// ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(NT) keys(const uint32_t *__restrict__ rowptr, uint32_t nrows,
                                            const uint32_t *__restrict__ colind, uint32_t nnz, uint32_t ncols,
                                            uint32_t rb, uint32_t cb, int jbits, uint64_t *__restrict__ key,
@@ -130,12 +352,17 @@ using namespace sparsep::c2b;
 
 struct sparsep_bcsr_layout {
   uint32_t nrows = 0, ncols = 0, nnz = 0, rb = 0, cb = 0, nbr = 0, nblocks = 0;
-  int jbits = 0;
+  int dev = 0;
   const uint32_t *colind = nullptr;  // the caller's column indices (read again by the fill)
-  uint32_t *row = nullptr;           // row of each nonzero
-  uint32_t *sidx = nullptr;          // nonzeros in block order (input order inside a block)
-  uint32_t *bstart = nullptr;        // nblocks + 1 start positions in sidx
-  uint64_t *bkey = nullptr;          // block keys (block row << jbits | block column)
+  // block rows in shared memory
+  uint32_t *rowptr = nullptr;   // the row pointers
+  uint32_t *browptr = nullptr;  // nbr + 1
+  // the sort
+  int jbits = 0;
+  uint32_t *row = nullptr;     // row of each nonzero
+  uint32_t *sidx = nullptr;    // nonzeros in block order (input order inside a block)
+  uint32_t *bstart = nullptr;  // nblocks + 1 start positions in sidx
+  uint64_t *bkey = nullptr;    // block keys (block row << jbits | block column)
 };
 
 static int c2b_err(cudaError_t e) {
@@ -154,9 +381,61 @@ static int bits_for(uint64_t v) {  // bits of the largest value < v
 
 static unsigned grid_for(uint64_t n) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(16384, (n + NT - 1) / NT)); }
 
+static int col_shift(uint32_t cb) {  // log2 of a power of two, else -1
+  if (cb & (cb - 1)) return -1;
+  int s = 0;
+  while ((1u << s) < cb) ++s;
+  return s;
+}
+
+// Block rows in shared memory; *fits false where one is too long for that.
+static int layout_rows(const uint32_t *rowptr, sparsep_bcsr_layout *L, bool *fits, cudaStream_t s) {
+  using sparsep::radix::SCAN_CHUNK;
+  const uint32_t m = L->nbr + 1, nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
+  uint32_t *buf = nullptr;
+  int h_flag[2] = {0, 0};
+  int st = c2b_err(sparsep::ws_malloc((void **)&L->rowptr, ((size_t)L->nrows + 1) * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->browptr, (size_t)m * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&buf, ((size_t)nb + 4) * 4, s));
+  if (!st) {
+    int *flag = reinterpret_cast<int *>(buf + nb);
+    st = c2b_err(cudaMemsetAsync(flag, 0, 2 * sizeof(int), s));
+    if (!st) st = c2b_err(cudaMemsetAsync(L->browptr, 0, (size_t)m * 4, s));
+    if (!st)
+      st = c2b_err(cudaMemcpyAsync(L->rowptr, rowptr, ((size_t)L->nrows + 1) * 4, cudaMemcpyDeviceToDevice, s));
+    if (!st) {
+      const int cs = col_shift(L->cb);
+      if (L->nrows) check_rowptr<<<grid_for(L->nrows), NT, 0, s>>>(rowptr, L->nrows, L->nnz, flag);
+      if (L->nnz) {
+        constexpr int W = Table<LIM_SMALL>::WARPS;
+        const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + W - 1) / W);
+        count_blocks<LIM_SMALL><<<grid, 32 * W, 0, s>>>(rowptr, L->nrows, L->colind, L->nnz, L->ncols, L->rb, L->cb, cs,
+                                                        L->nbr, 0, L->browptr, flag);
+        count_blocks<LIM_LARGE><<<std::min<uint32_t>(2048, L->nbr / 32 + 1), 32, 0, s>>>(rowptr, L->nrows, L->colind, L->nnz,
+                                                                                L->ncols, L->rb, L->cb, cs, L->nbr,
+                                                                                LIM_SMALL, L->browptr, flag);
+        sparsep::radix::scan_reduce<<<nb, sparsep::radix::NT, 0, s>>>(L->browptr, m, buf);
+        sparsep::radix::scan_top<<<1, sparsep::radix::NT, 0, s>>>(buf, nb);
+        sparsep::radix::scan_down<<<nb, sparsep::radix::NT, 0, s>>>(L->browptr, m, buf);
+      }
+      st = c2b_err(cudaGetLastError());
+    }
+    if (!st) st = c2b_err(cudaMemcpyAsync(h_flag, flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (!st)
+      st = c2b_err(cudaMemcpyAsync(&L->nblocks, L->browptr + L->nbr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (!st) st = c2b_err(cudaStreamSynchronize(s));
+    if (!st && h_flag[0]) st = SPARSEP_EINVAL;
+  }
+  sparsep::ws_free(buf, s);
+  *fits = !h_flag[1];
+  return st;
+}
+
+static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_t nrows, uint32_t ncols, uint32_t nnz,
+                         uint32_t rb, uint32_t cb, sparsep_bcsr_layout *L, cudaStream_t s);
+
 static int layout(const uint32_t *rowptr, const uint32_t *colind, uint32_t nrows, uint32_t ncols, uint32_t nnz,
                   uint32_t rb, uint32_t cb, sparsep_bcsr_layout *L, cudaStream_t s) {
-  using sparsep::radix::radix_scratch_words;
   L->nrows = nrows;
   L->ncols = ncols;
   L->nnz = nnz;
@@ -164,66 +443,66 @@ static int layout(const uint32_t *rowptr, const uint32_t *colind, uint32_t nrows
   L->cb = cb;
   L->colind = colind;
   L->nbr = (uint32_t)(((uint64_t)nrows + rb - 1) / rb);
+  int st = c2b_err(cudaGetDevice(&L->dev));
+  bool fits = true;
+  if (!st) st = layout_rows(rowptr, L, &fits, s);
+  if (st || fits) return st;
+  sparsep::ws_free(L->rowptr, s);
+  sparsep::ws_free(L->browptr, s);
+  L->rowptr = L->browptr = nullptr;
+  return layout_sorted(rowptr, colind, nrows, ncols, nnz, rb, cb, L, s);
+}
+
+static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_t nrows, uint32_t ncols, uint32_t nnz,
+                         uint32_t rb, uint32_t cb, sparsep_bcsr_layout *L, cudaStream_t s) {
+  using sparsep::radix::radix_scratch_words;
   const uint64_t nbc = ((uint64_t)ncols + cb - 1) / cb;
   L->jbits = bits_for(nbc);
   const int bits = L->jbits + bits_for(L->nbr);
   int *bad = nullptr;
-  uint32_t *dnb = nullptr;
-  int st = c2b_err(sparsep::dev_malloc((void **)&bad, 2 * sizeof(int)));
+  int st = c2b_err(sparsep::ws_malloc((void **)&bad, 2 * sizeof(int), s));
   if (st) return st;
-  dnb = reinterpret_cast<uint32_t *>(bad + 1);
-  int h_bad = 0;
-  st = c2b_err(cudaMemsetAsync(bad, 0, 2 * sizeof(int), s));
-  if (!st && nrows) check_rowptr<<<grid_for(nrows), NT, 0, s>>>(rowptr, nrows, nnz, bad);
-  if (!st && nnz) {
-    // scratch, in 32-bit words: input keys (2n), two key buffers (2n each), the
-    // radix scratch, the head flags (n) with their scan sums (nbs + 8), and
-    // the block starts (n + 1).  After the sort the input-key buffer holds the
-    // block keys.
-    const uint32_t nbs = (nnz + sparsep::radix::SCAN_CHUNK - 1) / sparsep::radix::SCAN_CHUNK;
-    const size_t rsw = radix_scratch_words(nnz);
-    const size_t words = 6 * (size_t)nnz + rsw + ((size_t)nnz + nbs + 8) + ((size_t)nnz + 1) + 8;
-    uint32_t *buf = nullptr;
-    st = c2b_err(sparsep::dev_malloc((void **)&buf, words * 4));
-    if (!st) st = c2b_err(sparsep::dev_malloc((void **)&L->row, (size_t)nnz * 4));
+  uint32_t *dnb = reinterpret_cast<uint32_t *>(bad + 1);
+  // scratch, in 32-bit words: input keys (2n), two key buffers (2n each), the
+  // radix scratch, the head flags (n) with their scan sums (nbs + 8), and
+  // the block starts (n + 1).  After the sort the input-key buffer holds the
+  // block keys.
+  const uint32_t nbs = (nnz + sparsep::radix::SCAN_CHUNK - 1) / sparsep::radix::SCAN_CHUNK;
+  const size_t rsw = (radix_scratch_words(nnz) + 1) & ~(size_t)1;
+  const size_t words = 6 * (size_t)nnz + rsw + ((size_t)nnz + nbs + 8) + ((size_t)nnz + 1) + 8;
+  uint32_t *buf = nullptr;
+  st = c2b_err(sparsep::ws_malloc((void **)&buf, words * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->row, (size_t)nnz * 4, s));
+  if (!st) {
+    uint64_t *key = reinterpret_cast<uint64_t *>(buf), *k0 = key + nnz, *k1 = k0 + nnz;
+    uint32_t *scratch = reinterpret_cast<uint32_t *>(k1 + nnz);
+    uint32_t *flag = scratch + rsw, *sums = flag + nnz, *bstart_tmp = sums + nbs + 8;
+    uint64_t *bkey_tmp = key;
+    keys<<<grid_for(nnz), NT, 0, s>>>(rowptr, nrows, colind, nnz, ncols, rb, cb, L->jbits, key, L->row, bad);
+    const uint64_t *skey = nullptr;
+    const uint32_t *sidx = nullptr;
+    st = c2b_err(sparsep::radix::radix_sort<uint64_t>(key, nnz, bits, k0, k1, scratch, &skey, &sidx, s));
     if (!st) {
-      uint64_t *key = reinterpret_cast<uint64_t *>(buf), *k0 = key + nnz, *k1 = k0 + nnz;
-      uint32_t *scratch = reinterpret_cast<uint32_t *>(k1 + nnz);
-      uint32_t *flag = scratch + rsw, *sums = flag + nnz, *bstart_tmp = sums + nbs + 8;
-      uint64_t *bkey_tmp = key;
-      keys<<<grid_for(nnz), NT, 0, s>>>(rowptr, nrows, colind, nnz, ncols, rb, cb, L->jbits, key, L->row, bad);
-      const uint64_t *skey = nullptr;
-      const uint32_t *sidx = nullptr;
-      st = c2b_err(sparsep::radix::radix_sort<uint64_t>(key, nnz, bits, k0, k1, scratch, &skey, &sidx, s));
-      if (!st) {
-        head_flags<<<grid_for(nnz), NT, 0, s>>>(skey, nnz, flag);
-        sparsep::radix::scan_reduce<<<nbs, sparsep::radix::NT, 0, s>>>(flag, nnz, sums);
-        sparsep::radix::scan_top<<<1, sparsep::radix::NT, 0, s>>>(sums, nbs);
-        sparsep::radix::scan_down<<<nbs, sparsep::radix::NT, 0, s>>>(flag, nnz, sums);
-        block_starts<<<grid_for(nnz), NT, 0, s>>>(skey, nnz, flag, bstart_tmp, bkey_tmp, dnb);
-        st = c2b_err(cudaGetLastError());
-      }
-      if (!st) st = c2b_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
-      if (!st) st = c2b_err(cudaMemcpyAsync(&L->nblocks, dnb, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      if (!st) st = c2b_err(cudaStreamSynchronize(s));
-      if (!st && h_bad) st = SPARSEP_EINVAL;
-      if (!st) st = c2b_err(sparsep::dev_malloc((void **)&L->sidx, (size_t)nnz * 4));
-      if (!st) st = c2b_err(sparsep::dev_malloc((void **)&L->bstart, ((size_t)L->nblocks + 1) * 4));
-      if (!st) st = c2b_err(sparsep::dev_malloc((void **)&L->bkey, (size_t)std::max<uint32_t>(L->nblocks, 1) * 8));
-      if (!st) st = c2b_err(cudaMemcpyAsync(L->sidx, sidx, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
-      if (!st)
-        st = c2b_err(cudaMemcpyAsync(L->bstart, bstart_tmp, ((size_t)L->nblocks + 1) * 4, cudaMemcpyDeviceToDevice, s));
-      if (!st) st = c2b_err(cudaMemcpyAsync(L->bkey, bkey_tmp, (size_t)L->nblocks * 8, cudaMemcpyDeviceToDevice, s));
-      if (!st) st = c2b_err(cudaStreamSynchronize(s));
+      head_flags<<<grid_for(nnz), NT, 0, s>>>(skey, nnz, flag);
+      sparsep::radix::scan_reduce<<<nbs, sparsep::radix::NT, 0, s>>>(flag, nnz, sums);
+      sparsep::radix::scan_top<<<1, sparsep::radix::NT, 0, s>>>(sums, nbs);
+      sparsep::radix::scan_down<<<nbs, sparsep::radix::NT, 0, s>>>(flag, nnz, sums);
+      block_starts<<<grid_for(nnz), NT, 0, s>>>(skey, nnz, flag, bstart_tmp, bkey_tmp, dnb);
+      st = c2b_err(cudaGetLastError());
     }
-    sparsep::dev_free(buf);
-  } else if (!st) {
-    st = c2b_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (!st) st = c2b_err(cudaMemcpyAsync(&L->nblocks, dnb, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (!st) st = c2b_err(cudaStreamSynchronize(s));
-    if (!st && h_bad) st = SPARSEP_EINVAL;
-    L->nblocks = 0;
+    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->sidx, (size_t)nnz * 4, s));
+    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bstart, ((size_t)L->nblocks + 1) * 4, s));
+    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bkey, (size_t)std::max<uint32_t>(L->nblocks, 1) * 8, s));
+    if (!st) st = c2b_err(cudaMemcpyAsync(L->sidx, sidx, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
+    if (!st)
+      st = c2b_err(cudaMemcpyAsync(L->bstart, bstart_tmp, ((size_t)L->nblocks + 1) * 4, cudaMemcpyDeviceToDevice, s));
+    if (!st) st = c2b_err(cudaMemcpyAsync(L->bkey, bkey_tmp, (size_t)L->nblocks * 8, cudaMemcpyDeviceToDevice, s));
+    if (!st) st = c2b_err(cudaStreamSynchronize(s));
   }
-  sparsep::dev_free(bad);
+  sparsep::ws_free(buf, s);
+  sparsep::ws_free(bad, s);
   return st;
 }
 
@@ -231,6 +510,22 @@ template <typename T>
 static int fill(const sparsep_bcsr_layout *L, const T *values, uint32_t *browptr, uint32_t *bcolind, T *bval,
                 uint32_t *nnz_per_block, cudaStream_t s) {
   if (!L || !browptr || (L->nblocks && (!values || !bcolind || !bval || !nnz_per_block))) return SPARSEP_EINVAL;
+  if (L->browptr) {
+    int st = c2b_err(cudaMemcpyAsync(browptr, L->browptr, ((size_t)L->nbr + 1) * 4, cudaMemcpyDeviceToDevice, s));
+    if (!st && L->nblocks) {
+      constexpr int W = Table<LIM_SMALL>::WARPS;
+      const int cs = col_shift(L->cb);
+      const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + W - 1) / W);
+      fill_rows<T, LIM_SMALL><<<grid, 32 * W, 0, s>>>(L->rowptr, L->nrows, L->colind, L->nnz, L->ncols, values, L->rb,
+                                                      L->cb, cs, L->nbr, 0, L->browptr, bcolind, bval, nnz_per_block);
+      fill_rows<T, LIM_LARGE><<<std::min<uint32_t>(2048, L->nbr / 32 + 1), 32, 0, s>>>(
+          L->rowptr, L->nrows, L->colind, L->nnz, L->ncols, values, L->rb, L->cb, cs, L->nbr, LIM_SMALL, L->browptr,
+          bcolind, bval, nnz_per_block);
+      st = c2b_err(cudaGetLastError());
+    }
+    if (!st) st = c2b_err(cudaStreamSynchronize(s));
+    return st;
+  }
   browptr_kernel<<<(L->nbr + 1 + 255) / 256, 256, 0, s>>>(L->bkey, L->nblocks, L->nbr, L->jbits, browptr);
   if (L->nblocks)
     fill_blocks<T><<<grid_for(L->nblocks), NT, 0, s>>>(L->bkey, L->bstart, L->nblocks, L->sidx, L->row, L->colind,
@@ -262,8 +557,14 @@ int sparsep_bcsr_layout_device(const uint32_t *d_rowptr, const uint32_t *d_colin
 
 void sparsep_bcsr_layout_free(sparsep_bcsr_layout *L) {
   if (!L) return;
-  for (void *d : {(void *)L->row, (void *)L->sidx, (void *)L->bstart, (void *)L->bkey})
-    if (d) sparsep::dev_free(d);
+  // layout and fill have synchronised their streams: nothing uses these any more
+  int dev = L->dev;
+  cudaGetDevice(&dev);
+  if (dev != L->dev) cudaSetDevice(L->dev);
+  for (void *d : {(void *)L->rowptr, (void *)L->browptr, (void *)L->row, (void *)L->sidx, (void *)L->bstart,
+                  (void *)L->bkey})
+    sparsep::ws_free(d, nullptr);
+  if (dev != L->dev) cudaSetDevice(dev);
   delete L;
 }
 

@@ -6,6 +6,7 @@
 // without faulting a GPU: a device allocation that fails (SPARSEP_ENOMEM) and
 // a bounded device wait that runs out (SPARSEP_ETIMEDOUT).
 #include <atomic>
+#include <mutex>
 
 #include "fault.hpp"
 #include "sparsep.h"
@@ -16,15 +17,58 @@ static std::atomic<long long> g_live{0};  // live device allocations
 static std::atomic<int> g_fail_in{0};     // the g_fail_in-th allocation from now fails (0: none)
 static std::atomic<int> g_wait_fault{0};
 
-cudaError_t dev_malloc(void **p, size_t bytes) {
+// The allocation that the tests asked to fail is this one.
+static bool fails_now() {
   int n = g_fail_in.load();
   while (n > 0 && !g_fail_in.compare_exchange_weak(n, n - 1)) {
   }
-  if (n == 1) {
-    *p = nullptr;
-    return cudaErrorMemoryAllocation;
+  return n == 1;
+}
+
+// The current device's pool, made on first use; null where the device has none.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64];
+static cudaMemPool_t pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    uint64_t keep = POOL_KEEP;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      if (p) cudaMemPoolDestroy(p);
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_pool[dev] = p;
   }
-  const cudaError_t e = cudaMalloc(p, bytes);
+  return g_pool[dev];
+}
+// What the current device's pool keeps and nobody uses, back to the device.
+static void trim_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool[dev]) {
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(g_pool[dev], 0);
+  }
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes) {
+  *p = nullptr;
+  if (fails_now()) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pool();
+    e = cudaMalloc(p, bytes);
+  }
   if (e == cudaSuccess) ++g_live;
   return e;
 }
@@ -32,6 +76,26 @@ cudaError_t dev_malloc(void **p, size_t bytes) {
 void dev_free(void *p) {
   if (!p) return;
   cudaFree(p);
+  --g_live;
+}
+
+cudaError_t ws_malloc(void **p, size_t bytes, cudaStream_t s) {
+  *p = nullptr;
+  if (fails_now()) return cudaErrorMemoryAllocation;
+  cudaMemPool_t pl = pool();
+  cudaError_t e = pl ? cudaMallocFromPoolAsync(p, bytes, pl, s) : cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pool();
+    e = pl ? cudaMallocFromPoolAsync(p, bytes, pl, s) : cudaMallocAsync(p, bytes, s);
+  }
+  if (e == cudaSuccess) ++g_live;
+  return e;
+}
+
+void ws_free(void *p, cudaStream_t s) {
+  if (!p) return;
+  cudaFreeAsync(p, s);
   --g_live;
 }
 

@@ -12,6 +12,15 @@ namespace sparsep {
 cudaError_t dev_malloc(void **p, size_t bytes);
 void dev_free(void *p);
 
+// Scratch memory that a call takes and gives back, ordered on its stream: from a
+// pool of the library's own per device, which keeps up to POOL_KEEP bytes between
+// calls (a quarter gigabyte from cudaMalloc and back costs a call milliseconds and
+// two device-wide synchronisations) and gives them up when the device is full.
+// Counted and failed on request like dev_malloc.
+constexpr size_t POOL_KEEP = (size_t)512 << 20;
+cudaError_t ws_malloc(void **p, size_t bytes, cudaStream_t s);
+void ws_free(void *p, cudaStream_t s);
+
 // Nonzero while test support asks the kernels with bounded staging waits to
 // add one wait that nothing completes (after their own copies have landed).
 int wait_fault();

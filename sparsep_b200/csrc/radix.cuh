@@ -1,43 +1,59 @@
-// radix.cuh -- stable LSD radix sort of (key, index) pairs on the device,
-// 4 bits per pass, used by the device format builders (COO -> CSR sorts by
-// row; CSR -> BCSR by (block row, block column)).
-//   hist     per 1024-element tile, counts of each digit  -> hist[d][tile]
+// radix.cuh -- stable LSD radix sort on the device, up to 7 bits per pass, used by
+// the device format builders: COO -> CSR sorts (row, column, value) records by
+// row; CSR -> BCSR, where a block row is too long for shared memory, (key, index)
+// pairs by (block row, block column).
+//   hist     per 4096-element tile, counts of each digit  -> hist[d][tile]
 //   scan     exclusive scan of hist in digit-major order (three launches)
-//   scatter  each element to scan[d][tile] + (earlier elements of its tile
-//            with digit d): the tile is walked in four 256-element rounds;
-//            inside a round, __match_any_sync gives the rank among the warp's
-//            lanes with the same digit, a prefix over the warps and a running
-//            count per digit over the rounds do the rest -- input order kept.
+//   scatter  each element to scan[d][tile] + (earlier elements of its tile with
+//            digit d).  A warp takes 512 consecutive elements, 32 at a time;
+//            __match_any_sync gives the rank among the lanes with the same digit
+//            and the warp's own counter per digit the rank before that, so the
+//            warps meet only twice.  Keys and payloads then go through shared
+//            memory one after the other, so that a digit's elements leave as runs
+//            of consecutive addresses.
+// Bound by HBM: an element's record is read and written once per pass.  With
+// 4-bit digits, 1024-element tiles and three barriers per 256 elements, 10.5 M
+// 32-bit keys and their indices took 107 us per pass and 5 passes for 19 bits.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace sparsep {
 namespace radix {
 namespace {  // internal linkage: every translation unit that sorts gets its own kernels
 
-constexpr int NT = 256;         // threads per CTA
-constexpr int ROUNDS = 4;       // elements per thread per tile
-constexpr int TILE = NT * ROUNDS;
-constexpr int RADIX = 16;       // 4-bit digits
+constexpr int NT = 256;            // threads per CTA
+constexpr int IPT = 16;            // elements per thread per tile
+constexpr int TILE = NT * IPT;
+constexpr int MAX_BITS = 7;        // bits of a digit
+constexpr int MAX_RADIX = 1 << MAX_BITS;
+constexpr unsigned FULL = 0xffffffffu;
 
 template <typename K>
-__global__ void __launch_bounds__(NT) hist(const K *__restrict__ key, uint32_t n, int shift, uint32_t nt,
+__global__ void __launch_bounds__(NT) hist(const K *__restrict__ key, uint32_t n, int shift, int bits, uint32_t nt,
                                            uint32_t *__restrict__ h, K bound, int *__restrict__ bad) {
-  __shared__ uint32_t c[RADIX];
-  if (threadIdx.x < RADIX) c[threadIdx.x] = 0;
+  __shared__ uint32_t c[NT / 32][MAX_RADIX];  // per warp: fewer lanes meet at one counter
+  const int warp = threadIdx.x >> 5, radix = 1 << bits;
+  for (int i = threadIdx.x; i < NT / 32 * MAX_RADIX; i += NT) (&c[0][0])[i] = 0;
   __syncthreads();
   const uint32_t base = blockIdx.x * TILE;
-  for (int r = 0; r < ROUNDS; ++r) {
+#pragma unroll 8
+  for (int r = 0; r < IPT; ++r) {
     const uint32_t i = base + r * NT + threadIdx.x;
     if (i < n) {
       const K k = key[i];
       if (bad && k >= bound) atomicExch(bad, 1);  // first pass only: keys must be < bound
-      atomicAdd(&c[(uint32_t)(k >> shift) & (RADIX - 1)], 1u);
+      atomicAdd(&c[warp][(uint32_t)(k >> shift) & (radix - 1)], 1u);
     }
   }
   __syncthreads();
-  if (threadIdx.x < RADIX) h[(size_t)threadIdx.x * nt + blockIdx.x] = c[threadIdx.x];
+  if (threadIdx.x < radix) {
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) t += c[w][threadIdx.x];
+    h[(size_t)threadIdx.x * nt + blockIdx.x] = t;
+  }
 }
 
 // Exclusive scan of the m digit counts in place, in three launches:
@@ -118,72 +134,157 @@ __global__ void __launch_bounds__(NT) scan_down(uint32_t *__restrict__ h, uint32
   scan_chunk(h, m, blockIdx.x * SCAN_CHUNK, sums[blockIdx.x]);
 }
 
-template <typename K>
-__global__ void __launch_bounds__(NT) scatter(const K *__restrict__ key, const uint32_t *__restrict__ idx,
-                                              uint32_t n, int shift, uint32_t nt, const uint32_t *__restrict__ off,
-                                              K *__restrict__ key_out, uint32_t *__restrict__ idx_out) {
-  __shared__ uint32_t warp_cnt[NT / 32][RADIX];
-  __shared__ uint32_t running[RADIX];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < RADIX) running[threadIdx.x] = 0;
-  const uint32_t base = blockIdx.x * TILE;
-  for (int r = 0; r < ROUNDS; ++r) {
-    const uint32_t i = base + r * NT + threadIdx.x;
-    const bool in = i < n;
-    const K k = in ? key[i] : K(0);
-    const uint32_t d = in ? (uint32_t)(k >> shift) & (RADIX - 1) : RADIX;  // out-of-range lanes form their own group
-    const unsigned same = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank = __popc(same & ((1u << lane) - 1u));
-    __syncthreads();  // the previous round's readers of warp_cnt / running are done
-    if (lane < RADIX) warp_cnt[warp][lane] = 0;
-    __syncwarp();
-    if (in && rank == 0) warp_cnt[warp][d] = __popc(same);  // the group's first lane
-    __syncthreads();
-    if (in) {
-      uint32_t before = running[d];
-      for (int w = 0; w < warp; ++w) before += warp_cnt[w][d];
-      const uint32_t pos = off[(size_t)d * nt + blockIdx.x] + before + rank;
-      key_out[pos] = k;
-      idx_out[pos] = idx ? idx[i] : i;
+// One pass.  The payload of an element is a 32-bit word (its index where w_in is
+// null) and, unless V is NoValue, a value.
+struct NoValue {};
+
+template <typename K, typename V>
+__global__ void __launch_bounds__(NT) scatter(const K *__restrict__ key, const uint32_t *__restrict__ w_in,
+                                              const V *__restrict__ v_in, uint32_t n, int shift, int bits, uint32_t nt,
+                                              const uint32_t *__restrict__ off, K *__restrict__ key_out,
+                                              uint32_t *__restrict__ w_out, V *__restrict__ v_out) {
+  constexpr bool VALUE = !std::is_same<V, NoValue>::value;
+  constexpr size_t UNIT = sizeof(K) > sizeof(V) ? sizeof(K) : sizeof(V);
+  __shared__ __align__(16) unsigned char stage[TILE * (UNIT > 4 ? UNIT : 4)];
+  __shared__ uint32_t cnt[NT / 32][MAX_RADIX];
+  __shared__ uint32_t first[MAX_RADIX];  // of the tile's elements, the first of each digit
+  __shared__ uint32_t dst[MAX_RADIX];    // its place in the output less that
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, radix = 1 << bits;
+  const uint32_t base = blockIdx.x * TILE, here = n - base < TILE ? n - base : TILE;
+  for (int i = threadIdx.x; i < NT / 32 * MAX_RADIX; i += NT) (&cnt[0][0])[i] = 0;
+  __syncthreads();
+  // this thread's elements: 32 apart, in the warp's 512
+  const uint32_t mine = warp * (32 * IPT) + lane;
+  K k[IPT];
+  uint32_t pos[IPT];
+#pragma unroll
+  for (int r = 0; r < IPT; ++r) k[r] = mine + r * 32 < here ? key[base + mine + r * 32] : K(0);
+#pragma unroll
+  for (int r = 0; r < IPT; ++r) {
+    const bool in = mine + r * 32 < here;
+    const uint32_t d = in ? (uint32_t)(k[r] >> shift) & (radix - 1) : MAX_RADIX;  // the others form their own group
+    const unsigned same = __match_any_sync(FULL, d);
+    const int leader = __ffs(same) - 1;
+    uint32_t before = 0;
+    if (in && lane == leader) {
+      before = cnt[warp][d];
+      cnt[warp][d] = before + __popc(same);
     }
+    pos[r] = __shfl_sync(FULL, before, leader) + __popc(same & ((1u << lane) - 1u));
+    __syncwarp();
+  }
+  __syncthreads();
+  uint32_t all = 0;
+  if (threadIdx.x < radix)
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      const uint32_t c = cnt[w][threadIdx.x];
+      cnt[w][threadIdx.x] = all;
+      all += c;
+    }
+  uint32_t total;
+  const uint32_t f = block_scan(all, &total);
+  if (threadIdx.x < radix) {
+    first[threadIdx.x] = f;
+    dst[threadIdx.x] = off[(size_t)threadIdx.x * nt + blockIdx.x] - f;
+  }
+  __syncthreads();
+  K *sk = reinterpret_cast<K *>(stage);
+#pragma unroll
+  for (int r = 0; r < IPT; ++r)
+    if (mine + r * 32 < here) {
+      const uint32_t d = (uint32_t)(k[r] >> shift) & (radix - 1);
+      pos[r] += first[d] + cnt[warp][d];
+      sk[pos[r]] = k[r];
+    }
+  __syncthreads();
+  uint32_t to[IPT];  // where the staged elements threadIdx.x, threadIdx.x + NT, ... go
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const uint32_t q = threadIdx.x + j * NT;
+    if (q < here) {
+      const K kk = sk[q];
+      to[j] = dst[(uint32_t)(kk >> shift) & (radix - 1)] + q;
+      key_out[to[j]] = kk;
+    }
+  }
+  __syncthreads();
+  uint32_t *sw = reinterpret_cast<uint32_t *>(stage);
+#pragma unroll
+  for (int r = 0; r < IPT; ++r)
+    if (mine + r * 32 < here) sw[pos[r]] = w_in ? w_in[base + mine + r * 32] : base + mine + r * 32;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const uint32_t q = threadIdx.x + j * NT;
+    if (q < here) w_out[to[j]] = sw[q];
+  }
+  if constexpr (VALUE) {
     __syncthreads();
-    if (threadIdx.x < RADIX) {
-      uint32_t t = 0;
-      for (int w = 0; w < NT / 32; ++w) t += warp_cnt[w][threadIdx.x];
-      running[threadIdx.x] += t;
+    V *sv = reinterpret_cast<V *>(stage);
+#pragma unroll
+    for (int r = 0; r < IPT; ++r)
+      if (mine + r * 32 < here) sv[pos[r]] = v_in[base + mine + r * 32];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const uint32_t q = threadIdx.x + j * NT;
+      if (q < here) v_out[to[j]] = sv[q];
     }
   }
 }
 
+// Passes for `bits` bits (at least one, so that the outputs are produced even for
+// none), and the bits of each.
+inline int passes(int bits) { return bits <= MAX_BITS ? 1 : (bits + MAX_BITS - 1) / MAX_BITS; }
+inline int pass_bits(int bits, int pass, int np) { return bits / np + (pass < bits % np ? 1 : 0); }
 
-// Scratch words (32-bit) radix_sort needs for n elements besides the key buffers.
-inline size_t radix_scratch_words(uint32_t n) {
-  const uint32_t nt = (n + TILE - 1) / TILE, m = RADIX * nt, nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  return 2 * (size_t)n + m + nb + 8;
+// Scratch words (32-bit) of the digit counts of n elements and their scan.
+inline size_t count_words(uint32_t n) {
+  const size_t nt = ((size_t)n + TILE - 1) / TILE, m = MAX_RADIX * nt, nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
+  return m + nb + 8;
 }
 
-// Stable sort of keys[0, n) by their low `bits` bits (at least one pass, so
-// that the index array is produced even for bits = 0), carrying the input
-// index.  k0/k1: two key buffers of n; scratch: radix_scratch_words(n) words.
-// On return *ks / *is point at the sorted keys and input indices (inside k0/k1
-// and scratch).  bad/bound: when bad is set, the first pass flags a key >= bound.
+// One pass over n elements from `shift` on; counts: count_words(n) words.
+template <typename K>
+cudaError_t count_pass(const K *key, uint32_t n, int shift, int bits, uint32_t *counts, cudaStream_t s,
+                       int *bad = nullptr, K bound = K(0)) {
+  const uint32_t nt = (uint32_t)(((uint64_t)n + TILE - 1) / TILE), m = nt << bits,
+                 nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
+  uint32_t *sums = counts + m;
+  hist<K><<<nt, NT, 0, s>>>(key, n, shift, bits, nt, counts, bound, bad);
+  scan_reduce<<<nb, NT, 0, s>>>(counts, m, sums);
+  scan_top<<<1, NT, 0, s>>>(sums, nb);
+  scan_down<<<nb, NT, 0, s>>>(counts, m, sums);
+  return cudaGetLastError();
+}
+template <typename K, typename V>
+cudaError_t scatter_pass(const K *key, const uint32_t *w_in, const V *v_in, uint32_t n, int shift, int bits,
+                         const uint32_t *counts, K *key_out, uint32_t *w_out, V *v_out, cudaStream_t s) {
+  const uint32_t nt = (uint32_t)(((uint64_t)n + TILE - 1) / TILE);
+  scatter<K, V><<<nt, NT, 0, s>>>(key, w_in, v_in, n, shift, bits, nt, counts, key_out, w_out, v_out);
+  return cudaGetLastError();
+}
+
+// Scratch words (32-bit) radix_sort needs for n elements besides the key buffers.
+inline size_t radix_scratch_words(uint32_t n) { return 2 * (size_t)n + count_words(n); }
+
+// Stable sort of keys[0, n) by their low `bits` bits, carrying the input index.
+// k0/k1: two key buffers of n; scratch: radix_scratch_words(n) words.  On return
+// *ks / *is point at the sorted keys and input indices (inside k0/k1 and scratch).
 template <typename K>
 cudaError_t radix_sort(const K *keys, uint32_t n, int bits, K *k0, K *k1, uint32_t *scratch, const K **ks,
-                       const uint32_t **is, cudaStream_t s, int *bad = nullptr, K bound = K(0)) {
-  const uint32_t nt = (n + TILE - 1) / TILE, m = RADIX * nt, nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  uint32_t *i0 = scratch, *i1 = i0 + n, *h = i1 + n, *sums = h + m;
+                       const uint32_t **is, cudaStream_t s) {
+  uint32_t *i0 = scratch, *i1 = i0 + n, *counts = i1 + n;
   const K *key = keys;
   const uint32_t *idx = nullptr;
-  for (int shift = 0; n && shift < (bits ? bits : 1); shift += 4) {
-    const bool odd = (shift / 4) % 2;
-    K *ko = odd ? k1 : k0;
-    uint32_t *io = odd ? i1 : i0;
-    hist<K><<<nt, NT, 0, s>>>(key, n, shift, nt, h, bound, shift == 0 ? bad : nullptr);
-    scan_reduce<<<nb, NT, 0, s>>>(h, m, sums);
-    scan_top<<<1, NT, 0, s>>>(sums, nb);
-    scan_down<<<nb, NT, 0, s>>>(h, m, sums);
-    scatter<K><<<nt, NT, 0, s>>>(key, idx, n, shift, nt, h, ko, io);
-    if (cudaError_t e = cudaGetLastError()) return e;
+  const int np = passes(bits);
+  for (int p = 0, shift = 0; n && p < np; shift += pass_bits(bits, p, np), ++p) {
+    K *ko = p % 2 ? k1 : k0;
+    uint32_t *io = p % 2 ? i1 : i0;
+    const int b = pass_bits(bits, p, np);
+    if (cudaError_t e = count_pass<K>(key, n, shift, b, counts, s)) return e;
+    if (cudaError_t e = scatter_pass<K, NoValue>(key, idx, nullptr, n, shift, b, counts, ko, io, nullptr, s)) return e;
     key = ko;
     idx = io;
   }

@@ -27,7 +27,8 @@
 //   fill   browptr by lower bound among the block keys, one thread per block
 // FP32, 10.5 M nonzeros in 1 M blocks of 4x4 (COO -> CSR -> BCSR as one ingest): 8.1
 // ms with the sort for every matrix and scratch from cudaMalloc, of which 1.9 ms in
-// kernels.
+// kernels; 0.67 ms now, of which layout 0.12 and fill 0.16 ms (fill_rows 134 us, bound
+// by its instructions: 850 for a block row of 80 nonzeros).
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -86,7 +87,8 @@ __device__ __forceinline__ uint32_t hash(uint32_t J, int shift) { return (J * 0x
 __device__ __forceinline__ uint32_t insert(uint32_t *t, uint32_t J, int shift, bool *fresh) {
   const uint32_t mask = (1u << (32 - shift)) - 1u;
   for (uint32_t s = hash(J, shift);; s = (s + 1) & mask) {  // at least half of the slots stay empty
-    const uint32_t old = atomicCAS(t + s, EMPTY, J);
+    uint32_t old = *(volatile uint32_t *)(t + s);
+    if (old == EMPTY) old = atomicCAS(t + s, EMPTY, J);
     if (old == EMPTY || old == J) {
       *fresh = old == EMPTY;
       return s;
@@ -180,21 +182,45 @@ __global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
     const uint32_t m = br.k1 - br.k0;
     if (m <= lo || m > LIM) return;
     const int shift = table_shift(m);
+    // all that memory has to give, at once: the first nonzeros, the rows' ends and the blocks' place
+    constexpr int PRE = 4;
+    uint32_t pc[PRE];
+    T pv[PRE];
+#pragma unroll
+    for (int q = 0; q < PRE; ++q) {
+      const uint32_t k = br.k0 + q * 32 + lane;
+      pc[q] = 0;
+      pv[q] = T(0);
+      if (k < br.k1) {
+        pc[q] = colind[k];
+        pv[q] = values[k];
+      }
+    }
+    const uint32_t rend = lane < rb && br.r0 + lane + 1 <= nrows ? rowptr[br.r0 + lane + 1] : 0xFFFFFFFFu;
+    const uint32_t b0 = browptr[I], room = browptr[I + 1] - b0;
     for (uint32_t i = lane; i < 1u << (32 - shift); i += 32) t[i] = EMPTY;
     if (lane == 0) count[warp] = 0;
     __syncwarp();
-    for (uint32_t k = br.k0 + lane; k < br.k1; k += 32) {
-      const uint32_t c = colind[k], J = block_col(c < ncols ? c : 0, cb, cshift);
+    auto enter = [&](uint32_t c) {
+      const uint32_t J = block_col(c < ncols ? c : 0, cb, cshift);
       bool fresh;
-      insert(t, J, shift, &fresh);
+      const uint32_t slot = insert(t, J, shift, &fresh);
       if (fresh) l[atomicAdd(&count[warp], 1u)] = J;
+      return slot;
+    };
+    uint32_t ps[PRE];
+#pragma unroll
+    for (int q = 0; q < PRE; ++q) {
+      ps[q] = 0;
+      if (br.k0 + q * 32 + lane < br.k1) ps[q] = enter(pc[q]);
     }
+    for (uint32_t k = br.k0 + PRE * 32 + lane; k < br.k1; k += 32) enter(colind[k]);
     __syncwarp();
-    const uint32_t b0 = browptr[I], room = browptr[I + 1] - b0;
     const uint32_t D = count[warp] < room ? count[warp] : room;  // equal, while colind is as it was counted
     for (uint32_t d = lane; d < D; d += 32) {
       const uint32_t J = l[d];
       uint32_t r = 0;
+#pragma unroll 4
       for (uint32_t e = 0; e < D; ++e) r += l[e] < J;
       rk[find(t, J, shift)] = (uint16_t)r;
       if (r < room) bcolind[b0 + r] = J;
@@ -206,37 +232,63 @@ __global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
     const bool in_smem = ne * sizeof(T) <= (uint64_t)Tb::BLOCKS;
     T *blk = in_smem ? reinterpret_cast<T *>(blocks[warp]) : gout;
     for (uint64_t e = lane; e < ne; e += 32) blk[e] = T(0);
-    // ends of the block row's rows, one per lane
-    const uint32_t rend = lane < rb && br.r0 + lane + 1 <= nrows ? rowptr[br.r0 + lane + 1] : 0xFFFFFFFFu;
     __syncwarp();
-    for (uint32_t k = br.k0; k < br.k1; k += 32) {  // input order: a later duplicate wins
-      const bool in = k + lane < br.k1;
-      uint32_t rl = 0;  // row in the block: the block row's rows that end at or before this nonzero
-      if (rb <= 32) {
-        for (uint32_t q = 0; q + 1 < rb; ++q) rl += __shfl_sync(FULL, rend, q) <= k + lane;
-      } else if (in) {
-        uint32_t a = 0, b = rb - 1;
-        while (a < b) {
-          const uint32_t mid = (a + b) >> 1;
-          const uint64_t r = (uint64_t)br.r0 + mid + 1;
-          if (r <= nrows && rowptr[r] <= k + lane) a = mid + 1; else b = mid;
+    // The list is done with: which lane came to a position.  Matching 64-bit positions
+    // in every group of 32 cost FP32 4x4 65 us of 222 (10.5 M nonzeros).
+    unsigned char *tag = reinterpret_cast<unsigned char *>(l);
+    auto place_all = [&](auto zero) {  // positions as wide as this
+      using P = decltype(zero);
+      const P nel = (P)ne, bsz = (P)bs;
+      auto place = [&](uint32_t k, uint32_t c, T v, auto slot_of) {  // nonzeros [k, k + 32)
+        const bool in = k + lane < br.k1;
+        uint32_t rl = 0;  // row in the block: the block row's rows that end at or before this nonzero
+        if (rb <= 32) {
+          for (uint32_t q = 0; q + 1 < rb; ++q) rl += __shfl_sync(FULL, rend, q) <= k + lane;
+        } else if (in) {
+          uint32_t a = 0, b = rb - 1;
+          while (a < b) {
+            const uint32_t mid = (a + b) >> 1;
+            const uint64_t r = (uint64_t)br.r0 + mid + 1;
+            if (r <= nrows && rowptr[r] <= k + lane) a = mid + 1; else b = mid;
+          }
+          rl = a;
         }
-        rl = a;
+        P pos = ~(P)lane;  // its own, for lanes without a nonzero
+        if (in) {
+          if (c >= ncols) c = 0;
+          const uint32_t J = block_col(c, cb, cshift);
+          pos = rk[slot_of(J)] * bsz + (P)rl * cb + (c - J * cb);
+        }
+        bool last = in && pos < nel;  // of the lanes with this position, the last
+        bool twice = true;            // there may be two lanes with one position
+        if (nel <= sizeof(list[warp])) {
+          if (last) tag[pos] = (unsigned char)lane;
+          __syncwarp();
+          twice = __any_sync(FULL, last && tag[pos] != lane);
+        }
+        if (twice) last &= lane == 31 - __clz(__match_any_sync(FULL, pos));
+        if (last) blk[pos] = v;
+        __syncwarp();
+      };
+      // input order: a later duplicate wins
+#pragma unroll
+      for (int q = 0; q < PRE; ++q)
+        if (br.k0 + q * 32 < br.k1) place(br.k0 + q * 32, pc[q], pv[q], [&](uint32_t) { return ps[q]; });
+      for (uint32_t k = br.k0 + PRE * 32; k < br.k1; k += 32) {
+        const bool in = k + lane < br.k1;
+        place(k, in ? colind[k + lane] : 0, in ? values[k + lane] : T(0),
+              [&](uint32_t J) { return find(t, J, shift); });
       }
-      uint64_t pos = ~(uint64_t)lane;  // its own, for lanes without a nonzero
-      T v = T(0);
-      if (in) {
-        uint32_t c = colind[k + lane];
-        if (c >= ncols) c = 0;
-        const uint32_t J = block_col(c, cb, cshift);
-        pos = rk[find(t, J, shift)] * bs + (uint64_t)rl * cb + (c - J * cb);
-        v = values[k + lane];
+    };
+    if (in_smem) place_all(0u); else place_all(0ull);
+    if (bs <= 32 && (bs & (bs - 1)) == 0 && in_smem) {  // 32 / bs blocks at a time
+      const uint32_t nel = (uint32_t)ne, b32 = (uint32_t)bs, s32 = __ffs(b32) - 1;
+      for (uint32_t e = lane; e - lane < nel; e += 32) {
+        const uint32_t some = __ballot_sync(FULL, e < nel && blk[e] != T(0));
+        if (e < nel && (e & (b32 - 1)) == 0)
+          nnz_per_block[b0 + (e >> s32)] = __popc(some >> lane & (0xFFFFFFFFu >> (32 - b32)));
       }
-      const unsigned same = __match_any_sync(FULL, (unsigned long long)pos);
-      if (in && pos < ne && lane == 31 - __clz(same)) blk[pos] = v;
-      __syncwarp();
-    }
-    for (uint32_t d = lane; d < D; d += 32) {
+    } else for (uint32_t d = lane; d < D; d += 32) {
       uint32_t nz = 0;
       for (uint32_t q = 0, e = d % (uint32_t)bs; q < bs; ++q) {  // lanes start apart: other banks
         nz += blk[d * bs + e] != T(0);

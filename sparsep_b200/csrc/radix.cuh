@@ -5,15 +5,19 @@
 //   hist     per 4096-element tile, counts of each digit  -> hist[d][tile]
 //   scan     exclusive scan of hist in digit-major order (three launches)
 //   scatter  each element to scan[d][tile] + (earlier elements of its tile with
-//            digit d).  A warp takes 512 consecutive elements, 32 at a time;
-//            __match_any_sync gives the rank among the lanes with the same digit
+//            digit d).  A warp takes 256 consecutive elements, 32 at a time;
+//            a vote per digit bit gives the rank among the lanes with the same digit
 //            and the warp's own counter per digit the rank before that, so the
-//            warps meet only twice.  Keys and payloads then go through shared
-//            memory one after the other, so that a digit's elements leave as runs
-//            of consecutive addresses.
-// Bound by HBM: an element's record is read and written once per pass.  With
-// 4-bit digits, 1024-element tiles and three barriers per 256 elements, 10.5 M
-// 32-bit keys and their indices took 107 us per pass and 5 passes for 19 bits.
+//            warps meet only twice.  Keys, payloads and values then go through
+//            shared memory, so that a digit's elements leave as runs of
+//            consecutive addresses.
+// Bound by HBM in the limit (a record is read and written once per pass: 38 us for
+// 10.5 M records of 12 bytes); a pass takes 12 us (hist) + 10 (scan) + 80 (scatter),
+// the scatter's ranking and its address arithmetic having half of the issue slots.
+// 512 threads and two CTAs per SM: 1024 threads are 8 to 20 % slower, 3 CTAs at 42
+// registers no faster.  With 256 threads of 16 elements and __match_any_sync the
+// scatter took 236 us; with 4-bit digits, 1024-element tiles and three barriers per
+// 256 elements, keys and indices alone 107 us per pass and 5 passes for 19 bits.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -24,8 +28,8 @@ namespace radix {
 namespace {  // internal linkage: every translation unit that sorts gets its own kernels
 
 constexpr int NT = 256;            // threads per CTA
-constexpr int IPT = 16;            // elements per thread per tile
-constexpr int TILE = NT * IPT;
+constexpr int TILE = 4096;         // elements per tile
+constexpr int SNT = 512;           // threads of the scatter: 8 elements each, 64 registers
 constexpr int MAX_BITS = 7;        // bits of a digit
 constexpr int MAX_RADIX = 1 << MAX_BITS;
 constexpr unsigned FULL = 0xffffffffu;
@@ -37,16 +41,24 @@ __global__ void __launch_bounds__(NT) hist(const K *__restrict__ key, uint32_t n
   const int warp = threadIdx.x >> 5, radix = 1 << bits;
   for (int i = threadIdx.x; i < NT / 32 * MAX_RADIX; i += NT) (&c[0][0])[i] = 0;
   __syncthreads();
+  constexpr int IPT = TILE / NT;
   const uint32_t base = blockIdx.x * TILE;
-#pragma unroll 8
+  // all loads first: left to the compiler, each waited for the counter before it
+  // (28 instead of 12 us for 10.5 M keys)
+  K k[IPT];
+#pragma unroll
   for (int r = 0; r < IPT; ++r) {
     const uint32_t i = base + r * NT + threadIdx.x;
-    if (i < n) {
-      const K k = key[i];
-      if (bad && k >= bound) atomicExch(bad, 1);  // first pass only: keys must be < bound
-      atomicAdd(&c[warp][(uint32_t)(k >> shift) & (radix - 1)], 1u);
-    }
+    k[r] = i < n ? key[i] : K(0);
   }
+  bool out = false;
+#pragma unroll
+  for (int r = 0; r < IPT; ++r)
+    if (base + r * NT + threadIdx.x < n) {
+      out |= k[r] >= bound;
+      atomicAdd(&c[warp][(uint32_t)(k[r] >> shift) & (radix - 1)], 1u);
+    }
+  if (bad && out) atomicExch(bad, 1);  // first pass only: keys must be < bound
   __syncthreads();
   if (threadIdx.x < radix) {
     uint32_t t = 0;
@@ -138,100 +150,131 @@ __global__ void __launch_bounds__(NT) scan_down(uint32_t *__restrict__ h, uint32
 // null) and, unless V is NoValue, a value.
 struct NoValue {};
 
+// The lanes of the warp that have this lane's digit d, a vote per bit:
+// __match_any_sync takes as many steps as the warp has different digits (142 instead
+// of 92 us per pass over 10.5 M records).
+__device__ __forceinline__ uint32_t same_digit(uint32_t d) {
+  uint32_t same = FULL;
+#pragma unroll
+  for (int b = 0; b < MAX_BITS; ++b) {
+    const int32_t mine = (int32_t)(d << (31 - b)) >> 31;  // the bit in all places
+    same &= ~(__ballot_sync(FULL, mine) ^ mine);
+  }
+  return same;
+}
+
+template <typename K, typename V> struct Stage {  // a tile's records in shared memory
+  static constexpr size_t VALUES = TILE * sizeof(K);
+  static constexpr size_t WORDS = VALUES + (std::is_same<V, NoValue>::value ? 0 : TILE * sizeof(V));
+  static constexpr size_t BYTES = WORDS + TILE * 4;
+};
+
 template <typename K, typename V>
-__global__ void __launch_bounds__(NT) scatter(const K *__restrict__ key, const uint32_t *__restrict__ w_in,
+__global__ void __launch_bounds__(SNT, 2) scatter(const K *__restrict__ key, const uint32_t *__restrict__ w_in,
                                               const V *__restrict__ v_in, uint32_t n, int shift, int bits, uint32_t nt,
                                               const uint32_t *__restrict__ off, K *__restrict__ key_out,
                                               uint32_t *__restrict__ w_out, V *__restrict__ v_out) {
   constexpr bool VALUE = !std::is_same<V, NoValue>::value;
-  constexpr size_t UNIT = sizeof(K) > sizeof(V) ? sizeof(K) : sizeof(V);
-  __shared__ __align__(16) unsigned char stage[TILE * (UNIT > 4 ? UNIT : 4)];
-  __shared__ uint32_t cnt[NT / 32][MAX_RADIX];
+  constexpr int IPT = TILE / SNT, WARPS = SNT / 32;
+  extern __shared__ __align__(16) unsigned char stage[];  // Stage<K, V>::BYTES: keys, values, words
+  K *sk = reinterpret_cast<K *>(stage);
+  V *sv = reinterpret_cast<V *>(stage + Stage<K, V>::VALUES);
+  uint32_t *sw = reinterpret_cast<uint32_t *>(stage + Stage<K, V>::WORDS);
+  __shared__ uint32_t cnt[WARPS][MAX_RADIX];
   __shared__ uint32_t first[MAX_RADIX];  // of the tile's elements, the first of each digit
   __shared__ uint32_t dst[MAX_RADIX];    // its place in the output less that
+  __shared__ uint32_t sums[4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, radix = 1 << bits;
   const uint32_t base = blockIdx.x * TILE, here = n - base < TILE ? n - base : TILE;
-  for (int i = threadIdx.x; i < NT / 32 * MAX_RADIX; i += NT) (&cnt[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < WARPS * MAX_RADIX; i += SNT) (&cnt[0][0])[i] = 0;
   __syncthreads();
-  // this thread's elements: 32 apart, in the warp's 512
+  // this thread's elements: 32 apart, in the warp's share
   const uint32_t mine = warp * (32 * IPT) + lane;
-  K k[IPT];
-  uint32_t pos[IPT];
+  auto tile = [&](auto whole) {  // whole: TILE elements
+    constexpr bool WHOLE = decltype(whole)::value;
+    auto in = [&](int r) { return WHOLE || mine + r * 32 < here; };
+    auto digit = [&](K x) { return (uint32_t)(x >> shift) & (radix - 1); };
+    const K *kp = key + base + mine;
+    K k[IPT];
+    uint32_t w[IPT], pos[IPT];
 #pragma unroll
-  for (int r = 0; r < IPT; ++r) k[r] = mine + r * 32 < here ? key[base + mine + r * 32] : K(0);
+    for (int r = 0; r < IPT; ++r) k[r] = in(r) ? kp[r * 32] : K(0);
+    if (w_in) {
+      const uint32_t *wp = w_in + base + mine;
 #pragma unroll
-  for (int r = 0; r < IPT; ++r) {
-    const bool in = mine + r * 32 < here;
-    const uint32_t d = in ? (uint32_t)(k[r] >> shift) & (radix - 1) : MAX_RADIX;  // the others form their own group
-    const unsigned same = __match_any_sync(FULL, d);
-    const int leader = __ffs(same) - 1;
-    uint32_t before = 0;
-    if (in && lane == leader) {
-      before = cnt[warp][d];
-      cnt[warp][d] = before + __popc(same);
+      for (int r = 0; r < IPT; ++r) w[r] = in(r) ? wp[r * 32] : 0u;
+    } else {
+#pragma unroll
+      for (int r = 0; r < IPT; ++r) w[r] = base + mine + r * 32;
     }
-    pos[r] = __shfl_sync(FULL, before, leader) + __popc(same & ((1u << lane) - 1u));
-    __syncwarp();
-  }
-  __syncthreads();
-  uint32_t all = 0;
-  if (threadIdx.x < radix)
 #pragma unroll
-    for (int w = 0; w < NT / 32; ++w) {
-      const uint32_t c = cnt[w][threadIdx.x];
-      cnt[w][threadIdx.x] = all;
-      all += c;
+    for (int r = 0; r < IPT; ++r) {
+      uint32_t same = same_digit(digit(k[r]));
+      if constexpr (!WHOLE) same &= __ballot_sync(FULL, in(r));
+      const int leader = __ffs(same) - 1;
+      uint32_t before = 0;
+      if (in(r) && lane == leader) {
+        before = cnt[warp][digit(k[r])];
+        cnt[warp][digit(k[r])] = before + __popc(same);
+      }
+      pos[r] = __shfl_sync(FULL, before, leader < 0 ? 0 : leader) + __popc(same & ((1u << lane) - 1u));
+      __syncwarp();
     }
-  uint32_t total;
-  const uint32_t f = block_scan(all, &total);
-  if (threadIdx.x < radix) {
-    first[threadIdx.x] = f;
-    dst[threadIdx.x] = off[(size_t)threadIdx.x * nt + blockIdx.x] - f;
-  }
-  __syncthreads();
-  K *sk = reinterpret_cast<K *>(stage);
+    V v[IPT];
+    if constexpr (VALUE) {
+      const V *vp = v_in + base + mine;
 #pragma unroll
-  for (int r = 0; r < IPT; ++r)
-    if (mine + r * 32 < here) {
-      const uint32_t d = (uint32_t)(k[r] >> shift) & (radix - 1);
-      pos[r] += first[d] + cnt[warp][d];
-      sk[pos[r]] = k[r];
+      for (int r = 0; r < IPT; ++r)
+        if (in(r)) v[r] = vp[r * 32];
     }
-  __syncthreads();
-  uint32_t to[IPT];  // where the staged elements threadIdx.x, threadIdx.x + NT, ... go
-#pragma unroll
-  for (int j = 0; j < IPT; ++j) {
-    const uint32_t q = threadIdx.x + j * NT;
-    if (q < here) {
-      const K kk = sk[q];
-      to[j] = dst[(uint32_t)(kk >> shift) & (radix - 1)] + q;
-      key_out[to[j]] = kk;
-    }
-  }
-  __syncthreads();
-  uint32_t *sw = reinterpret_cast<uint32_t *>(stage);
-#pragma unroll
-  for (int r = 0; r < IPT; ++r)
-    if (mine + r * 32 < here) sw[pos[r]] = w_in ? w_in[base + mine + r * 32] : base + mine + r * 32;
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < IPT; ++j) {
-    const uint32_t q = threadIdx.x + j * NT;
-    if (q < here) w_out[to[j]] = sw[q];
-  }
-  if constexpr (VALUE) {
     __syncthreads();
-    V *sv = reinterpret_cast<V *>(stage);
+    uint32_t all = 0, inc = 0;
+    if (threadIdx.x < MAX_RADIX) {
+      if (threadIdx.x < radix)
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) {
+          const uint32_t c = cnt[q][threadIdx.x];
+          cnt[q][threadIdx.x] = all;
+          all += c;
+        }
+      inc = all;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (lane == 31) sums[warp] = inc;
+    }
+    __syncthreads();
+    if (threadIdx.x < radix) {
+      uint32_t f = inc - all;
+      for (int q = 0; q < warp; ++q) f += sums[q];
+      first[threadIdx.x] = f;
+      dst[threadIdx.x] = off[(size_t)threadIdx.x * nt + blockIdx.x] - f;
+    }
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < IPT; ++r)
-      if (mine + r * 32 < here) sv[pos[r]] = v_in[base + mine + r * 32];
+      if (in(r)) {
+        const uint32_t p = pos[r] + first[digit(k[r])] + cnt[warp][digit(k[r])];
+        sk[p] = k[r];
+        sw[p] = w[r];
+        if constexpr (VALUE) sv[p] = v[r];
+      }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
-      const uint32_t q = threadIdx.x + j * NT;
-      if (q < here) v_out[to[j]] = sv[q];
+      const uint32_t q = threadIdx.x + j * SNT;
+      if (WHOLE || q < here) {
+        const K kk = sk[q];
+        const uint32_t to = dst[digit(kk)] + q;
+        key_out[to] = kk;
+        w_out[to] = sw[q];
+        if constexpr (VALUE) v_out[to] = sv[q];
+      }
     }
-  }
+  };
+  if (here == TILE) tile(std::true_type{}); else tile(std::false_type{});
 }
 
 // Passes for `bits` bits (at least one, so that the outputs are produced even for
@@ -262,7 +305,10 @@ template <typename K, typename V>
 cudaError_t scatter_pass(const K *key, const uint32_t *w_in, const V *v_in, uint32_t n, int shift, int bits,
                          const uint32_t *counts, K *key_out, uint32_t *w_out, V *v_out, cudaStream_t s) {
   const uint32_t nt = (uint32_t)(((uint64_t)n + TILE - 1) / TILE);
-  scatter<K, V><<<nt, NT, 0, s>>>(key, w_in, v_in, n, shift, bits, nt, counts, key_out, w_out, v_out);
+  constexpr size_t bytes = Stage<K, V>::BYTES;
+  if (cudaError_t e = cudaFuncSetAttribute(scatter<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes))
+    return e;
+  scatter<K, V><<<nt, SNT, bytes, s>>>(key, w_in, v_in, n, shift, bits, nt, counts, key_out, w_out, v_out);
   return cudaGetLastError();
 }
 

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(SNT, 2) scatter(const K *__restrict__ key, con
       pos[r] = __shfl_sync(FULL, before, leader < 0 ? 0 : leader) + __popc(same & ((1u << lane) - 1u));
       __syncwarp();
     }
-    V v[IPT];
+    [[maybe_unused]] V v[IPT];
     if constexpr (VALUE) {
       const V *vp = v_in + base + mine;
 #pragma unroll

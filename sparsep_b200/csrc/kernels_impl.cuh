@@ -4,16 +4,20 @@
 // One kernel template executes a list of work items (device.cuh: Item); one
 // CTA runs one item.  The item kinds cover every reference kernel family:
 //   CSR rows  (spmv/1D/CSR-*/dpu/task.c:31-215, spmv/2D/*DCSR/dpu/task.c)
-//       -> L lanes per row (L = 1..32), 128-bit loads of colind / values
+//       -> products of a chunk of rows through shared memory (csr_stream), or
+//          L lanes per row (L = 1..32); 128-bit loads of colind / values
 //   CSR long-row chunks (no reference counterpart; the nnz balance remedy of
 //       partition_by_nnz pushed below row granularity) -> CTA-wide reduction
 //   COO elements (spmv/1D/COO-nnz/dpu/task.c lf :21-679, lb-fg :686-1338)
-//       -> lock-free: block segmented scan + carries fixed up by the last CTA
-//       -> atomic:    warp segmented scan + red.global per row run
-//   BCSR block rows (spmv/1D/BCSR-nnz/dpu/task.c:231-380) -> dense block in
-//       registers, L lanes per block row
-//   BCOO blocks (spmv/1D/BCOO-nnz/dpu/task.c:22-894) -> as COO with a
-//       row-block-wide payload
+//       -> a stream of elements per warp, summed per row by segmented scans
+//          (coo_items); rows that items share: lock-free, by the last item to
+//          arrive, in item order, or red.global
+//   BCSR block rows (spmv/1D/BCSR-nnz/dpu/task.c:231-380) -> chunks of blocks in
+//       shared memory (bcsr_chunks), or for the block sizes without a template
+//       the block in registers, L lanes per block row (bcsr_rows)
+//   BCOO blocks (spmv/1D/BCOO-nnz/dpu/task.c:22-894) -> chunks likewise
+//       (bcoo_chunks), or a block segmented scan with a row-block-wide payload
+//       and carries added by the last CTA (bcoo_lf)
 // 2D tiles are items whose x-segment is staged into shared memory by bulk
 // (TMA) copies; their partial y goes to per-stripe slices merged on the device.
 #pragma once
@@ -952,7 +956,8 @@ __device__ void arrive(const Params<T> &P, T *out, uint32_t item, uint64_t row_e
 // stream over chunks brought into shared memory by bulk copies 116 us, with
 // windows dealt out through 1.5 KB of it per warp 112 us, 8 warps per CTA 100 us,
 // x a window ahead (64 registers) 107 us.  FP64 203 -> 102 us; equal tiles 16 x 16
-// of the 524,309-row matrix 116 -> 94 us.
+// of the 524,309-row matrix, most of whose rows are empty, 116 -> 76 us (94 while
+// each lane zeroed the rows before its own nonzeros one by one).
 //
 // GROUPS: the planner numbered the rows that items share; otherwise the item's
 // first row goes to y as far as the item has it, and a last row that goes on in
@@ -1053,14 +1058,16 @@ __device__ __forceinline__ void coo_stream(const Params<T> &P, const Item &it, c
         hb |= (d ? 1u : 0u) << j;
         gap = d > gap ? d : gap;
       }
+      const uint32_t before = last;
+      last = __shfl_sync(FULL, k[K - 1], 31);
       if constexpr (!ATOMIC) {
-        if (__any_sync(FULL, gap > 1)) {  // rows without nonzeros in between
-          zeros(prev, k[0], 1, 1);
-#pragma unroll
-          for (int j = 1; j < K; ++j) zeros(k[j - 1], k[j], 1, 1);
+        // Rows without nonzeros in between: all rows between the window's first and
+        // last are zeroed side by side, and those with nonzeros written after that.
+        if (__any_sync(FULL, gap > 1)) {
+          zeros(before, last, lane + 1, 32);
+          __syncwarp();
         }
       }
-      last = __shfl_sync(FULL, k[K - 1], 31);
       row_window<K, A>(S, v, hb, k, &ends.first[warp], write);
     }
     leave_ends<A>(ends, warp, S);

@@ -105,7 +105,8 @@ typedef struct sparsep_opts {
   int32_t part_balance;    /* sparsep_balance across parts (reference: DPUs)     */
   int32_t worker_balance;  /* sparsep_balance across workers (reference: tasklets)*/
   int32_t sync;            /* sparsep_sync                                       */
-  int32_t nr_parts;        /* reference NR_DPUS: parts = CTAs (BCSR: 1+); 0 = auto */
+  int32_t nr_parts;        /* reference NR_DPUS: parts, run by one or more CTAs  */
+                           /* each (lanes > 0: by one); 0 = auto                 */
   int32_t nr_workers;      /* reference NR_TASKLETS: warps per part; 0 = auto    */
   int32_t vert_partitions; /* reference -v (2D schemes built from COO)           */
   int32_t row_block_size;  /* reference -r (BCSR/BCOO built from CSR)            */

@@ -301,14 +301,19 @@ static void number_long_rows(std::vector<Item> &items) {
 
 // Element (COO) / block (BCOO) range [e0, e1) of a tile whose keys (rows or
 // block rows) run over [k_lo, k_hi): split into items, each owning the keys
-// from its first unit's key to the next item's first key.
+// from its first unit's key to the next item's first key.  No item is of more than
+// `cap` units, and those of more than twice `aim` are cut further (0: no limit).
 template <typename KeyFn>
 static void elem_tile_items(std::vector<Item> &items, const Tile &t, uint64_t e0, uint64_t e1, uint32_t k_lo,
-                            uint32_t k_hi, const std::vector<uint64_t> &cuts_in, uint64_t cap, const KeyFn &key) {
+                            uint32_t k_hi, const std::vector<uint64_t> &cuts_in, uint64_t cap, uint64_t aim, const KeyFn &key) {
   std::vector<uint64_t> b;  // boundaries: the cuts inside (e0, e1), and every cap units in between
   b.push_back(e0);
   auto upto = [&](uint64_t c) {
     while (cap && c - b.back() > cap) b.push_back(b.back() + cap);
+    if (aim && c - b.back() > 2 * aim) {  // even pieces, on the 16-byte reads' boundaries
+      const uint64_t from = b.back(), n = (c - from + aim - 1) / aim;
+      for (uint64_t i = 1; i < n; ++i) b.push_back((from + (c - from) / n * i + 3) & ~3ull);
+    }
     b.push_back(c);
   };
   for (uint64_t c : cuts_in)
@@ -938,11 +943,26 @@ static int plan_csr(const typename Types<T>::csr *A, const sparsep_opts *o, spar
   t.row_end = A->nrows;
   const bool faithful = oo.nr_parts > 0;
   bool has_long = false;
+  uint32_t nparts = 0;  // that have rows
   if (faithful) {
     std::vector<uint32_t> split(oo.nr_parts + 2);
     if (oo.part_balance == SPARSEP_BAL_ROW) sparsep_partition_by_row(A->nrows, oo.nr_parts, split.data());
     else sparsep_partition_by_nnz(A->rowptr, A->nrows, oo.nr_parts, split.data());
-    for (int i = 0; i < oo.nr_parts; ++i) csr_tile_items(items, t, A->rowptr, split[i], split[i + 1], oo, true, false);
+    // The row kernel's parts are cut into items of the slim form: a part is where
+    // items end, not what one CTA runs alone, so that parts of unequal work (equal
+    // rows, a long row) don't wait for the longest.  Fixed lanes per row stay with
+    // a CTA per part, whose warps share it by worker_balance.  2048 parts by nonzeros
+    // of 524,288 rows and 8.4 M nonzeros, FP32 power-law / uniform / banded: 108 / 58 /
+    // 32 us with a CTA per part, 47 / 48 / 28 cut; 64 parts 350 / 277 / 202, now 48 /
+    // 52 / 26.
+    p->slim = oo.lanes == 0;
+    for (int i = 0; i < oo.nr_parts; ++i) {
+      nparts += split[i] < split[i + 1];
+      csr_tile_items(items, t, A->rowptr, split[i], split[i + 1], oo, !p->slim, p->slim,
+                     csr_item_nnz(sizeof(T), A->nnz, p->sms), csr_chunk_nnz(sizeof(T), true) / 4);
+    }
+    number_long_rows(items);
+    for (auto &it : items) has_long |= it.kind == ITEM_LONG;
   } else {
     // a split plan when the heavy rows' x gathers are worth moving into
     // shared-memory stripes (host arrays only: the re-layout reads columns)
@@ -977,6 +997,7 @@ static int plan_csr(const typename Types<T>::csr *A, const sparsep_opts *o, spar
   p->n_idx = p->n_val = (uint64_t)A->nnz + 16;
   p->info.compulsory_bytes = compulsory_csr(A->nnz, A->nrows, A->ncols, sizeof(T));
   if ((st = finish_plan(p, items, oo))) return st;
+  if (faithful) p->info.items = nparts;
   p->t[0] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   *out = guard.release();
   return SPARSEP_OK;
@@ -1002,13 +1023,27 @@ static int plan_csr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t n
   p->nnz = nnz;
   std::vector<Item> items;
   const bool faithful = oo.nr_parts > 0;
+  // A CTA per tile only for fixed lanes per row.  The row kernel's items are of the
+  // slim form unless they bring their tile's x along.  8 x 8 tiles of 524,288 rows and
+  // 8.4 M nonzeros, power-law / uniform / banded, automatic items of 4080 nonzeros and
+  // now: FP32 73 / 69 / 50 -> 69 / 67 / 48 us, FP64 107 / 89 / 82 -> 94 / 83 / 79; a CTA
+  // per tile 598 / 479 / 1564 us (FP32).
+  bool staged = false;
+  uint32_t nparts = 0;  // tiles that have rows
+  for (const Tile &t : tiles_in) staged |= stage_width(p, oo, t.xw) != 0;
+  p->slim = oo.lanes == 0 && !staged && (faithful || oo.item_nnz <= 0);
   for (size_t i = 0; i < tiles_in.size(); ++i) {
     Tile t = tiles_in[i];
     t.xw = stage_width(p, oo, t.xw);
-    csr_tile_items(items, t, drowptr + t.ptr_base, ranges[i].first, ranges[i].second, oo, faithful, false);
+    nparts += ranges[i].first < ranges[i].second;
+    csr_tile_items(items, t, drowptr + t.ptr_base, ranges[i].first, ranges[i].second, oo, faithful && oo.lanes, p->slim,
+                   p->slim ? csr_item_nnz(sizeof(T), nnz, p->sms) : 0, csr_chunk_nnz(sizeof(T), true) / 4);
   }
   (void)H;
-  set_out_mode(p, oo, V, false, 1);
+  number_long_rows(items);
+  bool has_long = false;
+  for (const Item &it : items) has_long |= it.kind == ITEM_LONG;
+  set_out_mode(p, oo, V, has_long, 1);
   if ((st = upload(p, drowptr, rowptr_len, 4, 16, (const void **)&p->rowptr))) return st;
   if ((st = upload(p, dcolind, nnz, 4, 16, (const void **)&p->colind))) return st;
   if ((st = upload(p, dval, nnz, sizeof(T), 16, &p->val))) return st;
@@ -1016,6 +1051,7 @@ static int plan_csr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t n
   p->n_idx = p->n_val = nnz + 16;
   p->info.compulsory_bytes = compulsory_csr(nnz, nrows, ncols, sizeof(T));
   if ((st = finish_plan(p, items, oo))) return st;
+  if (faithful) p->info.items = nparts;
   p->t[0] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   *out = guard.release();
   return SPARSEP_OK;
@@ -1141,9 +1177,12 @@ static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint6
   p->cb = cb;
   std::vector<Item> items;
   const bool faithful = oo.nr_parts > 0;
-  // COO, and BCOO in chunks of at most `cap` blocks: shared rows are numbered;
-  // the general BCOO kernel leaves carries
+  // COO, and BCOO in chunks of at most `cap` blocks: shared rows are numbered; the
+  // general BCOO kernel leaves carries.  COO parts much larger than an automatic item
+  // are cut like CSR's; up to twice its size they stay whole, since cutting parts that
+  // are even already only adds items (2048 parts of 4096 nonzeros: 49 -> 54 us).
   const uint64_t cap = fmt == SPARSEP_FMT_COO ? 0 : bcoo_chunk_blocks(rb, cb, sizeof(T));
+  const uint64_t aim = fmt == SPARSEP_FMT_COO ? per_item : 0;
   p->by_groups = fmt == SPARSEP_FMT_COO || cap != 0;
   uint64_t nparts = 0;
   set_out_mode(p, oo, V, true, fmt == SPARSEP_FMT_BCOO ? rb : 1);
@@ -1155,7 +1194,7 @@ static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint6
     for (uint64_t c : cuts) nparts += c > et.e0 && c < et.e1;
     ++nparts;
     const size_t first = items.size();
-    elem_tile_items(items, t, et.e0, et.e1, et.k_lo, et.k_hi, cuts, cap, key);
+    elem_tile_items(items, t, et.e0, et.e1, et.k_lo, et.k_hi, cuts, cap, aim, key);
     if (p->by_groups && p->out_mode != OUT_ATOMIC) group_shared_rows(items, first, p->ngroups, key);
   }
   if (cap) {

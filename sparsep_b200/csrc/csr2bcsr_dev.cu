@@ -124,7 +124,7 @@ __device__ __forceinline__ void each_block_row(const uint32_t *__restrict__ rowp
 }
 
 // cnt[I] = blocks of block row I, for block rows of (lo, LIM] nonzeros (and the
-// empty ones); flag[0]: a bad column, flag[1]: a longer block row.
+// empty ones); flag[0]: a bad column among these, flag[1]: a longer block row.
 template <int LIM>
 __global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
     count_blocks(const uint32_t *__restrict__ rowptr, uint32_t nrows, const uint32_t *__restrict__ colind, uint32_t nnz,
@@ -515,6 +515,8 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
   int st = c2b_err(sparsep::ws_malloc((void **)&bad, 2 * sizeof(int), s));
   if (st) return st;
   uint32_t *dnb = reinterpret_cast<uint32_t *>(bad + 1);
+  int h_bad = 0;
+  st = c2b_err(cudaMemsetAsync(bad, 0, 2 * sizeof(int), s));
   // scratch, in 32-bit words: input keys (2n), two key buffers (2n each), the
   // radix scratch, the head flags (n) with their scan sums (nbs + 8), and
   // the block starts (n + 1).  After the sort the input-key buffer holds the
@@ -523,7 +525,7 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
   const size_t rsw = (radix_scratch_words(nnz) + 1) & ~(size_t)1;
   const size_t words = 6 * (size_t)nnz + rsw + ((size_t)nnz + nbs + 8) + ((size_t)nnz + 1) + 8;
   uint32_t *buf = nullptr;
-  st = c2b_err(sparsep::ws_malloc((void **)&buf, words * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&buf, words * 4, s));
   if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->row, (size_t)nnz * 4, s));
   if (!st) {
     uint64_t *key = reinterpret_cast<uint64_t *>(buf), *k0 = key + nnz, *k1 = k0 + nnz;
@@ -542,8 +544,11 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
       block_starts<<<grid_for(nnz), NT, 0, s>>>(skey, nnz, flag, bstart_tmp, bkey_tmp, dnb);
       st = c2b_err(cudaGetLastError());
     }
+    // the columns of the longer block rows are looked at here for the first time
+    if (!st) st = c2b_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (!st) st = c2b_err(cudaMemcpyAsync(&L->nblocks, dnb, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (!st) st = c2b_err(cudaStreamSynchronize(s));
+    if (!st && h_bad) st = SPARSEP_EINVAL;
     if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->sidx, (size_t)nnz * 4, s));
     if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bstart, ((size_t)L->nblocks + 1) * 4, s));
     if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bkey, (size_t)std::max<uint32_t>(L->nblocks, 1) * 8, s));

@@ -17,7 +17,7 @@
 //   where they fit (else in place), 32 nonzeros at a time in input order, so that
 //   a later duplicate of a position overwrites an earlier one; the nonzero values
 //   of each block counted.
-// Matrices with a block row of more than LIM_LARGE nonzeros go through a sort of
+// Matrices with a block row of more than LIM nonzeros go through a sort of
 // all nonzeros by (block row, block column) instead (radix.cuh):
 //   keys   per nonzero k: its row r (binary search in rowptr) and the key
 //          (r / rb) << jbits | colind[k] / cb
@@ -53,13 +53,16 @@ __global__ void check_rowptr(const uint32_t *__restrict__ rowptr, uint32_t nrows
 // ---------------------------------------------------------------------------
 // A block row per warp
 // ---------------------------------------------------------------------------
-constexpr int LIM_SMALL = 256, LIM_LARGE = 2048;  // nonzeros of a block row
-constexpr uint32_t EMPTY = 0xFFFFFFFFu;           // no block column: columns are below 2^32 - 1
-template <int LIM> struct Table {
-  static constexpr int SLOTS = 2 * LIM;
-  static constexpr int WARPS = LIM == LIM_SMALL ? 4 : 1;  // block rows per CTA
-  static constexpr int BLOCKS = LIM == LIM_SMALL ? 2048 : 8192;  // bytes for a block row's blocks
-};
+// Nonzeros of a block row that go through a table.  Layout and fill of 4 M nonzeros,
+// 4x4, block rows of 250: 665 us with scattered columns (250 blocks each), 172 with
+// 32 blocks each; by the sort, block rows of 260: 840 and 550 us.  A table for up to
+// 2048, a warp per block row with its block columns ranked pair by pair, was slower
+// than the sort from the start: 3.5 ms at 260 scattered nonzeros, 70 at 2000.
+constexpr int LIM = 256;
+constexpr uint32_t EMPTY = 0xFFFFFFFFu;  // no block column: columns are below 2^32 - 1
+constexpr int SLOTS = 2 * LIM;
+constexpr int WARPS = 4;      // block rows per CTA
+constexpr int BLOCKS = 2048;  // bytes for a block row's blocks
 
 struct BlockRow {
   uint32_t r0, k0, k1;  // first row, nonzeros [k0, k1)
@@ -101,44 +104,26 @@ __device__ __forceinline__ uint32_t find(const uint32_t *t, uint32_t J, int shif
   for (uint32_t i = 0; i < mask && t[s] != J; ++i) s = (s + 1) & mask;
   return s;
 }
-// Calls f(I) with the whole warp for the block rows I of (lo, LIM] nonzeros: a warp
-// per block row for the many short ones, 32 looked over at a time for the few long ones.
-template <int LIM, typename F>
-__device__ __forceinline__ void each_block_row(const uint32_t *__restrict__ rowptr, uint32_t nrows, uint32_t nnz,
-                                               uint32_t rb, uint32_t nbr, uint32_t lo, F f) {
-  constexpr uint32_t W = Table<LIM>::WARPS;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if constexpr (LIM == LIM_SMALL) {
-    for (uint64_t I = (uint64_t)blockIdx.x * W + warp; I < nbr; I += (uint64_t)gridDim.x * W) f((uint32_t)I);
-  } else {
-    for (uint64_t I0 = ((uint64_t)blockIdx.x * W + warp) * 32; I0 < nbr; I0 += (uint64_t)gridDim.x * W * 32) {
-      uint32_t m = 0;
-      if (I0 + lane < nbr) {
-        const BlockRow b = block_row(rowptr, nrows, nnz, rb, (uint32_t)(I0 + lane));
-        m = b.k1 - b.k0;
-      }
-      for (uint32_t some = __ballot_sync(0xffffffffu, m > lo && m <= LIM); some; some &= some - 1)
-        f((uint32_t)I0 + __ffs(some) - 1);
-    }
-  }
+// Calls f(I) with the whole warp for every block row I.
+template <typename F> __device__ __forceinline__ void each_block_row(uint32_t nbr, F f) {
+  for (uint64_t I = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5); I < nbr; I += (uint64_t)gridDim.x * WARPS)
+    f((uint32_t)I);
 }
 
-// cnt[I] = blocks of block row I, for block rows of (lo, LIM] nonzeros (and the
-// empty ones); flag[0]: a bad column among these, flag[1]: a longer block row.
-template <int LIM>
-__global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
+// cnt[I] = blocks of block row I, for block rows of up to LIM nonzeros; flag[0]: a
+// bad column among these, flag[1]: a longer block row.
+__global__ void __launch_bounds__(32 * WARPS)
     count_blocks(const uint32_t *__restrict__ rowptr, uint32_t nrows, const uint32_t *__restrict__ colind, uint32_t nnz,
-                 uint32_t ncols, uint32_t rb, uint32_t cb, int cshift, uint32_t nbr, uint32_t lo,
-                 uint32_t *__restrict__ cnt, int *__restrict__ flag) {
-  using Tb = Table<LIM>;
-  __shared__ uint32_t table[Tb::WARPS][Tb::SLOTS];
+                 uint32_t ncols, uint32_t rb, uint32_t cb, int cshift, uint32_t nbr, uint32_t *__restrict__ cnt,
+                 int *__restrict__ flag) {
+  __shared__ uint32_t table[WARPS][SLOTS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  each_block_row<LIM>(rowptr, nrows, nnz, rb, nbr, lo, [&](uint32_t I) {
+  each_block_row(nbr, [&](uint32_t I) {
     const BlockRow br = block_row(rowptr, nrows, nnz, rb, I);
     const uint32_t m = br.k1 - br.k0;
-    if (m > LIM_LARGE && lane == 0) flag[1] = 1;
+    if (m > LIM && lane == 0) flag[1] = 1;
     if (m == 0 && lane == 0) cnt[I] = 0;
-    if (m <= lo || m > LIM) return;
+    if (m == 0 || m > LIM) return;
     const int shift = table_shift(m);
     uint32_t *t = table[warp];
     for (uint32_t i = lane; i < 1u << (32 - shift); i += 32) t[i] = EMPTY;
@@ -160,27 +145,26 @@ __global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
   });
 }
 
-template <typename T, int LIM>
-__global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
+template <typename T>
+__global__ void __launch_bounds__(32 * WARPS)
     fill_rows(const uint32_t *__restrict__ rowptr, uint32_t nrows, const uint32_t *__restrict__ colind, uint32_t nnz,
               uint32_t ncols, const T *__restrict__ values, uint32_t rb, uint32_t cb, int cshift, uint32_t nbr,
-              uint32_t lo, const uint32_t *__restrict__ browptr, uint32_t *__restrict__ bcolind, T *__restrict__ bval,
+              const uint32_t *__restrict__ browptr, uint32_t *__restrict__ bcolind, T *__restrict__ bval,
               uint32_t *__restrict__ nnz_per_block) {
-  using Tb = Table<LIM>;
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ uint32_t table[Tb::WARPS][Tb::SLOTS];
-  __shared__ uint16_t rank_of[Tb::WARPS][Tb::SLOTS];
-  __shared__ uint32_t list[Tb::WARPS][LIM];
-  __shared__ uint32_t count[Tb::WARPS];
-  __shared__ __align__(16) unsigned char blocks[Tb::WARPS][Tb::BLOCKS];
+  __shared__ uint32_t table[WARPS][SLOTS];
+  __shared__ uint16_t rank_of[WARPS][SLOTS];
+  __shared__ uint32_t list[WARPS][LIM];
+  __shared__ uint32_t count[WARPS];
+  __shared__ __align__(16) unsigned char blocks[WARPS][BLOCKS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t *t = table[warp], *l = list[warp];
   uint16_t *rk = rank_of[warp];
   const uint64_t bs = (uint64_t)rb * cb;
-  each_block_row<LIM>(rowptr, nrows, nnz, rb, nbr, lo, [&](uint32_t I) {
+  each_block_row(nbr, [&](uint32_t I) {
     const BlockRow br = block_row(rowptr, nrows, nnz, rb, I);
     const uint32_t m = br.k1 - br.k0;
-    if (m <= lo || m > LIM) return;
+    if (m == 0 || m > LIM) return;
     const int shift = table_shift(m);
     // all that memory has to give, at once: the first nonzeros, the rows' ends and the blocks' place
     constexpr int PRE = 4;
@@ -229,7 +213,7 @@ __global__ void __launch_bounds__(32 * Table<LIM>::WARPS)
     // the blocks: in shared memory where they fit, else where they belong
     T *gout = bval + b0 * bs;
     const uint64_t ne = D * bs;
-    const bool in_smem = ne * sizeof(T) <= (uint64_t)Tb::BLOCKS;
+    const bool in_smem = ne * sizeof(T) <= (uint64_t)BLOCKS;
     T *blk = in_smem ? reinterpret_cast<T *>(blocks[warp]) : gout;
     for (uint64_t e = lane; e < ne; e += 32) blk[e] = T(0);
     __syncwarp();
@@ -459,13 +443,9 @@ static int layout_rows(const uint32_t *rowptr, sparsep_bcsr_layout *L, bool *fit
       const int cs = col_shift(L->cb);
       if (L->nrows) check_rowptr<<<grid_for(L->nrows), NT, 0, s>>>(rowptr, L->nrows, L->nnz, flag);
       if (L->nnz) {
-        constexpr int W = Table<LIM_SMALL>::WARPS;
-        const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + W - 1) / W);
-        count_blocks<LIM_SMALL><<<grid, 32 * W, 0, s>>>(rowptr, L->nrows, L->colind, L->nnz, L->ncols, L->rb, L->cb, cs,
-                                                        L->nbr, 0, L->browptr, flag);
-        count_blocks<LIM_LARGE><<<std::min<uint32_t>(2048, L->nbr / 32 + 1), 32, 0, s>>>(rowptr, L->nrows, L->colind, L->nnz,
-                                                                                L->ncols, L->rb, L->cb, cs, L->nbr,
-                                                                                LIM_SMALL, L->browptr, flag);
+        const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + WARPS - 1) / WARPS);
+        count_blocks<<<grid, 32 * WARPS, 0, s>>>(rowptr, L->nrows, L->colind, L->nnz, L->ncols, L->rb, L->cb, cs,
+                                                 L->nbr, L->browptr, flag);
         sparsep::radix::scan_reduce<<<nb, sparsep::radix::NT, 0, s>>>(L->browptr, m, buf);
         sparsep::radix::scan_top<<<1, sparsep::radix::NT, 0, s>>>(buf, nb);
         sparsep::radix::scan_down<<<nb, sparsep::radix::NT, 0, s>>>(L->browptr, m, buf);
@@ -570,14 +550,10 @@ static int fill(const sparsep_bcsr_layout *L, const T *values, uint32_t *browptr
   if (L->browptr) {
     int st = c2b_err(cudaMemcpyAsync(browptr, L->browptr, ((size_t)L->nbr + 1) * 4, cudaMemcpyDeviceToDevice, s));
     if (!st && L->nblocks) {
-      constexpr int W = Table<LIM_SMALL>::WARPS;
       const int cs = col_shift(L->cb);
-      const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + W - 1) / W);
-      fill_rows<T, LIM_SMALL><<<grid, 32 * W, 0, s>>>(L->rowptr, L->nrows, L->colind, L->nnz, L->ncols, values, L->rb,
-                                                      L->cb, cs, L->nbr, 0, L->browptr, bcolind, bval, nnz_per_block);
-      fill_rows<T, LIM_LARGE><<<std::min<uint32_t>(2048, L->nbr / 32 + 1), 32, 0, s>>>(
-          L->rowptr, L->nrows, L->colind, L->nnz, L->ncols, values, L->rb, L->cb, cs, L->nbr, LIM_SMALL, L->browptr,
-          bcolind, bval, nnz_per_block);
+      const unsigned grid = (unsigned)std::min<uint64_t>(16384, ((uint64_t)L->nbr + WARPS - 1) / WARPS);
+      fill_rows<T><<<grid, 32 * WARPS, 0, s>>>(L->rowptr, L->nrows, L->colind, L->nnz, L->ncols, values, L->rb, L->cb,
+                                               cs, L->nbr, L->browptr, bcolind, bval, nnz_per_block);
       st = c2b_err(cudaGetLastError());
     }
     if (!st) st = c2b_err(cudaStreamSynchronize(s));

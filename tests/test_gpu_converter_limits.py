@@ -1,5 +1,7 @@
 """What the device converters refuse and how far they reach, in block rows of every
 length: a column past the last one is refused wherever it lies."""
+import time
+
 import numpy as np
 import pytest
 
@@ -33,3 +35,41 @@ def test_column_past_the_end_is_einval(longest, ncols, cb, where):
     layout = capi.BcsrLayout(drp.data_ptr(), dci.data_ptr(), 41, ncols, int(rowptr[-1]), 4, cb)
     assert layout.nblocks > 0
     layout.free()
+
+
+def convert_us(per, nnz=2_000_000):
+    """Time of layout and fill into 4x4 blocks, block rows of `per` nonzeros at random columns."""
+    import torch
+
+    nbr = nnz // per
+    nrows, ncols = 4 * nbr, 100_000
+    lens = np.full(nrows, per // 4)
+    lens[::4] += per % 4
+    rowptr = torch.from_numpy(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)).cuda()
+    nnz = nbr * per
+    g = torch.Generator(device="cuda").manual_seed(per)
+    colind = torch.randint(0, ncols, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    vals = torch.rand(nnz, generator=g, device="cuda")
+    times = []
+    for _ in range(5):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        layout = capi.BcsrLayout(rowptr.data_ptr(), colind.data_ptr(), nrows, ncols, nnz, 4, 4)
+        nb = layout.nblocks
+        i32 = dict(dtype=torch.int32, device="cuda")
+        bp, bc, npb = torch.empty(nbr + 1, **i32), torch.empty(nb, **i32), torch.empty(nb, **i32)
+        bv = torch.empty(nb * 16, device="cuda")
+        layout.fill("f32", vals.data_ptr(), bp.data_ptr(), bc.data_ptr(), bv.data_ptr(), npb.data_ptr())
+        torch.cuda.synchronize()
+        times.append((time.perf_counter() - t0) * 1e6)
+        layout.free()
+    return min(times)
+
+
+def test_no_length_of_a_block_row_is_out_of_line():
+    """The same number of nonzeros in block rows of every length: within a factor of
+    four of the longest ones, which are sorted."""
+    longest = convert_us(4000)
+    us = {per: convert_us(per) for per in (64, 256, 257, 500, 1000, 2000, 2048, 2049)}
+    print(us, longest)
+    assert max(us.values()) < 4 * longest

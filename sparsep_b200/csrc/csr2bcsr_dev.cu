@@ -45,7 +45,7 @@ constexpr int NT = 256;
 
 // rowptr[0] == 0, non-decreasing, rowptr[nrows] == nnz
 __global__ void check_rowptr(const uint32_t *__restrict__ rowptr, uint32_t nrows, uint32_t nnz, int *__restrict__ bad) {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
+  for (uint64_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
     if (rowptr[r] > rowptr[r + 1]) atomicExch(bad, 1);
   if (blockIdx.x == 0 && threadIdx.x == 0 && (rowptr[0] != 0 || rowptr[nrows] != nnz)) atomicExch(bad, 1);
 }
@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(32 * WARPS)
     for (uint32_t i = lane; i < 1u << (32 - shift); i += 32) t[i] = EMPTY;
     __syncwarp();
     uint32_t mine = 0;
-    for (uint32_t k = br.k0 + lane; k < br.k1; k += 32) {
-      uint32_t c = colind[k];
+    for (uint32_t i = lane; i < m; i += 32) {  // k0 + i of a lane past the end may pass 2^32: compare i
+      uint32_t c = colind[br.k0 + i];
       if (c >= ncols) {
         flag[0] = 1;
         c = 0;
@@ -172,12 +172,12 @@ __global__ void __launch_bounds__(32 * WARPS)
     T pv[PRE];
 #pragma unroll
     for (int q = 0; q < PRE; ++q) {
-      const uint32_t k = br.k0 + q * 32 + lane;
+      const uint32_t i = q * 32 + lane;
       pc[q] = 0;
       pv[q] = T(0);
-      if (k < br.k1) {
-        pc[q] = colind[k];
-        pv[q] = values[k];
+      if (i < m) {
+        pc[q] = colind[br.k0 + i];
+        pv[q] = values[br.k0 + i];
       }
     }
     const uint32_t rend = lane < rb && br.r0 + lane + 1 <= nrows ? rowptr[br.r0 + lane + 1] : 0xFFFFFFFFu;
@@ -196,9 +196,9 @@ __global__ void __launch_bounds__(32 * WARPS)
 #pragma unroll
     for (int q = 0; q < PRE; ++q) {
       ps[q] = 0;
-      if (br.k0 + q * 32 + lane < br.k1) ps[q] = enter(pc[q]);
+      if (q * 32 + lane < m) ps[q] = enter(pc[q]);
     }
-    for (uint32_t k = br.k0 + PRE * 32 + lane; k < br.k1; k += 32) enter(colind[k]);
+    for (uint32_t i = PRE * 32 + lane; i < m; i += 32) enter(colind[br.k0 + i]);
     __syncwarp();
     const uint32_t D = count[warp] < room ? count[warp] : room;  // equal, while colind is as it was counted
     for (uint32_t d = lane; d < D; d += 32) {
@@ -223,17 +223,18 @@ __global__ void __launch_bounds__(32 * WARPS)
     auto place_all = [&](auto zero) {  // positions as wide as this
       using P = decltype(zero);
       const P nel = (P)ne, bsz = (P)bs;
-      auto place = [&](uint32_t k, uint32_t c, T v, auto slot_of) {  // nonzeros [k, k + 32)
-        const bool in = k + lane < br.k1;
+      auto place = [&](uint32_t i, uint32_t c, T v, auto slot_of) {  // nonzeros [k0 + i, k0 + i + 32)
+        const bool in = i + lane < m;
+        const uint32_t k = br.k0 + i + lane;
         uint32_t rl = 0;  // row in the block: the block row's rows that end at or before this nonzero
         if (rb <= 32) {
-          for (uint32_t q = 0; q + 1 < rb; ++q) rl += __shfl_sync(FULL, rend, q) <= k + lane;
+          for (uint32_t q = 0; q + 1 < rb; ++q) rl += __shfl_sync(FULL, rend, q) <= k;
         } else if (in) {
           uint32_t a = 0, b = rb - 1;
           while (a < b) {
             const uint32_t mid = (a + b) >> 1;
             const uint64_t r = (uint64_t)br.r0 + mid + 1;
-            if (r <= nrows && rowptr[r] <= k + lane) a = mid + 1; else b = mid;
+            if (r <= nrows && rowptr[r] <= k) a = mid + 1; else b = mid;
           }
           rl = a;
         }
@@ -257,10 +258,10 @@ __global__ void __launch_bounds__(32 * WARPS)
       // input order: a later duplicate wins
 #pragma unroll
       for (int q = 0; q < PRE; ++q)
-        if (br.k0 + q * 32 < br.k1) place(br.k0 + q * 32, pc[q], pv[q], [&](uint32_t) { return ps[q]; });
-      for (uint32_t k = br.k0 + PRE * 32; k < br.k1; k += 32) {
-        const bool in = k + lane < br.k1;
-        place(k, in ? colind[k + lane] : 0, in ? values[k + lane] : T(0),
+        if (q * 32 < m) place(q * 32, pc[q], pv[q], [&](uint32_t) { return ps[q]; });
+      for (uint32_t i = PRE * 32; i < m; i += 32) {
+        const bool in = i + lane < m;
+        place(i, in ? colind[br.k0 + i + lane] : 0, in ? values[br.k0 + i + lane] : T(0),
               [&](uint32_t J) { return find(t, J, shift); });
       }
     };

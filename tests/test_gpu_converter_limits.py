@@ -73,3 +73,30 @@ def test_no_length_of_a_block_row_is_out_of_line():
     us = {per: convert_us(per) for per in (64, 256, 257, 500, 1000, 2000, 2048, 2049)}
     print(us, longest)
     assert max(us.values()) < 4 * longest
+
+
+def test_nonzeros_up_to_the_last_index():
+    """2^32 - 1 nonzeros: the last block rows end where a 32-bit index would wrap."""
+    import torch
+
+    nnz, per = 2**32 - 1, 255
+    nrows = nnz // per  # exactly: 2^32 - 1 = 255 x 16,843,009
+    free = torch.cuda.mem_get_info()[0]
+    if free < 40 << 30:
+        pytest.skip("needs 40 GB of device memory")
+    rowptr = torch.arange(nrows + 1, device="cuda", dtype=torch.int64).mul_(per).to(torch.int32)  # mod 2^32
+    colind = torch.zeros(nnz, dtype=torch.int32, device="cuda")
+    colind[-1] = 5  # the last row has a block of its own for its last nonzero
+    vals = torch.zeros(nnz, dtype=torch.int8, device="cuda")
+    vals[-1], vals[-2], vals[0] = 7, 3, 9
+    layout = capi.BcsrLayout(rowptr.data_ptr(), colind.data_ptr(), nrows, 8, nnz, 1, 4)
+    assert layout.nblocks == nrows + 1
+    i32 = dict(dtype=torch.int32, device="cuda")
+    bp, bc, npb = torch.empty(nrows + 1, **i32), torch.empty(nrows + 1, **i32), torch.empty(nrows + 1, **i32)
+    bv = torch.full(((nrows + 1) * 4,), 1, dtype=torch.int8, device="cuda")
+    layout.fill("i8", vals.data_ptr(), bp.data_ptr(), bc.data_ptr(), bv.data_ptr(), npb.data_ptr())
+    layout.free()
+    assert bp[-3:].tolist() == [nrows - 2, nrows - 1, nrows + 1] and bc[-3:].tolist() == [0, 0, 1]
+    # in each of the rows all nonzeros but the last row's last lie at column 0, where the last of them stays
+    assert bv[:8].tolist() == [0] * 8 and bv[-8:].tolist() == [3, 0, 0, 0, 0, 7, 0, 0]
+    assert npb[-2:].tolist() == [1, 1] and int(npb.sum()) == 2

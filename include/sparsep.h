@@ -582,6 +582,17 @@ int sparsep_batch_get_info(const sparsep_batch *b, uint64_t *compulsory_bytes, u
 int sparsep_batch_item_kinds(const sparsep_batch *b, uint64_t *window_items, uint64_t *chunk_items);
 
 /* ------------------------------------------------------------------------ */
+/* Scratch kept between calls                                                */
+/* ------------------------------------------------------------------------ */
+/* The device converters below take their scratch from a memory pool of the
+ * library's own, which keeps up to 512 MB per device for the next call.  Other
+ * allocators of the process do not see that memory; this call gives what the
+ * current device's pool holds unused back to the device (the library does so
+ * by itself where one of its own allocations would fail).  Waits for the
+ * device's work; not for use while a stream is being captured. */
+int sparsep_trim_scratch(void);
+
+/* ------------------------------------------------------------------------ */
 /* COO -> CSR on the device (no reference counterpart on the device; the     */
 /* arrays equal coo2csr's, spmv/1D/CSR-row/support/matrix.h:113-152)         */
 /* ------------------------------------------------------------------------ */

@@ -432,6 +432,12 @@ class Plan:
             pass
 
 
+def trim_scratch() -> None:
+    """Give the scratch memory that the device converters keep between calls back
+    to the current device (sparsep_trim_scratch)."""
+    check(lib().sparsep_trim_scratch(), "trim_scratch")
+
+
 class BcsrLayout:
     """The block structure of a device CSR (sparsep_bcsr_layout_device): sorts
     the nonzeros into rb x cb blocks once; fill() then writes the BCSR arrays

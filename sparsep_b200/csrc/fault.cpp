@@ -50,14 +50,15 @@ static cudaMemPool_t pool() {
   return g_pool[dev];
 }
 // What the current device's pool keeps and nobody uses, back to the device.
-static void trim_pool() {
+static cudaError_t trim_pool() {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (dev < 0 || dev >= 64) return cudaSuccess;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (g_pool[dev]) {
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(g_pool[dev], 0);
-  }
+  if (!g_pool[dev]) return cudaSuccess;
+  // what is given back on a stream counts once the stream has come to that
+  if (cudaError_t e = cudaDeviceSynchronize()) return e;
+  return cudaMemPoolTrimTo(g_pool[dev], 0);
 }
 
 cudaError_t dev_malloc(void **p, size_t bytes) {
@@ -104,6 +105,8 @@ int wait_fault() { return g_wait_fault.load(); }
 }  // namespace sparsep
 
 extern "C" {
+
+int sparsep_trim_scratch(void) { return sparsep::trim_pool() == cudaSuccess ? SPARSEP_OK : SPARSEP_EIO; }
 
 int sparsep_test_fail_alloc(int nth) {
   if (nth < 0) return SPARSEP_EINVAL;

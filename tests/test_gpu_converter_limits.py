@@ -1,11 +1,14 @@
-"""What the device converters refuse and how far they reach, in block rows of every
-length: a column past the last one is refused wherever it lies."""
+"""What the device converters refuse, how far they reach and what they keep: a column
+past the last one is refused wherever it lies, block rows may be of any length, the
+scratch kept between calls can be had back."""
+import ctypes as C
 import time
 
 import numpy as np
 import pytest
 
 from sparsep_b200 import capi
+from test_gpu_csr2bcsr_device import TORCH
 
 pytestmark = pytest.mark.gpu
 
@@ -100,3 +103,40 @@ def test_nonzeros_up_to_the_last_index():
     # in each of the rows all nonzeros but the last row's last lie at column 0, where the last of them stays
     assert bv[:8].tolist() == [0] * 8 and bv[-8:].tolist() == [3, 0, 0, 0, 0, 7, 0, 0]
     assert npb[-2:].tolist() == [1, 1] and int(npb.sum()) == 2
+
+
+def coo2csr(dtype, nnz, nrows, seed=0):
+    """One conversion of a random list; the list, and (rowptr, colind, values)."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rows = torch.randint(0, nrows, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    cols = torch.randint(0, 2**31 - 1, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    vals = torch.randint(-100, 100, (nnz,), generator=g, device="cuda").to(getattr(torch, TORCH[dtype]))
+    rowptr = torch.full((nrows + 1,), -1, dtype=torch.int32, device="cuda")
+    colind, out = torch.full_like(cols, -1), torch.zeros_like(vals)
+    f = getattr(capi.lib(), f"sparsep_coo2csr_device_{dtype}")
+    f.argtypes = [C.c_void_p] * 3 + [C.c_uint32, C.c_uint32] + [C.c_void_p] * 4
+    torch.cuda.synchronize()
+    capi.check(f(rows.data_ptr(), cols.data_ptr(), vals.data_ptr(), nnz, nrows, rowptr.data_ptr(), colind.data_ptr(),
+                 out.data_ptr(), None), "coo2csr_device")
+    return (rows, cols, vals), (rowptr, colind, out)
+
+
+def free_bytes():
+    import torch
+
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_trim_gives_the_kept_scratch_back():
+    coo2csr("f32", 8 << 20, 1 << 20)  # at least 12 bytes per nonzero of scratch, below the 512 MB that are kept
+    before = free_bytes()
+    capi.trim_scratch()
+    assert free_bytes() - before >= 64 << 20
+    kept = free_bytes()
+    capi.trim_scratch()  # nothing left to give
+    assert free_bytes() == kept
+    (rows, cols, vals), (_, colind, out) = coo2csr("f32", 100_000, 999)  # and the pool still serves
+    order = rows.argsort(stable=True)
+    assert bool((colind == cols[order]).all()) and bool((out == vals[order]).all())

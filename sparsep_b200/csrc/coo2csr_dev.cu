@@ -68,9 +68,10 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
   // keys in a set that is free by then, the digit counts, a flag
   const size_t n = nnz, sets = np > 2 ? 2 : 1, vb = ((n * sizeof(V)) + 15) & ~(size_t)15;
   const size_t kb = ((n * 4) + 15) & ~(size_t)15, set = 2 * kb + vb;
-  unsigned char *buf = nullptr;
-  int st = c2c_err(sparsep::ws_malloc((void **)&buf, sets * set + kb + count_words(nnz) * 4 + 64, s));
+  sparsep::Scratch mem;
+  int st = c2c_err(sparsep::ws_malloc(&mem, sets * set + kb + count_words(nnz) * 4 + 64, s));
   if (st) return st;
+  unsigned char *buf = static_cast<unsigned char *>(mem.p);
   auto key_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set); };
   auto col_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set + kb); };
   auto val_of = [&](size_t q) { return reinterpret_cast<V *>(buf + q * set + 2 * kb); };
@@ -101,7 +102,7 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
     rowptr_kernel<<<(nrows + 1 + 255) / 256, 256, 0, s>>>(key, nnz, nrows, rowptr);
     st = c2c_err(cudaGetLastError());
   }
-  sparsep::ws_free(buf, s);
+  sparsep::ws_free(&mem, s);
   if (!st) st = c2c_err(cudaStreamSynchronize(s));
   return st;
 }

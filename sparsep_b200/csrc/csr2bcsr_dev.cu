@@ -400,6 +400,8 @@ struct sparsep_bcsr_layout {
   uint32_t *sidx = nullptr;    // nonzeros in block order (input order inside a block)
   uint32_t *bstart = nullptr;  // nblocks + 1 start positions in sidx
   uint64_t *bkey = nullptr;    // block keys (block row << jbits | block column)
+  sparsep::Scratch mem[4];     // where these lie
+  int nmem = 0;
 };
 
 static int c2b_err(cudaError_t e) {
@@ -425,16 +427,31 @@ static int col_shift(uint32_t cb) {  // log2 of a power of two, else -1
   return s;
 }
 
+// Memory of the layout's own.
+template <typename T>
+static cudaError_t take(sparsep_bcsr_layout *L, T **p, size_t bytes, cudaStream_t s) {
+  const cudaError_t e = sparsep::ws_malloc(&L->mem[L->nmem], bytes, s);
+  if (e == cudaSuccess) *p = static_cast<T *>(L->mem[L->nmem++].p);
+  return e;
+}
+
+static void give_back(sparsep_bcsr_layout *L, cudaStream_t s) {
+  while (L->nmem) sparsep::ws_free(&L->mem[--L->nmem], s);
+  L->rowptr = L->browptr = L->row = L->sidx = L->bstart = nullptr;
+  L->bkey = nullptr;
+}
+
 // Block rows in shared memory; *fits false where one is too long for that.
 static int layout_rows(const uint32_t *rowptr, sparsep_bcsr_layout *L, bool *fits, cudaStream_t s) {
   using sparsep::radix::SCAN_CHUNK;
   const uint32_t m = L->nbr + 1, nb = (m + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  uint32_t *buf = nullptr;
+  sparsep::Scratch sums;
   int h_flag[2] = {0, 0};
-  int st = c2b_err(sparsep::ws_malloc((void **)&L->rowptr, ((size_t)L->nrows + 1) * 4, s));
-  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->browptr, (size_t)m * 4, s));
-  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&buf, ((size_t)nb + 4) * 4, s));
+  int st = c2b_err(take(L, &L->rowptr, ((size_t)L->nrows + 1) * 4, s));
+  if (!st) st = c2b_err(take(L, &L->browptr, (size_t)m * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc(&sums, ((size_t)nb + 4) * 4, s));
   if (!st) {
+    uint32_t *buf = static_cast<uint32_t *>(sums.p);
     int *flag = reinterpret_cast<int *>(buf + nb);
     st = c2b_err(cudaMemsetAsync(flag, 0, 2 * sizeof(int), s));
     if (!st) st = c2b_err(cudaMemsetAsync(L->browptr, 0, (size_t)m * 4, s));
@@ -459,7 +476,7 @@ static int layout_rows(const uint32_t *rowptr, sparsep_bcsr_layout *L, bool *fit
     if (!st) st = c2b_err(cudaStreamSynchronize(s));
     if (!st && h_flag[0]) st = SPARSEP_EINVAL;
   }
-  sparsep::ws_free(buf, s);
+  sparsep::ws_free(&sums, s);
   *fits = !h_flag[1];
   return st;
 }
@@ -480,9 +497,7 @@ static int layout(const uint32_t *rowptr, const uint32_t *colind, uint32_t nrows
   bool fits = true;
   if (!st) st = layout_rows(rowptr, L, &fits, s);
   if (st || fits) return st;
-  sparsep::ws_free(L->rowptr, s);
-  sparsep::ws_free(L->browptr, s);
-  L->rowptr = L->browptr = nullptr;
+  give_back(L, s);
   return layout_sorted(rowptr, colind, nrows, ncols, nnz, rb, cb, L, s);
 }
 
@@ -492,9 +507,10 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
   const uint64_t nbc = ((uint64_t)ncols + cb - 1) / cb;
   L->jbits = bits_for(nbc);
   const int bits = L->jbits + bits_for(L->nbr);
-  int *bad = nullptr;
-  int st = c2b_err(sparsep::ws_malloc((void **)&bad, 2 * sizeof(int), s));
+  sparsep::Scratch flags, work;
+  int st = c2b_err(sparsep::ws_malloc(&flags, 2 * sizeof(int), s));
   if (st) return st;
+  int *bad = static_cast<int *>(flags.p);
   uint32_t *dnb = reinterpret_cast<uint32_t *>(bad + 1);
   int h_bad = 0;
   st = c2b_err(cudaMemsetAsync(bad, 0, 2 * sizeof(int), s));
@@ -505,11 +521,10 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
   const uint32_t nbs = (nnz + sparsep::radix::SCAN_CHUNK - 1) / sparsep::radix::SCAN_CHUNK;
   const size_t rsw = (radix_scratch_words(nnz) + 1) & ~(size_t)1;
   const size_t words = 6 * (size_t)nnz + rsw + ((size_t)nnz + nbs + 8) + ((size_t)nnz + 1) + 8;
-  uint32_t *buf = nullptr;
-  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&buf, words * 4, s));
-  if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->row, (size_t)nnz * 4, s));
+  if (!st) st = c2b_err(sparsep::ws_malloc(&work, words * 4, s));
+  if (!st) st = c2b_err(take(L, &L->row, (size_t)nnz * 4, s));
   if (!st) {
-    uint64_t *key = reinterpret_cast<uint64_t *>(buf), *k0 = key + nnz, *k1 = k0 + nnz;
+    uint64_t *key = static_cast<uint64_t *>(work.p), *k0 = key + nnz, *k1 = k0 + nnz;
     uint32_t *scratch = reinterpret_cast<uint32_t *>(k1 + nnz);
     uint32_t *flag = scratch + rsw, *sums = flag + nnz, *bstart_tmp = sums + nbs + 8;
     uint64_t *bkey_tmp = key;
@@ -530,17 +545,17 @@ static int layout_sorted(const uint32_t *rowptr, const uint32_t *colind, uint32_
     if (!st) st = c2b_err(cudaMemcpyAsync(&L->nblocks, dnb, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (!st) st = c2b_err(cudaStreamSynchronize(s));
     if (!st && h_bad) st = SPARSEP_EINVAL;
-    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->sidx, (size_t)nnz * 4, s));
-    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bstart, ((size_t)L->nblocks + 1) * 4, s));
-    if (!st) st = c2b_err(sparsep::ws_malloc((void **)&L->bkey, (size_t)std::max<uint32_t>(L->nblocks, 1) * 8, s));
+    if (!st) st = c2b_err(take(L, &L->sidx, (size_t)nnz * 4, s));
+    if (!st) st = c2b_err(take(L, &L->bstart, ((size_t)L->nblocks + 1) * 4, s));
+    if (!st) st = c2b_err(take(L, &L->bkey, (size_t)std::max<uint32_t>(L->nblocks, 1) * 8, s));
     if (!st) st = c2b_err(cudaMemcpyAsync(L->sidx, sidx, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, s));
     if (!st)
       st = c2b_err(cudaMemcpyAsync(L->bstart, bstart_tmp, ((size_t)L->nblocks + 1) * 4, cudaMemcpyDeviceToDevice, s));
     if (!st) st = c2b_err(cudaMemcpyAsync(L->bkey, bkey_tmp, (size_t)L->nblocks * 8, cudaMemcpyDeviceToDevice, s));
     if (!st) st = c2b_err(cudaStreamSynchronize(s));
   }
-  sparsep::ws_free(buf, s);
-  sparsep::ws_free(bad, s);
+  sparsep::ws_free(&work, s);
+  sparsep::ws_free(&flags, s);
   return st;
 }
 
@@ -595,9 +610,7 @@ void sparsep_bcsr_layout_free(sparsep_bcsr_layout *L) {
   int dev = L->dev;
   cudaGetDevice(&dev);
   if (dev != L->dev) cudaSetDevice(L->dev);
-  for (void *d : {(void *)L->rowptr, (void *)L->browptr, (void *)L->row, (void *)L->sidx, (void *)L->bstart,
-                  (void *)L->bkey})
-    sparsep::ws_free(d, nullptr);
+  give_back(L, nullptr);
   if (dev != L->dev) cudaSetDevice(dev);
   delete L;
 }

@@ -28,6 +28,7 @@ static bool fails_now() {
 // The current device's pool, made on first use; null where the device has none.
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[64];
+static std::atomic<size_t> g_pool_used[64];  // bytes of the pool's memory in use
 static cudaMemPool_t pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -80,23 +81,43 @@ void dev_free(void *p) {
   --g_live;
 }
 
-cudaError_t ws_malloc(void **p, size_t bytes, cudaStream_t s) {
-  *p = nullptr;
+cudaError_t ws_malloc(Scratch *m, size_t bytes, cudaStream_t s) {
+  *m = Scratch();
   if (fails_now()) return cudaErrorMemoryAllocation;
   cudaMemPool_t pl = pool();
-  cudaError_t e = pl ? cudaMallocFromPoolAsync(p, bytes, pl, s) : cudaMallocAsync(p, bytes, s);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    trim_pool();
-    e = pl ? cudaMallocFromPoolAsync(p, bytes, pl, s) : cudaMallocAsync(p, bytes, s);
+  if (pl) {
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    if (g_pool_used[dev].fetch_add(bytes) + bytes <= POOL_KEEP) m->pool = dev;
+    else g_pool_used[dev].fetch_sub(bytes);
   }
-  if (e == cudaSuccess) ++g_live;
+  auto get = [&] { return m->pool >= 0 ? cudaMallocFromPoolAsync(&m->p, bytes, pl, s) : cudaMalloc(&m->p, bytes); };
+  cudaError_t e = get();
+  if (e == cudaErrorMemoryAllocation) {
+    trim_pool();
+    e = get();
+  }
+  if (e == cudaSuccess) {
+    m->bytes = bytes;
+    ++g_live;
+  } else {
+    if (m->pool >= 0) g_pool_used[m->pool].fetch_sub(bytes);
+    *m = Scratch();
+  }
+  cudaGetLastError();  // a failure is in e: no later launch is to report it
   return e;
 }
 
-void ws_free(void *p, cudaStream_t s) {
-  if (!p) return;
-  cudaFreeAsync(p, s);
+void ws_free(Scratch *m, cudaStream_t s) {
+  if (!m->p) return;
+  if (m->pool >= 0) {
+    cudaFreeAsync(m->p, s);
+    g_pool_used[m->pool].fetch_sub(m->bytes);
+  } else {
+    cudaStreamSynchronize(s);  // the work that uses it
+    cudaFree(m->p);
+  }
+  *m = Scratch();
   --g_live;
 }
 

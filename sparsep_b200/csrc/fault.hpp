@@ -16,12 +16,19 @@ void dev_free(void *p);
 // pool of the library's own per device, which keeps up to POOL_KEEP bytes between
 // calls (a quarter gigabyte from cudaMalloc and back costs a call milliseconds and
 // two device-wide synchronisations) until sparsep_trim_scratch or an allocation of the
-// library's own that finds the device full.  POOL_KEEP holds what converting some 30 M
-// nonzeros takes; scratch beyond it goes back to the device after every call, as all
-// of it did from cudaMalloc.  Counted and failed on request like dev_malloc.
+// library's own that finds the device full.  What does not fit into POOL_KEEP bytes
+// with the scratch in use comes from cudaMalloc and goes back: a pool that maps and
+// unmaps memory in every call is slower than that (COO -> CSR of 60 M nonzeros, FP32:
+// 16.4 ms from the pool, 3.6 from cudaMalloc; inside POOL_KEEP, 15 M nonzeros: 0.5
+// against 2.5 ms).  Counted and failed on request like dev_malloc.
 constexpr size_t POOL_KEEP = (size_t)512 << 20;
-cudaError_t ws_malloc(void **p, size_t bytes, cudaStream_t s);
-void ws_free(void *p, cudaStream_t s);
+struct Scratch {
+  void *p = nullptr;
+  size_t bytes = 0;
+  int pool = -1;  // the device whose pool it is from, -1: cudaMalloc
+};
+cudaError_t ws_malloc(Scratch *m, size_t bytes, cudaStream_t s);
+void ws_free(Scratch *m, cudaStream_t s);  // nothing where m holds none
 
 // Nonzero while test support asks the kernels with bounded staging waits to
 // add one wait that nothing completes (after their own copies have landed).

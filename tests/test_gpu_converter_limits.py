@@ -140,3 +140,33 @@ def test_trim_gives_the_kept_scratch_back():
     (rows, cols, vals), (_, colind, out) = coo2csr("f32", 100_000, 999)  # and the pool still serves
     order = rows.argsort(stable=True)
     assert bool((colind == cols[order]).all()) and bool((out == vals[order]).all())
+
+
+def coo2csr_us(nnz, nrows=1 << 20):
+    import torch
+
+    rows = torch.randint(0, nrows, (nnz,), device="cuda", dtype=torch.int32)
+    vals = torch.rand(nnz, device="cuda")
+    rowptr = torch.empty(nrows + 1, dtype=torch.int32, device="cuda")
+    colind, out = torch.empty_like(rows), torch.empty_like(vals)
+    f = capi.lib().sparsep_coo2csr_device_f32
+    f.argtypes = [C.c_void_p] * 3 + [C.c_uint32, C.c_uint32] + [C.c_void_p] * 4
+    times = []
+    for _ in range(5):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        capi.check(f(rows.data_ptr(), rows.data_ptr(), vals.data_ptr(), nnz, nrows, rowptr.data_ptr(),
+                     colind.data_ptr(), out.data_ptr(), None))
+        times.append((time.perf_counter() - t0) * 1e6)
+    return min(times)
+
+
+def test_scratch_beyond_what_is_kept_costs_an_allocation():
+    """Scratch of more than the 512 MB that are kept comes from cudaMalloc, at most
+    a few milliseconds, not from a pool that maps it anew in every call."""
+    us = {n: coo2csr_us(n) for n in (8 << 20, 80 << 20)}
+    print(us)
+    assert us[80 << 20] < 10 * us[8 << 20] + 8000
+    before = free_bytes()
+    capi.trim_scratch()
+    assert free_bytes() - before <= 600 << 20

@@ -8,6 +8,12 @@
 // writes the columns and values where they belong, so nothing is gathered
 // afterwards.  Then rowptr[r] = first sorted position with row >= r (a binary
 // search per row).
+//
+// Scratch: the outputs hold the columns and values of every second pass, so that one
+// more set of them and two of keys do: 12 bytes per nonzero and a value (4 bytes with
+// one pass).  Where the device has no room for that, values of 8 bytes, for which it is
+// more than the 16 bytes of a sort of indices, are sorted by their indices, which lie
+// in the outputs until a gather replaces them: 8 bytes per nonzero.
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -32,6 +38,17 @@ __global__ void rowptr_kernel(const uint32_t *__restrict__ key, uint32_t n, uint
     else hi = mid;
   }
   rowptr[r] = lo;
+}
+
+// colind holds the nonzeros' indices in order: their columns and values instead
+template <typename V>
+__global__ void gather(uint32_t n, const uint32_t *__restrict__ cols, const V *__restrict__ vals, uint32_t *colind,
+                       V *__restrict__ vals_out) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = colind[i];
+    colind[i] = cols[k];
+    vals_out[i] = vals[k];
+  }
 }
 
 }  // namespace c2c
@@ -64,38 +81,50 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
   while (bits < 32 && (nrows - 1) >> bits) ++bits;  // bits of the largest row index
   if (nrows <= 1) bits = 0;
   const int np = passes(bits);
-  // records of the passes before the last (two sets at most), the last pass's
-  // keys in a set that is free by then, the digit counts, a flag
-  const size_t n = nnz, sets = np > 2 ? 2 : 1, vb = ((n * sizeof(V)) + 15) & ~(size_t)15;
-  const size_t kb = ((n * 4) + 15) & ~(size_t)15, set = 2 * kb + vb;
+  const size_t n = nnz, vb = ((n * sizeof(V)) + 15) & ~(size_t)15, kb = ((n * 4) + 15) & ~(size_t)15;
+  const size_t keys = np > 1 ? 2 * kb : kb, set = np > 1 ? kb + vb : 0, rest = count_words(nnz) * 4 + 64;
   sparsep::Scratch mem;
-  int st = c2c_err(sparsep::ws_malloc(&mem, sets * set + kb + count_words(nnz) * 4 + 64, s));
+  bool by_index = false;
+  cudaError_t e = sparsep::ws_malloc(&mem, keys + set + rest, s);
+  if (e == cudaErrorMemoryAllocation && sizeof(V) == 8 && np > 1) {
+    by_index = true;
+    e = sparsep::ws_malloc(&mem, keys + rest, s);
+  }
+  int st = c2c_err(e);
   if (st) return st;
   unsigned char *buf = static_cast<unsigned char *>(mem.p);
-  auto key_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set); };
-  auto col_of = [&](size_t q) { return reinterpret_cast<uint32_t *>(buf + q * set + kb); };
-  auto val_of = [&](size_t q) { return reinterpret_cast<V *>(buf + q * set + 2 * kb); };
-  uint32_t *last_key = reinterpret_cast<uint32_t *>(buf + sets * set);
-  uint32_t *counts = reinterpret_cast<uint32_t *>(buf + sets * set + kb);
+  uint32_t *key_buf[2] = {reinterpret_cast<uint32_t *>(buf), reinterpret_cast<uint32_t *>(buf + keys - kb)};
+  uint32_t *col_set = reinterpret_cast<uint32_t *>(buf + keys);
+  V *val_set = reinterpret_cast<V *>(buf + keys + kb);
+  uint32_t *counts = reinterpret_cast<uint32_t *>(buf + keys + (by_index ? 0 : set));
   int *bad = reinterpret_cast<int *>(counts + count_words(nnz));
-  const uint32_t *key = rows, *col = cols;
+  const uint32_t *key = rows, *col = by_index ? nullptr : cols;
   const V *val = vals;
   if (nnz) {
     int h_bad = 0;
     st = c2c_err(cudaMemsetAsync(bad, 0, sizeof(int), s));
     for (int p = 0, shift = 0; !st && p < np; shift += pass_bits(bits, p, np), ++p) {
       const int b = pass_bits(bits, p, np);
-      const bool last = p + 1 == np;
-      uint32_t *ko = last ? last_key : key_of(p % 2), *co = last ? colind : col_of(p % 2);
-      V *vo = last ? vals_out : val_of(p % 2);
+      const bool out = (np - 1 - p) % 2 == 0;  // the last pass writes the outputs
       st = c2c_err(count_pass<uint32_t>(key, nnz, shift, b, counts, s, p ? nullptr : bad, nrows));
       if (!st && p == 0) {  // nothing of the outputs is written for a row index >= nrows
         st = c2c_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
         if (!st) st = c2c_err(cudaStreamSynchronize(s));
         if (!st && h_bad) st = SPARSEP_EINVAL;
       }
-      if (!st) st = c2c_err(scatter_pass<uint32_t, V>(key, col, val, nnz, shift, b, counts, ko, co, vo, s));
-      key = ko, col = co, val = vo;
+      uint32_t *ko = key_buf[p % 2], *co = out ? colind : by_index ? reinterpret_cast<uint32_t *>(vals_out) : col_set;
+      if (!st && by_index)
+        st = c2c_err(scatter_pass<uint32_t, NoValue>(key, col, nullptr, nnz, shift, b, counts, ko, co, nullptr, s));
+      V *vo = out ? vals_out : val_set;
+      if (!st && !by_index) {
+        st = c2c_err(scatter_pass<uint32_t, V>(key, col, val, nnz, shift, b, counts, ko, co, vo, s));
+        val = vo;
+      }
+      key = ko, col = co;
+    }
+    if (!st && by_index) {  // the indices are in colind now
+      gather<V><<<(unsigned)std::min<uint64_t>(16384, (n + 255) / 256), 256, 0, s>>>(nnz, cols, vals, colind, vals_out);
+      st = c2c_err(cudaGetLastError());
     }
   }
   if (!st) {

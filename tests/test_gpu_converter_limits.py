@@ -170,3 +170,35 @@ def test_scratch_beyond_what_is_kept_costs_an_allocation():
     before = free_bytes()
     capi.trim_scratch()
     assert free_bytes() - before <= 600 << 20
+
+
+@pytest.mark.parametrize("dtype", ["i8", "i16", "f32", "f64"])
+@pytest.mark.parametrize("nrows", [100, 9000, 1 << 20, 1 << 24])  # one to four passes
+def test_scratch_per_nonzero(dtype, nrows):
+    """At most 12 bytes and a value per nonzero, as the pool shows that held nothing before."""
+    nnz = 8 << 20
+    capi.trim_scratch()
+    (rows, cols, vals), (rowptr, colind, out) = coo2csr(dtype, nnz, nrows)
+    held = free_bytes()
+    capi.trim_scratch()
+    held = free_bytes() - held
+    assert held <= nnz * (12 + vals.element_size()) + nnz // 4 + (40 << 20)  # and digit counts, a pool's granularity
+    order = rows.argsort(stable=True)
+    assert bool((colind == cols[order]).all()) and bool((out == vals[order]).all())
+
+
+@pytest.mark.parametrize("dtype", ["i64", "f64"])
+@pytest.mark.parametrize("nrows", [100, 129, 9000, 1 << 14, 1 << 20, (1 << 21) + 1, 1 << 24])
+@pytest.mark.parametrize("nnz", [1, 4097, 300_001])
+def test_without_room_values_of_8_bytes_go_by_index(dtype, nrows, nnz):
+    L = capi.lib()
+    live = L.sparsep_test_live_allocations()
+    if nrows > 128:  # one pass asks for no more
+        L.sparsep_test_fail_alloc(1)
+    (rows, cols, vals), (rowptr, colind, out) = coo2csr(dtype, nnz, nrows, seed=nnz)
+    L.sparsep_test_fail_alloc(0)
+    assert L.sparsep_test_live_allocations() == live
+    order = rows.argsort(stable=True)
+    assert bool((colind == cols[order]).all()) and bool((out == vals[order]).all())
+    want = rows.bincount(minlength=nrows).cumsum(0)
+    assert rowptr[0] == 0 and bool((rowptr[1:] == want).all())

@@ -1219,11 +1219,17 @@ __global__ void __launch_bounds__(512, 3) bcoo_chunks(Params<T> P) {
   uint32_t *run = reinterpret_cast<uint32_t *>(sm + St::RUN);
   // block rows' first blocks, in order
   const uint32_t words = (n + 31) / 32;
+  bool gap = false;  // a block row without blocks before this thread's
   for (uint32_t b = threadIdx.x; b < words * 32; b += blockDim.x) {
-    const uint32_t m = __ballot_sync(0xffffffffu, b < n && (b == 0 || ind[b].rowind != ind[b - 1].rowind));
+    const uint32_t step = b == 0 ? 1u : b < n ? ind[b].rowind - ind[b - 1].rowind : 0u;
+    gap |= step > 1;
+    const uint32_t m = __ballot_sync(0xffffffffu, step != 0);
     if (lane == 0) ballots[b / 32] = m;
   }
-  __syncthreads();
+  // Rows without blocks between the chunk's first and last block row: the CTA zeroes
+  // all rows in between side by side, and those with blocks are written after the next
+  // barrier.  A thread per gap took 2.3 ms for 40 block rows 20,000 rows apart (FP32 4x4).
+  if (__syncthreads_or(gap)) zero_rows(row_of((uint64_t)ind[0].rowind + 1), row_of(ind[n - 1].rowind));
   const uint32_t mine = lane < words ? ballots[lane] : 0u;
   uint32_t before = __popc(mine);  // inclusive, then exclusive
 #pragma unroll
@@ -1240,14 +1246,9 @@ __global__ void __launch_bounds__(512, 3) bcoo_chunks(Params<T> P) {
   }
   if (threadIdx.x == 0) run[k] = n;
   __syncthreads();
-  // rows of no block: before the first, between two, after the last block row
-  if (!atomic) {
-    zero_rows(row_of(it.own0), row_of(ind[0].rowind));
-    for (uint32_t i = threadIdx.x + 1; i < k; i += blockDim.x)
-      for (uint64_t r = row_of((uint64_t)ind[run[i] - 1].rowind + 1); r < row_of(ind[run[i]].rowind) && r < it.row_end; ++r)
-        put<T>(P, out, r, A(0));
-    if (!gb.n) zero_rows(row_of((uint64_t)ind[n - 1].rowind + 1), row_of(it.own1));
-  }
+  // and rows of no block before the first and after the last block row
+  zero_rows(row_of(it.own0), row_of(ind[0].rowind));
+  if (!gb.n) zero_rows(row_of((uint64_t)ind[n - 1].rowind + 1), row_of(it.own1));
   const T *xt = xb + it.col_off;
   const uint32_t *scol = &ind[0].colind;
   const bool whole = x_whole<T, RB, CB, 2>(P, it, xt, scol, n);

@@ -917,20 +917,13 @@ __device__ void arrive(const Params<T> &P, T *out, uint32_t item, uint64_t row_e
     __threadfence();
     const RowGroup g = s.g;
     A sum = A(0);
-    if constexpr (W == 1) {  // 32 parts per round trip, added one after the other
-      for (uint32_t c0 = 0; c0 + 1 < g.n; c0 += 32) {
-        const uint32_t c = c0 + lane;
-        const A v = c + 1 < g.n ? bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + c))) : A(0);
-        for (uint32_t j = 0; j < 32 && c0 + j + 1 < g.n; ++j) {
-          const A t = __shfl_sync(0xffffffffu, v, j);
-          sum = c0 + j ? sum + t : t;
-        }
-      }
-    } else if (lane < W) {
-#pragma unroll 4
-      for (uint32_t c = 0; c + 1 < g.n; ++c) {
-        const A t = bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + c) + lane));
-        sum = c ? sum + t : t;
+    constexpr uint32_t N = 32 / W;  // items whose parts come in one round trip, added one after the other
+    for (uint32_t c0 = 0; c0 + 1 < g.n; c0 += N) {
+      const uint32_t c = c0 + lane / W;
+      const A v = c + 1 < g.n ? bits_acc<A>(__ldcg(P.carry_val + slot(g, g.f + c) + lane % W)) : A(0);
+      for (uint32_t j = 0; j < N && c0 + j + 1 < g.n; ++j) {
+        const A t = __shfl_sync(0xffffffffu, v, j * W + lane % W);
+        sum = c0 + j ? sum + t : t;
       }
     }
     if (lane < W) {

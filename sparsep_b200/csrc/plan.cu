@@ -1444,13 +1444,18 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
   uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb)), nparts = 0;
   const uint64_t S = bcsr_chunk_blocks(rb, cb, sizeof(T));
   uint64_t rcap = UINT64_MAX;
+  const uint64_t lpb = std::max<uint64_t>(1, (uint64_t)rb * cb * sizeof(T) / 16);  // lanes per block
+  const uint64_t workers = oo.nr_workers > 0 ? oo.nr_workers : 8;
   if (S) {
-    per = std::min<uint64_t>(S, std::max<uint64_t>(32, nblocks / (4 * (uint64_t)p->sms)));
-    // whole passes of the CTA's warps over the chunk's block rows
     const uint64_t m = std::max<uint64_t>(1, nblocks * rb / (std::max<uint64_t>(1, nrows) * V));
-    const uint64_t lpb = std::max<uint64_t>(1, (uint64_t)rb * cb * sizeof(T) / 16);
+    // A chunk, less where that leaves SMs idle, down to 32 blocks or some block rows: 1000
+    // block rows of 20 in chunks of one each are more CTAs than run at once (INT8 4x4
+    // 5.5 us).
+    const uint64_t least = std::min<uint64_t>(96, std::max<uint64_t>(32, 4 * m));
+    per = std::min<uint64_t>(S, std::max<uint64_t>(least, nblocks / (4 * (uint64_t)p->sms)));
+    // whole passes of the CTA's warps over the chunk's block rows
     const uint64_t lanes = std::min<uint64_t>(32, lpb * (oo.lanes ? (uint64_t)oo.lanes : chunk_lanes(m)));
-    const uint64_t pass = 32 / lanes * (oo.nr_workers > 0 ? oo.nr_workers : 8);
+    const uint64_t pass = 32 / lanes * workers;
     rcap = std::min<uint64_t>(BCSR_CHUNK_ROWS, per / m >= pass ? per / m / pass * pass : UINT64_MAX);
   }
   for (size_t i = 0; i < tiles.size(); ++i) {
@@ -1469,6 +1474,12 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
         it.n1 = t.nnz_base + bp[x1];
         uint64_t m = ((uint64_t)bp[x1] - bp[x0] + (x1 - x0) - 1) / (x1 - x0);
         it.lanes = oo.lanes ? (uint16_t)oo.lanes : (uint16_t)(S ? chunk_lanes(m) : pow2ceil((m + 1) / 2));
+        // In a chunk of few block rows the other lanes would idle while the steps of each
+        // go on one after the other: 1000 block rows of 20 blocks, INT8 / INT16 4x4, 5.5 /
+        // 6.2 us in chunks of one or two block rows with 2 lane groups each, 3.0 / 3.6
+        // in chunks of four with 8.
+        if (S && !oo.lanes)
+          while (it.lanes < 8 && it.lanes < m && (x1 - x0) * lpb * it.lanes * 2 <= 32 * workers) it.lanes *= 2;
         items.push_back(it);
       };
       // block rows [x0, x1) in items of at most cap blocks and rcap block rows

@@ -1,0 +1,59 @@
+"""The rules by which plans choose their items, at both sides of their lines: lanes of
+BCSR chunks with few block rows, the row kernel's two forms by row length and warps,
+COO items by warps and atomics.  Integers bit for bit, FP within gamma_n sum|a x|."""
+import numpy as np
+import pytest
+
+import sparsep_b200 as sp
+from sparsep_b200 import capi
+from helpers import random_x
+from test_gpu_elem_chunks import check
+from test_gpu_elem_gaps import run
+
+pytestmark = pytest.mark.gpu
+
+
+def matrix(dtype, lens, ncols=5003, seed=1):
+    rng = np.random.default_rng(seed)
+    r = np.repeat(np.arange(lens.size, dtype=np.uint32), lens)
+    c = rng.integers(0, ncols, r.size).astype(np.uint32)
+    c = c[np.lexsort((c, r))]
+    return lens.size, r, c, random_x(rng, r.size, dtype), random_x(rng, ncols, dtype), dtype
+
+
+def csr(want):
+    nrows, r, c, v, x, dtype = want
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=nrows))]).astype(np.uint32)
+    return sp.csr(dtype, nrows, x.size, rowptr, c, v)
+
+
+def items(A, want, **o):
+    """Items of the plan, whose results are checked twice."""
+    plan = sp.Plan(A, sp.default_opts(**o))
+    for _ in range(2):
+        check(run(plan, want[4], want[0]), *want)
+    n = int(plan.info.items)
+    plan.free()
+    return n
+
+
+@pytest.mark.parametrize("dtype", ["i8", "i16", "f32", "f64"])
+@pytest.mark.parametrize("b", [4, 8])
+@pytest.mark.parametrize("per", [1, 3, 20])
+def test_few_block_rows_take_more_lanes(dtype, b, per):
+    rng = np.random.default_rng(per)
+    for nbr in (1, 60, 700):
+        ncb = 40
+        bcol = np.concatenate([np.sort(rng.choice(ncb, per, replace=False)) for _ in range(nbr)]).astype(np.uint32)
+        bval, x = random_x(rng, nbr * per * b * b, dtype), random_x(rng, ncb * b, dtype)
+        A = capi.bcsr(dtype, nbr * b, ncb * b, b, b, np.arange(nbr + 1) * per, bcol, bval, bval.size,
+                      np.full(nbr * per, b * b, np.uint32))
+        row = np.repeat(np.arange(nbr), per)[:, None, None] * b + np.arange(b)[None, :, None] + np.zeros((1, 1, b), int)
+        col = bcol.astype(int)[:, None, None] * b + np.arange(b)[None, None, :] + np.zeros((1, b, 1), int)
+        plan = sp.Plan(A)
+        for _ in range(2):
+            check(run(plan, x, nbr * b), nbr * b, row.reshape(-1).astype(np.uint32), col.reshape(-1).astype(np.uint32),
+                  bval, x, dtype)
+        if per == 20 and b * b * bval.itemsize <= 128:  # 4 block rows per chunk: room for 8 lane groups each
+            assert plan.info.lanes == 8 and plan.info.items >= nbr / 4
+        plan.free()

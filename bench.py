@@ -286,7 +286,7 @@ def run_ours(args, rank, world):
         "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded Zipf power-law matrix, numpy PCG64 seed 1)",
         "config": {"workload": WORKLOAD, "nrows": n, "ncols": m, "nnz": nnz, "format": "csr",
                    "scheme": "1d", "balance": "nnz (auto items)", "variant": info.variant.decode(),
-                   "items": int(info.items), "l2": "flushed (256 MB write) before every timed step",
+                   "items": int(info.cta_items), "l2": "flushed (256 MB write) before every timed step",
                    "compulsory_bytes_per_step": cb, "parallelism": f"replicas x{world}"},
         "roofline": {"bound": "hbm", "achieved": round(gbs_rank, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(gbs_rank / peak, 4), "traffic": traffic, "peak_source": peak_kind,

@@ -345,8 +345,9 @@ typedef struct sparsep_plan_info {
   uint32_t nrows, ncols;
   uint64_t nnz;           /* stored nonzeros (blocks: stored entries)          */
   uint64_t nblocks;       /* BCSR/BCOO                                          */
-  uint64_t items;         /* CTA work items per execution                      */
-  uint64_t tiles;         /* tiles (parts) per execution                       */
+  uint64_t items;         /* work items: with nr_parts > 0 the parts that have
+                             rows (of every tile), else the CTA items          */
+  uint64_t tiles;         /* tiles of a 2D plan, 1 for a 1D plan               */
   uint64_t compulsory_bytes; /* bytes one SpMV must move (values, indices, x, y) */
   uint64_t device_bytes;  /* device memory held by the plan                    */
   uint64_t scratch_bytes; /* of which scratch (partials, carries, counters)   */
@@ -355,6 +356,8 @@ typedef struct sparsep_plan_info {
   char variant[96];       /* human-readable variant name                      */
   int32_t y_bands;        /* host-buffer path: row bands of y copied back while
                              the kernel runs (0: one copy after the kernel)     */
+  uint32_t cta_items;     /* CTA items per execution: `items`, or more where
+                             parts are cut (nr_parts)                           */
 } sparsep_plan_info;
 
 int sparsep_plan_get_info(const sparsep_plan *plan, sparsep_plan_info *info);

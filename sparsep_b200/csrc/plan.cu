@@ -526,7 +526,8 @@ static int finish_plan(sparsep_plan *p, std::vector<Item> &items, const sparsep_
   p->info.ncols = p->ncols;
   p->info.nnz = p->nnz;
   p->info.nblocks = p->nblocks;
-  p->info.items = p->nitems;
+  p->info.items = p->info.cta_items = p->nitems;
+  if (p->info.tiles == 0) p->info.tiles = 1;
   p->info.device_bytes += p->info.scratch_bytes;
   p->info.kernel_launches = p->split.on ? 2 : 1 + (p->out_mode == OUT_PARTIAL ? 1 : 0);
   p->info.workers = workers;
@@ -887,6 +888,8 @@ static int plan_multi_rhs(sparsep_plan *p, const typename Types<T>::csr *A, uint
   p->info.ncols = p->ncols;
   p->info.nnz = p->nnz;
   p->info.items = items;
+  p->info.cta_items = (uint32_t)items;
+  p->info.tiles = 1;
   p->info.compulsory_bytes = cb;
   p->info.kernel_launches = 1;
   sparsep_batch_variant v{};
@@ -1030,6 +1033,7 @@ static int plan_csr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t n
   // per tile 598 / 479 / 1564 us (FP32).
   bool staged = false;
   uint32_t nparts = 0;  // tiles that have rows
+  p->info.tiles = tiles_in.size();
   for (const Tile &t : tiles_in) staged |= stage_width(p, oo, t.xw) != 0;
   p->slim = oo.lanes == 0 && !staged && (faithful || oo.item_nnz <= 0);
   for (size_t i = 0; i < tiles_in.size(); ++i) {
@@ -1185,6 +1189,7 @@ static int plan_elems(int fmt, int scheme, uint32_t nrows, uint32_t ncols, uint6
   const uint64_t aim = fmt == SPARSEP_FMT_COO ? per_item : 0;
   p->by_groups = fmt == SPARSEP_FMT_COO || cap != 0;
   uint64_t nparts = 0;
+  p->info.tiles = tiles.size();
   set_out_mode(p, oo, V, true, fmt == SPARSEP_FMT_BCOO ? rb : 1);
   for (const ElemTile &et : tiles) {
     Tile t = et.t;
@@ -1444,6 +1449,7 @@ static int plan_bcsr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t 
   uint64_t per = std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb)), nparts = 0;
   const uint64_t S = bcsr_chunk_blocks(rb, cb, sizeof(T));
   uint64_t rcap = UINT64_MAX;
+  p->info.tiles = tiles.size();
   const uint64_t lpb = std::max<uint64_t>(1, (uint64_t)rb * cb * sizeof(T) / 16);  // lanes per block
   const uint64_t workers = oo.nr_workers > 0 ? oo.nr_workers : 8;
   if (S) {

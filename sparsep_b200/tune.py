@@ -129,7 +129,7 @@ def autotune(A: capi.HostMatrix, x: np.ndarray, reps: int = 5, grids=GRIDS, bloc
             us = float(np.median(ts))
             cb = int(p.info.compulsory_bytes)
             rec.update(status=0, us=round(us, 2), gbs=round(cb / (us * 1e-6) / 1e9, 1), compulsory_bytes=cb,
-                       variant=p.info.variant.decode(), items=int(p.info.items))
+                       variant=p.info.variant.decode(), items=int(p.info.cta_items))
             p.free()
             records.append(rec)
             if log:

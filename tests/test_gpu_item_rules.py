@@ -57,3 +57,28 @@ def test_few_block_rows_take_more_lanes(dtype, b, per):
         if per == 20 and b * b * bval.itemsize <= 128:  # 4 block rows per chunk: room for 8 lane groups each
             assert plan.info.lanes == 8 and plan.info.items >= nbr / 4
         plan.free()
+
+
+@pytest.mark.parametrize("dtype", ["i16", "f32"])
+@pytest.mark.parametrize("b", [2, 4, 8])
+def test_parts_smaller_than_a_chunk_share_it(dtype, b):
+    rng = np.random.default_rng(b)
+    nbr, ncb = 3000, 40
+    per = rng.integers(0, 9, nbr)
+    per[1000:1400] = 0
+    per[5], per[2000] = 40, 39
+    bcol = np.concatenate([np.sort(rng.choice(ncb, p, replace=False)) for p in per]).astype(np.uint32)
+    bval, x = random_x(rng, bcol.size * b * b, dtype), random_x(rng, ncb * b, dtype)
+    A = capi.bcsr(dtype, nbr * b, ncb * b, b, b, np.concatenate([[0], np.cumsum(per)]), bcol, bval, bval.size,
+                  np.full(bcol.size, b * b, np.uint32))
+    row = np.repeat(np.arange(nbr), per)[:, None, None] * b + np.arange(b)[None, :, None] + np.zeros((1, 1, b), int)
+    col = bcol.astype(int)[:, None, None] * b + np.arange(b)[None, None, :] + np.zeros((1, b, 1), int)
+    for parts in (1, 7, 300, 2048, 5000):
+        for bal in (capi.BAL_ROW, capi.BAL_BLOCK):
+            plan = sp.Plan(A, sp.default_opts(nr_parts=parts, part_balance=bal))
+            for _ in range(2):
+                check(run(plan, x, nbr * b), nbr * b, row.reshape(-1).astype(np.uint32),
+                      col.reshape(-1).astype(np.uint32), bval, x, dtype)
+            if parts >= 2048:  # one or two block rows each
+                assert plan.info.items > 1400 and 100 < plan.info.cta_items < 700
+            plan.free()

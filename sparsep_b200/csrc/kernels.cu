@@ -74,8 +74,12 @@ cudaError_t launch_items(const Params<T> &P, int fmt, uint32_t carry_w, int thre
   const uint32_t rb = P.rb, cb = P.cb;
   switch (fmt) {
     case SPARSEP_FMT_CSR:
-      return slim ? launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), true)>(P, carry_w, threads, smem, st)
-                  : launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), false)>(P, carry_w, threads, smem, st);
+      if (slim) return launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), true)>(P, carry_w, threads, smem, st);
+      // 16 warps take 2048 nonzeros per pass: 8-byte types in 32 KB then (FP64, 16 warps,
+      // 400,000 rows of 12, power-law: 52 us in 16 KB, 42)
+      return threads > 256
+                 ? launch_t<T, SPARSEP_FMT_CSR, 0, 0, 4096>(P, carry_w, threads, smem, st)
+                 : launch_t<T, SPARSEP_FMT_CSR, 0, 0, csr_chunk_nnz(sizeof(T), false)>(P, carry_w, threads, smem, st);
     case SPARSEP_FMT_COO:
       return P.out_mode == OUT_ATOMIC ? launch_coo<T, true>(P, threads, smem, st)
                                       : launch_coo<T, false>(P, threads, smem, st);

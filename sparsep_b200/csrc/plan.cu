@@ -378,6 +378,25 @@ static uint64_t csr_item_nnz(size_t es, uint64_t nnz, int sms) {
   return std::min<uint64_t>(csr_chunk_nnz(es, true), std::max<uint64_t>(256, (nnz / (4 * (uint64_t)sms) + 3) & ~3ull));
 }
 
+// Whether the row kernel's wide form (kernels.hpp) is the better one for automatic CSR
+// items.  With more than 8 warps asked for, a slim chunk is less than a pass of
+// theirs: 16 warps, FP32 / FP64, 400,000 banded rows of 12 nonzeros slim
+// 19.5 / 46 us, wide 14.5 / 24.  And where
+// most nonzeros lie in rows of which a slim chunk holds one or none: one warp sums
+// that row and the others wait, or the row goes in pieces of 2048.  Rows around 2500,
+// INT8 / FP32, 20 M nonzeros, slim 97 / 102 us, wide 63 / 94; around 1500 58 / 74 and 50 / 76;
+// around 1000 68 / 94 and 74 / 100.  8-byte types are bound by their gathers, for which the
+// slim form leaves more room at every length (FP64, around 2500: 101 and 106 us).
+static bool wide_items(size_t es, const uint32_t *rp, uint32_t nrows, const sparsep_opts &o) {
+  if (o.nr_workers > 8) return true;
+  if (es == 8) return false;
+  const uint32_t limit = es == 4 && o.nr_workers <= 4 ? 2048 : 1024;
+  uint64_t inside = 0;  // nonzeros of the longer rows
+  for (uint32_t r = 0; r < nrows; ++r)
+    if (rp[r + 1] - rp[r] > limit) inside += rp[r + 1] - rp[r];
+  return 2 * inside > rp[nrows];
+}
+
 // Blocks per BCOO item: a chunk, less where that leaves SMs idle.
 static uint64_t bcoo_item_blocks(uint32_t rb, uint32_t cb, size_t es, uint64_t nblocks) {
   const uint64_t S = bcoo_chunk_blocks(rb, cb, es);
@@ -984,7 +1003,8 @@ static int plan_csr(const typename Types<T>::csr *A, const sparsep_opts *o, spar
       }
     }
     // the slim form of the row kernel for automatic items
-    p->slim = oo.lanes == 0 && oo.pipeline != 1 && oo.item_nnz <= 0;
+    p->slim = oo.lanes == 0 && oo.pipeline != 1 && oo.item_nnz <= 0 &&
+              !wide_items(sizeof(T), A->rowptr, A->nrows, oo);
     csr_tile_items(items, t, A->rowptr, 0, A->nrows, oo, false, true, p->slim ? csr_item_nnz(sizeof(T), A->nnz, p->sms) : 0,
                    csr_chunk_nnz(sizeof(T), true) / 4);
     number_long_rows(items);
@@ -1035,7 +1055,7 @@ static int plan_csr_tiles(int scheme, uint32_t nrows, uint32_t ncols, uint64_t n
   uint32_t nparts = 0;  // tiles that have rows
   p->info.tiles = tiles_in.size();
   for (const Tile &t : tiles_in) staged |= stage_width(p, oo, t.xw) != 0;
-  p->slim = oo.lanes == 0 && !staged && (faithful || oo.item_nnz <= 0);
+  p->slim = oo.lanes == 0 && !staged && (faithful || (oo.item_nnz <= 0 && oo.nr_workers <= 8));
   for (size_t i = 0; i < tiles_in.size(); ++i) {
     Tile t = tiles_in[i];
     t.xw = stage_width(p, oo, t.xw);

@@ -82,3 +82,18 @@ def test_parts_smaller_than_a_chunk_share_it(dtype, b):
             if parts >= 2048:  # one or two block rows each
                 assert plan.info.items > 1400 and 100 < plan.info.cta_items < 700
             plan.free()
+
+
+@pytest.mark.parametrize("dtype", ["i8", "i16", "i32", "f32", "i64", "f64"])
+@pytest.mark.parametrize("length", [700, 1500, 3000])
+def test_long_rows_run_in_the_wide_form(dtype, length):
+    lens = np.full(800, length)
+    lens[::7] = 3
+    want = matrix(dtype, lens)
+    n = items(csr(want), want)
+    limit = {1: 1024, 2: 1024, 4: 2048, 8: 10**9}[np.dtype(capi.DTYPES[dtype].np).itemsize]
+    nnz = lens.sum()
+    if length > limit:  # whole rows, up to 4080 nonzeros per item
+        assert n <= np.ceil(800 / (4080 // length)) + 2
+    else:
+        assert n > nnz / 2048

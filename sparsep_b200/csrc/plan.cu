@@ -397,6 +397,20 @@ static bool wide_items(size_t es, const uint32_t *rp, uint32_t nrows, const spar
   return 2 * inside > rp[nrows];
 }
 
+// Nonzeros per automatic COO item of a plan: more warps asked for than the automatic
+// 4 get items as much larger, so that a warp's share stays what it was (16 warps, FP32,
+// 20,000 rows of 20 / 400,000 of 12 nonzeros: 17.8 / 47 us in the
+// automatic items, 10.4 / 30 like this).  Atomics on 1- and 2-byte types are
+// compare-and-swap loops on words that neighbouring rows share; with rows longer than
+// an item all items meet on a few words, so that fewer items are better (INT8, 200
+// rows of 5000: 21 us in 846 items, 17 in 245).
+static uint32_t coo_item(const sparsep_opts &o, uint64_t nnz, uint64_t nrows, size_t es) {
+  uint32_t item = coo_item_elems(nnz);
+  if (o.sync != SPARSEP_SYNC_LF && es < 4 && nnz > nrows * (uint64_t)item) item = 4096;
+  if (o.nr_workers > 4) item = (item * (uint32_t)std::min(o.nr_workers, 16) / 4 + 3) & ~3u;
+  return item;
+}
+
 // Blocks per BCOO item: a chunk, less where that leaves SMs idle.
 static uint64_t bcoo_item_blocks(uint32_t rb, uint32_t cb, size_t es, uint64_t nblocks) {
   const uint64_t S = bcoo_chunk_blocks(rb, cb, es);
@@ -1304,7 +1318,7 @@ static int plan_cooe(const typename Types<T>::cooe *A, const sparsep_opts *o, sp
   }
   std::vector<ElemTile> tiles{et};
   return plan_elems<T>(SPARSEP_FMT_COO, SPARSEP_1D, A->nrows, A->ncols, A->nnz, A->nnz, 1, A->nnzs, sizeof(E), tiles,
-                       [el](uint64_t u) { return el[u].rowind; }, coo_item_elems(A->nnz), o, out);
+                       [el](uint64_t u) { return el[u].rowind; }, coo_item(oo, A->nnz, A->nrows, sizeof(T)), o, out);
 }
 
 // SoA COO (the CSR-family reader's output, in file order): sorted into the
@@ -1375,7 +1389,7 @@ static int plan_dcoo(const typename Types<T>::dcoo *A, const sparsep_opts *o, sp
     for (uint64_t n = et.e0; n < et.e1; ++n) roff[n] = et.t.row_off;
   auto key = [el, r = std::move(roff)](uint64_t u) { return el[u].rowind + r[u]; };
   return plan_elems<T>(SPARSEP_FMT_COO, SPARSEP_2D_EQUAL, A->nrows, A->ncols, A->nnz, A->nnz, V, A->nnzs, sizeof(E),
-                       tiles, key, coo_item_elems(A->nnz), &oo, out);
+                       tiles, key, coo_item(oo, A->nnz, A->nrows, sizeof(T)), &oo, out);
 }
 
 template <typename T, typename S>
@@ -1414,11 +1428,12 @@ static int plan_stripes_coo(int scheme, const S *A, const uint32_t *widths, cons
   if (base != A->nnz) return SPARSEP_EINVAL;
   if (oo.nr_parts <= 0) oo.nr_parts = 0;
   const E *el = A->nnzs;
+  const uint32_t item = coo_item(oo, A->nnz, A->nrows, sizeof(T));
   sparsep_opts o2 = oo;
   if (o2.nr_parts == 0) {
     // GPU sizing, but never coarser than the reference's H parts per stripe
     for (auto &et : tiles) {
-      auto extra = even_cuts(et.e0, et.e1, coo_item_elems(A->nnz));
+      auto extra = even_cuts(et.e0, et.e1, item);
       et.cuts.insert(et.cuts.end(), extra.begin(), extra.end());
       std::sort(et.cuts.begin(), et.cuts.end());
       et.cuts.erase(std::unique(et.cuts.begin(), et.cuts.end()), et.cuts.end());
@@ -1426,7 +1441,7 @@ static int plan_stripes_coo(int scheme, const S *A, const uint32_t *widths, cons
     o2.nr_parts = 1;  // cuts are final
   }
   return plan_elems<T>(SPARSEP_FMT_COO, scheme, A->nrows, A->ncols, A->nnz, A->nnz, V, A->nnzs, sizeof(E), tiles,
-                       [el](uint64_t u) { return el[u].rowind; }, coo_item_elems(A->nnz), &o2, out);
+                       [el](uint64_t u) { return el[u].rowind; }, item, &o2, out);
 }
 
 template <typename T>

@@ -97,3 +97,28 @@ def test_long_rows_run_in_the_wide_form(dtype, length):
         assert n <= np.ceil(800 / (4080 // length)) + 2
     else:
         assert n > nnz / 2048
+
+
+@pytest.mark.parametrize("dtype", ["i8", "i32", "f32", "f64"])
+@pytest.mark.parametrize("workers", [0, 8, 9, 16])
+def test_many_warps_take_larger_items(dtype, workers):
+    lens = np.full(20_000, 20)
+    lens[5] = 30_011  # in chunks
+    want = matrix(dtype, lens)
+    n, nnz = items(csr(want), want, nr_workers=workers), int(lens.sum())
+    assert n < nnz / 3600 if workers > 8 else n > nnz / 1500
+    nrows, r, c, v, x, _ = want
+    E = sp.cooe(dtype, nrows, x.size, r, c, v)
+    n = items(E, want, nr_workers=workers)
+    assert abs(n - nnz / (512 * max(1, workers / 4))) < 3  # 512 nonzeros for 4 warps
+    for conv in ("cooe2dcsr", "cooe2bdcsr", "cooe2bdcoo"):
+        items(sp.convert(conv, E, 3, 2), want, nr_workers=workers, stage_x=0)
+
+
+@pytest.mark.parametrize("dtype", ["i8", "i16", "i32"])
+def test_atomics_on_small_types_take_larger_items(dtype):
+    want = matrix(dtype, np.full(200, 5000))
+    nrows, r, c, v, x, _ = want
+    E = sp.cooe(dtype, nrows, x.size, r, c, v)
+    n = items(E, want, sync=capi.SYNC_ATOMIC)
+    assert n == 245 if dtype != "i32" else n > 800

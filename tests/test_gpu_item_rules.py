@@ -122,3 +122,21 @@ def test_atomics_on_small_types_take_larger_items(dtype):
     E = sp.cooe(dtype, nrows, x.size, r, c, v)
     n = items(E, want, sync=capi.SYNC_ATOMIC)
     assert n == 245 if dtype != "i32" else n > 800
+
+
+@pytest.mark.parametrize("b", [2, 4, 8])
+def test_bcoo_lanes_by_the_items_own_block_rows(b):
+    """A stripe's blocks lie in a few of its block rows: more lanes than the mean over all of them asks for."""
+    rng = np.random.default_rng(b)
+    n, per = 4000, 24
+    r = np.repeat(np.arange(n), per)
+    c = np.clip(r + rng.integers(-200, 200, r.size), 0, n - 1)
+    first = np.unique(r * n + c)  # each position once
+    r, c = (first // n).astype(np.uint32), (first % n).astype(np.uint32)
+    v, x = random_x(rng, r.size, "f32"), random_x(rng, n, "f32")
+    D = sp.convert("rbdcsr2rbdbcoo", sp.convert("cooe2rbdcsr", sp.cooe("f32", n, n, r, c, v), 4, 16), b, b)
+    for o in (dict(), dict(sync=capi.SYNC_ATOMIC), dict(lanes=8)):
+        plan = sp.Plan(D, sp.default_opts(**o))
+        for _ in range(2):
+            check(run(plan, x, n), n, r, c, v, x, "f32")
+        plan.free()

@@ -28,6 +28,9 @@ flushed), GB/s of compulsory bytes, fraction of the measured HBM copy
 bandwidth, the reference's host SpMV for that kind on one core, and the check
 against its result (integers bit-exact, FP within 2 gamma_n sum|a x|).
 
+The configurations and the batched runs are printed on lines of their own; the last
+line is the result's one JSON line, with `configs_checked` and the batched times.
+
 The headline run is gated: its y must match the reference's host SpMV within
 that bound, or the run fails.
 
@@ -808,6 +811,25 @@ def run_reference(args, rank, world):
             "e2e": {"value": v, "unit": "GB/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
 
 
+# what the last line keeps of a batched run
+BATCH_KEYS = ("dtype", "nnz", "plain_per_matrix_ms", "queue_default_ms", "queue_learned_ms", "queue_autotuned_ms",
+              "learned_speedup_vs_plain", "learned_over_autotuned")
+
+
+def output_lines(res):
+    """The lines of a result: a line per configuration and per batched run, then the
+    one JSON line, which is the last and short enough (under 4000 characters) to be
+    read from the end of a log."""
+    res = dict(res)
+    lines = ["config " + json.dumps(e) for e in res.pop("configs", [])]
+    for k in ("batched", "batched_i32"):
+        if k in res:
+            full = res[k]
+            lines.append(f"{k} " + json.dumps(full))
+            res[k] = {q: full[q] for q in BATCH_KEYS if q in full} | {"check_ok": full.get("check", {}).get("ok")}
+    return lines + [json.dumps(res)]
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -870,7 +892,7 @@ def main():
 
         dist.destroy_process_group()
     if rank == 0 and res is not None:
-        print(json.dumps(res), flush=True)
+        print("\n".join(output_lines(res)), flush=True)
 
 
 if __name__ == "__main__":

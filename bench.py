@@ -606,7 +606,7 @@ def measure_struct(cfg, workload, A, A_abs, x, counts, cases, peak, stream, flus
     return out
 
 
-PARTS = 2048  # parts of the reference's 2048-DPU runs: one part = one CTA
+PARTS = 2048  # parts of the reference's 2048-DPU runs
 
 
 def run_configs(args, peak):

@@ -105,15 +105,21 @@ typedef struct sparsep_opts {
   int32_t part_balance;    /* sparsep_balance across parts (reference: DPUs)     */
   int32_t worker_balance;  /* sparsep_balance across workers (reference: tasklets)*/
   int32_t sync;            /* sparsep_sync                                       */
-  int32_t nr_parts;        /* reference NR_DPUS: parts, run by one or more CTAs  */
-                           /* each (lanes > 0: by one); 0 = auto                 */
-  int32_t nr_workers;      /* reference NR_TASKLETS: warps per part; 0 = auto    */
+  int32_t nr_parts;        /* reference NR_DPUS: parts, cut into items of the     */
+                           /* automatic size where larger (small BCSR parts share */
+                           /* one); a CTA each for CSR with lanes > 0 and for     */
+                           /* block sizes other than 2x2, 4x4, 8x8; 0 = auto      */
+  int32_t nr_workers;      /* reference NR_TASKLETS: warps per CTA; 0 = auto     */
   int32_t vert_partitions; /* reference -v (2D schemes built from COO)           */
   int32_t row_block_size;  /* reference -r (BCSR/BCOO built from CSR)            */
   int32_t col_block_size;  /* reference -c                                       */
   int32_t lanes;           /* lanes per row / block row: 1,2,4,8,16,32; 0 = auto */
   int32_t nrhs;            /* right-hand sides (x is ncols x nrhs row-major)     */
-  int32_t stage_x;         /* 2D: stage the x-segment in shared memory (1/0/-1=auto) */
+  int32_t stage_x;         /* 2D: stage the x-segment in shared memory (1/0/-1=auto):
+                              1 where it fits (200 KB; 176 KB beside the chunks of
+                              2x2, 4x4 and 8x8 blocks; info.stage_x tells), -1 up
+                              to 96 KB and not for those blocks, whose chunks are
+                              faster without */
   int32_t item_nnz;        /* auto plans: target nonzeros per CTA work item (0 = auto) */
   int32_t pipeline;        /* 1D CSR auto plans: 1 = persistent TMA-pipelined kernel */
   int32_t autotune;        /* 0 = the options as given; 1 = learned choice of the
@@ -635,13 +641,15 @@ SPARSEP_DECLARE_PLAN_DEVICE(double, f64)
 /* countNNZperBlockBCSRMatrix)                                              */
 /* ------------------------------------------------------------------------ */
 /* Two steps.  sparsep_bcsr_layout_device finds the rb x cb blocks of a device
- * CSR (rowptr nrows + 1, colind nnz) and returns the block count; EINVAL for a malformed rowptr or a column >= ncols.  The fill then
- * writes caller-allocated device arrays: browptr[ceil(nrows/rb) + 1],
- * bcolind[nblocks], bval[nblocks * rb * cb] (row-major blocks, blocks of a
- * block row by ascending block column, a later duplicate entry overwrites an
- * earlier one) and nnz_per_block[nblocks] (entries != 0).  One layout serves
- * any number of fills (e.g. several value arrays of one pattern) while the
- * CSR's colind stays unchanged; both steps synchronise the stream. */
+ * CSR (rowptr nrows + 1, colind nnz) and returns the block count; EINVAL for a
+ * malformed rowptr or a column >= ncols.  The fill then writes caller-allocated
+ * device arrays: browptr[ceil(nrows/rb) + 1], bcolind[nblocks],
+ * bval[nblocks * rb * cb] (row-major blocks, blocks of a block row by ascending
+ * block column, a later duplicate entry overwrites an earlier one) and
+ * nnz_per_block[nblocks] (entries != 0).  One layout serves any number of fills
+ * (e.g. several value arrays of one pattern) while the CSR's colind stays
+ * unchanged; both steps synchronise the stream.  Matrices with a block row of
+ * more than 256 nonzeros are sorted as a whole: 44 bytes of scratch per nonzero. */
 typedef struct sparsep_bcsr_layout sparsep_bcsr_layout;
 int sparsep_bcsr_layout_device(const uint32_t *d_rowptr, const uint32_t *d_colind, uint32_t nrows, uint32_t ncols,
                                uint32_t nnz, uint32_t rb, uint32_t cb, sparsep_bcsr_layout **out, uint64_t *nblocks,

@@ -18,7 +18,7 @@
 // them itself, all in the same order, while its first vectors are on their way.
 // 592 CTAs of 256 threads with two 16-byte loads per vector and thread: as fast with
 // one (43.1 to 44.2 us per iteration, FP64, 1024 x 1024 Laplacian), slower with four
-// (49.4, registers spill), with 512 threads (44.7 to 53.2) or 1024 (49.2).  Five
+// (49.4), with 512 threads (44.7 to 53.2) or 1024 (49.2).  Five
 // kernels with scalar loads and one-CTA sums between them: 48.4 us.  Of the 43.6, the
 // SpMV takes 27.
 #include <algorithm>

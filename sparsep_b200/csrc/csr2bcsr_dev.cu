@@ -28,7 +28,9 @@
 // FP32, 10.5 M nonzeros in 1 M blocks of 4x4 (COO -> CSR -> BCSR as one ingest): 8.1
 // ms with the sort for every matrix and scratch from cudaMalloc, of which 1.9 ms in
 // kernels; 0.67 ms now, of which layout 0.12 and fill 0.16 ms (fill_rows 134 us, bound
-// by its instructions: 850 for a block row of 80 nonzeros).
+// by its instructions: 850 for a block row of 80 nonzeros).  With longer block rows, by
+// the sort: 98 M nonzeros (2 M rows, banded, block rows around 190 and up to more than
+// 256) 13.7 ms, 20.6 with the earlier sort.
 #include <algorithm>
 #include <cstdio>
 #include <new>
@@ -56,8 +58,8 @@ __global__ void check_rowptr(const uint32_t *__restrict__ rowptr, uint32_t nrows
 // Nonzeros of a block row that go through a table.  Layout and fill of 4 M nonzeros,
 // 4x4, block rows of 250: 665 us with scattered columns (250 blocks each), 172 with
 // 32 blocks each; by the sort, block rows of 260: 840 and 550 us.  A table for up to
-// 2048, a warp per block row with its block columns ranked pair by pair, was slower
-// than the sort from the start: 3.5 ms at 260 scattered nonzeros, 70 at 2000.
+// 2048, a warp per block row with its block columns ranked pair by pair, was slower than
+// the sort at once: 3.5 ms at 260 scattered nonzeros, 70 at 2000.
 constexpr int LIM = 256;
 constexpr uint32_t EMPTY = 0xFFFFFFFFu;  // no block column: columns are below 2^32 - 1
 constexpr int SLOTS = 2 * LIM;

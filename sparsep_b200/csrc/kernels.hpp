@@ -35,13 +35,14 @@ constexpr uint32_t BCSR_CHUNK_ROWS = 512;
 // A gather of x holds a line of L1 while it is under way, and shared memory is
 // taken from L1: with 32 KB of FP64 products per CTA the gathers stood in line
 // (1M-row power-law matrix, FP64 188 us; 16 KB 107 us; 8 KB and 4 warps per CTA 93
-// us; FP32 with 16 KB 87 us, 8 KB and 4 warps 83.5 us).  Automatic items are slim;
-// parts and tiles, whose items are the caller's, keep the wide form (2048 parts of
-// the FP32 matrix: 8192 nonzeros each).
+// us; FP32 with 16 KB 87 us, 8 KB and 4 warps 83.5 us).  Automatic items, parts and
+// tiles are slim; wide are those of a given size (item_nnz), of tiles whose x is staged,
+// and where the planner finds that better (wide_items in plan.cu: more than 8 warps, most
+// nonzeros in long rows).
 constexpr int csr_chunk_nnz(size_t es, bool slim) { return (slim ? 8192 : 16384) / (es == 8 ? 8 : 4); }
 
 // Nonzeros per automatic COO item: 4096, fewer where that leaves less than six
-// items per SM (1.5 M nonzeros, FP32: 20 us in 366 items, 16.5 us in 733; 16.7 M:
+// items per SM of a B200's 148 (1.5 M nonzeros, FP32: 20 us in 366 items, 16.5 us in 733; 16.7 M:
 // 94 us in items of 2048, 91 us of 4096).
 constexpr uint32_t coo_item_elems(uint64_t nnz) {
   return nnz >= 4096 * 888ull ? 4096 : nnz <= 512 * 888ull ? 512 : (uint32_t)((nnz / 888 + 3) & ~3ull);

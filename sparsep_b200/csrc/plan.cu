@@ -5,10 +5,11 @@
 // partitions rows / nnz / blocks over NR_DPUS DPUs and NR_TASKLETS tasklets
 // (support/partition.h) and scatters the pieces with dpu_push_xfer
 // (spmv/1D/CSR-row/host/app.c:221-252).  Here the same partitions become CTA
-// work items over one device copy of the matrix; nr_parts > 0 reproduces the
-// reference split exactly (one part = one CTA, one tasklet = one warp; a BCSR
-// part of 2x2, 4x4 or 8x8 blocks is cut further into chunks of one CTA each) and
-// nr_parts = 0 lets the planner size items for the GPU.
+// work items over one device copy of the matrix; nr_parts > 0 takes the reference's
+// split, whose parts are cut into items of the automatic size (small BCSR parts
+// share one); a part is one CTA's, and a warp a tasklet's, with fixed lanes per row (CSR)
+// and in the block sizes without chunks.  nr_parts = 0 lets the planner size items
+// for the GPU alone.
 #include <algorithm>
 #include <climits>
 #include <chrono>
@@ -380,13 +381,13 @@ static uint64_t csr_item_nnz(size_t es, uint64_t nnz, int sms) {
 
 // Whether the row kernel's wide form (kernels.hpp) is the better one for automatic CSR
 // items.  With more than 8 warps asked for, a slim chunk is less than a pass of
-// theirs: 16 warps, FP32 / FP64, 400,000 banded rows of 12 nonzeros slim
-// 19.5 / 46 us, wide 14.5 / 24.  And where
-// most nonzeros lie in rows of which a slim chunk holds one or none: one warp sums
-// that row and the others wait, or the row goes in pieces of 2048.  Rows around 2500,
-// INT8 / FP32, 20 M nonzeros, slim 97 / 102 us, wide 63 / 94; around 1500 58 / 74 and 50 / 76;
-// around 1000 68 / 94 and 74 / 100.  8-byte types are bound by their gathers, for which the
-// slim form leaves more room at every length (FP64, around 2500: 101 and 106 us).
+// theirs: 16 warps, FP32 / FP64, 400,000 banded rows of 12 nonzeros, slim 19.5 / 46 us,
+// wide 14.5 / 24.  And where most nonzeros lie in rows of which a slim chunk holds one
+// or none: one warp sums that row and the others wait, or the row goes in pieces of
+// 2048.  INT8 / FP32, slim and wide: 8000 rows around 2500 nonzeros 97 / 102 and 63 / 94 us,
+// 10,000 around 1500 58 / 74 and 50 / 76, 20,000 around 1000 68 / 94 and 74 / 100.  8-byte
+// types are bound by their gathers, for which the slim form leaves more room at every
+// length (FP64, around 2500: 101 and 106 us).
 static bool wide_items(size_t es, const uint32_t *rp, uint32_t nrows, const sparsep_opts &o) {
   if (o.nr_workers > 8) return true;
   if (es == 8) return false;
@@ -399,11 +400,11 @@ static bool wide_items(size_t es, const uint32_t *rp, uint32_t nrows, const spar
 
 // Nonzeros per automatic COO item of a plan: more warps asked for than the automatic
 // 4 get items as much larger, so that a warp's share stays what it was (16 warps, FP32,
-// 20,000 rows of 20 / 400,000 of 12 nonzeros: 17.8 / 47 us in the
-// automatic items, 10.4 / 30 like this).  Atomics on 1- and 2-byte types are
-// compare-and-swap loops on words that neighbouring rows share; with rows longer than
-// an item all items meet on a few words, so that fewer items are better (INT8, 200
-// rows of 5000: 21 us in 846 items, 17 in 245).
+// 20,000 rows of 20 / 400,000 of 12 nonzeros: 17.8 / 47 us in the automatic items, 10.4 /
+// 30 like this).  Atomics on 1- and 2-byte types are compare-and-swap loops on words
+// that neighbouring rows share; with rows longer than an item all items meet on a few
+// words, so that fewer items are better (INT8, 200 rows of 5000: 21 us in 846 items, 17
+// in 245).
 static uint32_t coo_item(const sparsep_opts &o, uint64_t nnz, uint64_t nrows, size_t es) {
   uint32_t item = coo_item_elems(nnz);
   if (o.sync != SPARSEP_SYNC_LF && es < 4 && nnz > nrows * (uint64_t)item) item = 4096;
@@ -415,7 +416,7 @@ static uint32_t coo_item(const sparsep_opts &o, uint64_t nnz, uint64_t nrows, si
 static uint64_t bcoo_item_blocks(uint32_t rb, uint32_t cb, size_t es, uint64_t nblocks) {
   const uint64_t S = bcoo_chunk_blocks(rb, cb, es);
   if (!S) return std::max<uint64_t>(1, AUTO_ITEM_ENTRIES / ((uint64_t)rb * cb));
-  return std::min<uint64_t>(S, std::max<uint64_t>(32, (nblocks / 592 + 3) & ~3ull));
+  return std::min<uint64_t>(S, std::max<uint64_t>(32, (nblocks / 592 + 3) & ~3ull));  // 4 per SM of a B200
 }
 
 static std::vector<uint64_t> even_cuts(uint64_t e0, uint64_t e1, uint64_t per) {

@@ -140,3 +140,22 @@ def test_bcoo_lanes_by_the_items_own_block_rows(b):
         for _ in range(2):
             check(run(plan, x, n), n, r, c, v, x, "f32")
         plan.free()
+
+
+@pytest.mark.parametrize("dtype,width", [("f32", 45_048), ("f64", 22_524), ("i8", 180_192)])  # 176 KB less 32 bytes
+@pytest.mark.parametrize("kind", ["dbcsr", "dbcoo"])
+def test_staged_x_up_to_the_limit(dtype, width, kind):
+    rng = np.random.default_rng(3)
+    n = 600
+    for w, fits in ((width, 1), (width + 4, 0)):
+        r = np.repeat(np.arange(n), 20)
+        c = rng.integers(0, 2 * w, r.size)
+        at = np.unique(r * (2 * w) + c)
+        r, c = (at // (2 * w)).astype(np.uint32), (at % (2 * w)).astype(np.uint32)
+        v, x = random_x(rng, r.size, dtype), random_x(rng, 2 * w, dtype)
+        D = sp.convert("dcsr2" + kind, sp.convert("cooe2dcsr", sp.cooe(dtype, n, 2 * w, r, c, v), 1, 2), 4, 4)
+        plan = sp.Plan(D, sp.default_opts(stage_x=1))
+        assert plan.info.stage_x == fits
+        for _ in range(2):
+            check(run(plan, x, n), n, r, c, v, x, dtype)
+        plan.free()

@@ -573,15 +573,11 @@ __device__ __forceinline__ void load_xpiece(const Params<T> &P, const Item &it, 
 // costs FP32 1 to 2 % and FP64 3 to 4 % (1M rows 4x4, FP64: 116 -> 120 us; two plain sums
 // in turn 118.5 us, but 200 blocks 8x8 no better than bcsr_rows).
 template <typename T> struct RowSum {
-  Acc<T> s = Acc<T>(0), off = Acc<T>(0);
+  Acc<T> s = Acc<T>(0), off = Acc<T>(0);  // off: floating point only
   __device__ __forceinline__ void add(Acc<T> x) {
-    if constexpr (std::is_floating_point<T>::value) {
-      const Acc<T> t = s + x;
-      off += x - (t - s);
-      s = t;
-    } else {
-      s += x;
-    }
+    const Acc<T> t = s + x;
+    off += x - (t - s);
+    s = t;
   }
   // off is not a number once a sum is infinite
   __device__ __forceinline__ Acc<T> get() const {
@@ -604,6 +600,11 @@ __device__ __forceinline__ void pieces_mv(const uint32_t (&v)[N][Pieces<T, RB, C
 #pragma unroll
         for (int q = 0; q < G::NX / 4; ++q)
           acc[r].s = (uint32_t)__dp4a((int)v[n][r * (G::NX / 4) + q], (int)x[n][q], (int)acc[r].s);
+    } else if constexpr (!std::is_floating_point<T>::value) {
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int c = 0; c < G::NX; ++c) acc[r].s += mul<T>(word_elem<T>(v[n], r * G::NX + c), word_elem<T>(x[n], c));
     } else {
       Acc<T> sum = Acc<T>(0);
 #pragma unroll
@@ -648,8 +649,8 @@ __device__ __forceinline__ void sum_pieces(Acc<T> (&acc)[Pieces<T, RB, CB>::RPC]
 // per warp over contiguous block rows 185 us (143 M instructions at the block
 // rows' ends); persistent CTAs with two chunks in flight 176 us and with x
 // gathered a chunk ahead 160 us (24 warps per SM cannot hide the x loads).
-// Chunks of 24 / 28 / 40 KB: 133 / 125 / 127 us against 119 us for 32 KB, five
-// CTAs per SM; 46 instead of 40 registers (four CTAs) 126 us.
+// Chunks of 24 / 28 / 40 KB: 133 / 125 / 127 us against 119 us for 32 KB, six
+// CTAs per SM; 46 instead of 40 registers (five CTAs) 126 us.
 // ---------------------------------------------------------------------------
 template <typename T, int RB, int CB> struct BlockStage {
   using G = Pieces<T, RB, CB>;

@@ -13,7 +13,7 @@
 //            consecutive addresses.
 // Bound by HBM in the limit (a record is read and written once per pass: 38 us for
 // 10.5 M records of 12 bytes); a pass takes 12 us (hist) + 10 (scan) + 80 (scatter),
-// the scatter's ranking and its address arithmetic having half of the issue slots.
+// the scatter issuing in 40 % of the cycles for its ranking and address arithmetic.
 // 512 threads and two CTAs per SM: 1024 threads are 8 to 20 % slower, 3 CTAs at 42
 // registers no faster.  With 256 threads of 16 elements and __match_any_sync the
 // scatter took 236 us; with 4-bit digits, 1024-element tiles and three barriers per

@@ -609,8 +609,9 @@ int sparsep_trim_scratch(void);
  * nrows + 1, d_colind / d_vals_out: nnz.  Rows ascending, input order kept
  * inside a row (stable).  EINVAL if a row index is >= nrows.  Allocates its
  * own scratch, 12 bytes and a value per nonzero (4 bytes up to 128 rows; where
- * the device has no room, 8 bytes per nonzero for values of 8 bytes); the
- * outputs must not overlap the inputs.  Synchronises the stream. */
+ * the device has no room, 8 bytes per nonzero for values of 8 bytes).  With more
+ * than 128 rows the outputs may lie over the inputs, for 4 more bytes and another
+ * value from 16,385 rows on.  Synchronises the stream. */
 #define SPARSEP_DECLARE_C2C(T, S)                                                                               \
   int sparsep_coo2csr_device_##S(const uint32_t *d_rows, const uint32_t *d_cols, const T *d_vals, uint32_t nnz, \
                                  uint32_t nrows, uint32_t *d_rowptr, uint32_t *d_colind, T *d_vals_out,         \

@@ -15,7 +15,9 @@
 // more than the 16 bytes of a sort of indices, are sorted by their indices, which lie
 // in the outputs until a gather replaces them: 8 bytes per nonzero.
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <new>
 
 #include "fault.hpp"
@@ -82,11 +84,23 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
   if (nrows <= 1) bits = 0;
   const int np = passes(bits);
   const size_t n = nnz, vb = ((n * sizeof(V)) + 15) & ~(size_t)15, kb = ((n * 4) + 15) & ~(size_t)15;
-  const size_t keys = np > 1 ? 2 * kb : kb, set = np > 1 ? kb + vb : 0, rest = count_words(nnz) * 4 + 64;
+  // Outputs that overlap the inputs are written by the last pass alone (the inputs are
+  // read by the first alone), with two more sets between.
+  auto meet = [](const void *a, size_t an, const void *b, size_t bn) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + bn && y < x + an;
+  };
+  bool in_place = false;
+  for (const void *in : {(const void *)rows, (const void *)cols, (const void *)vals}) {
+    const size_t bytes = n * (in == (const void *)vals ? sizeof(V) : 4);
+    in_place |= meet(colind, n * 4, in, bytes) || meet(vals_out, n * sizeof(V), in, bytes);
+  }
+  const size_t keys = np > 1 ? 2 * kb : kb, one = np > 1 ? kb + vb : 0, set = in_place && np > 2 ? 2 * one : one,
+               rest = count_words(nnz) * 4 + 64;
   sparsep::Scratch mem;
   bool by_index = false;
   cudaError_t e = sparsep::ws_malloc(&mem, keys + set + rest, s);
-  if (e == cudaErrorMemoryAllocation && sizeof(V) == 8 && np > 1) {
+  if (e == cudaErrorMemoryAllocation && sizeof(V) == 8 && np > 1 && !in_place) {
     by_index = true;
     e = sparsep::ws_malloc(&mem, keys + rest, s);
   }
@@ -94,8 +108,8 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
   if (st) return st;
   unsigned char *buf = static_cast<unsigned char *>(mem.p);
   uint32_t *key_buf[2] = {reinterpret_cast<uint32_t *>(buf), reinterpret_cast<uint32_t *>(buf + keys - kb)};
-  uint32_t *col_set = reinterpret_cast<uint32_t *>(buf + keys);
-  V *val_set = reinterpret_cast<V *>(buf + keys + kb);
+  auto col_set = [&](int p) { return reinterpret_cast<uint32_t *>(buf + keys + (in_place && p % 2 ? one : 0)); };
+  auto val_set = [&](int p) { return reinterpret_cast<V *>(buf + keys + (in_place && p % 2 ? one : 0) + kb); };
   uint32_t *counts = reinterpret_cast<uint32_t *>(buf + keys + (by_index ? 0 : set));
   int *bad = reinterpret_cast<int *>(counts + count_words(nnz));
   const uint32_t *key = rows, *col = by_index ? nullptr : cols;
@@ -105,17 +119,17 @@ static int coo2csr_device(const uint32_t *rows, const uint32_t *cols, const V *v
     st = c2c_err(cudaMemsetAsync(bad, 0, sizeof(int), s));
     for (int p = 0, shift = 0; !st && p < np; shift += pass_bits(bits, p, np), ++p) {
       const int b = pass_bits(bits, p, np);
-      const bool out = (np - 1 - p) % 2 == 0;  // the last pass writes the outputs
+      const bool out = in_place ? p == np - 1 : (np - 1 - p) % 2 == 0;  // the last pass writes the outputs
       st = c2c_err(count_pass<uint32_t>(key, nnz, shift, b, counts, s, p ? nullptr : bad, nrows));
       if (!st && p == 0) {  // nothing of the outputs is written for a row index >= nrows
         st = c2c_err(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
         if (!st) st = c2c_err(cudaStreamSynchronize(s));
         if (!st && h_bad) st = SPARSEP_EINVAL;
       }
-      uint32_t *ko = key_buf[p % 2], *co = out ? colind : by_index ? reinterpret_cast<uint32_t *>(vals_out) : col_set;
+      uint32_t *ko = key_buf[p % 2], *co = out ? colind : by_index ? reinterpret_cast<uint32_t *>(vals_out) : col_set(p);
       if (!st && by_index)
         st = c2c_err(scatter_pass<uint32_t, NoValue>(key, col, nullptr, nnz, shift, b, counts, ko, co, nullptr, s));
-      V *vo = out ? vals_out : val_set;
+      V *vo = out ? vals_out : val_set(p);
       if (!st && !by_index) {
         st = c2c_err(scatter_pass<uint32_t, V>(key, col, val, nnz, shift, b, counts, ko, co, vo, s));
         val = vo;

@@ -202,3 +202,28 @@ def test_without_room_values_of_8_bytes_go_by_index(dtype, nrows, nnz):
     assert bool((colind == cols[order]).all()) and bool((out == vals[order]).all())
     want = rows.bincount(minlength=nrows).cumsum(0)
     assert rowptr[0] == 0 and bool((rowptr[1:] == want).all())
+
+
+@pytest.mark.parametrize("dtype", ["i8", "f32", "f64"])
+@pytest.mark.parametrize("nrows", [129, 1 << 14, (1 << 14) + 1, 1 << 20, 1 << 24])  # two to four passes
+@pytest.mark.parametrize("what", ["both", "columns", "values", "crossed"])
+def test_outputs_over_the_inputs(dtype, nrows, what):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(nrows)
+    nnz = 3_000_001  # more tiles than run at once
+    rows = torch.randint(0, nrows, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    cols = torch.randint(0, 2**31 - 1, (nnz,), generator=g, device="cuda", dtype=torch.int32)
+    vals = torch.randint(-100, 100, (nnz,), generator=g, device="cuda").to(getattr(torch, TORCH[dtype]))
+    order = rows.argsort(stable=True)
+    want_c, want_v, want_r = cols[order], vals[order], rows.bincount(minlength=nrows).cumsum(0)
+    colind = cols if what in ("both", "columns") else rows if what == "crossed" else torch.empty_like(cols)
+    out = vals if what in ("both", "values") else torch.empty_like(vals)
+    rowptr = torch.empty(nrows + 1, dtype=torch.int32, device="cuda")
+    f = getattr(capi.lib(), f"sparsep_coo2csr_device_{dtype}")
+    f.argtypes = [C.c_void_p] * 3 + [C.c_uint32, C.c_uint32] + [C.c_void_p] * 4
+    torch.cuda.synchronize()
+    capi.check(f(rows.data_ptr(), cols.data_ptr(), vals.data_ptr(), nnz, nrows, rowptr.data_ptr(), colind.data_ptr(),
+                 out.data_ptr(), None), "coo2csr_device")
+    assert torch.equal(colind, want_c) and torch.equal(out, want_v)
+    assert rowptr[0] == 0 and bool((rowptr[1:] == want_r).all())
